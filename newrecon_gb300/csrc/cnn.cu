@@ -15,11 +15,11 @@
 // in the K-major core-matrix layout with rows 16 bytes apart; the three dx
 // taps are the same strip read from row offsets 0, 1, 2 (descriptor start +
 // 16 B).  The strips arrive by TMA (activations are stored in 8-channel planes
-// so that a strip's K chunk is one contiguous block); a CTA walks along y so
-// that each staged input row serves the three output rows that read it, and a
-// producer warp, an MMA warp and two groups of epilogue warps overlap staging,
-// MMAs and stores (conv32_walk_kernel).  Weights of all 27 taps stay in shared
-// memory.  1-channel inputs gather the 27 neighbours into one K = 32 row
+// so that a strip's K chunk is one contiguous block); a CTA walks along y and
+// adds each staged input row into the accumulators of the three output rows
+// that read it, and a producer warp, an MMA warp and groups of epilogue warps
+// overlap staging, MMAs and stores (conv32_ys_kernel).  Weights of all 27 taps
+// stay in shared memory.  1-channel inputs gather the 27 neighbours into one K = 32 row
 // instead.  Weight gradients are GEMMs over voxels on the tensor cores
 // (wgrad_tc_kernel), ending in a fixed-order reduction of per-CTA partials.
 #include <cuda_bf16.h>
@@ -38,7 +38,7 @@ constexpr int SROWS = TM + 2;         // strip rows incl. the x halo
 constexpr int KCH = 4;                // 16-byte K chunks per 32-channel row
 constexpr int WAIT_LIMIT = 1 << 24;   // polls before a wait gives up
 
-enum { EPI_RELU = 0, EPI_MASK = 1, EPI_RESID = 2 };
+enum { EPI_RELU = 0, EPI_MASK = 1 };
 
 struct Dims {
     int nx, ny, nz, nb;
@@ -101,25 +101,6 @@ __device__ __forceinline__ void load_strip(uint8_t* dst, int pstride, const CUte
     }
 }
 
-// Named barriers over the n threads of a group of warps (id >= 1; id 0 is
-// __syncthreads).  group_all is also a vote: true when v is true in every
-// thread.  Every warp of the group must reach each of them the same number of
-// times; callers take their decisions to stop from group_all, so that no warp
-// leaves while the others wait.
-__device__ __forceinline__ bool group_all(bool v, int id, int n) {
-    uint32_t r;
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, %2, %3, q;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(r)
-        : "r"((uint32_t)v), "r"(id), "r"(n)
-        : "memory");
-    return r != 0;
-}
-__device__ __forceinline__ void group_sync(int id, int n) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-
 // A bounded wait that also gives up once the block has aborted.
 __device__ __forceinline__ bool wait_live(uint64_t* bar, uint32_t parity, volatile int* abort) {
     for (int round = 0; round < WAIT_LIMIT / 1024; round++) {
@@ -129,51 +110,102 @@ __device__ __forceinline__ bool wait_live(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
-// ---- conv32: TMA + tcgen05, walking along y -----------------------------------
-// 32-channel input, NOUT = 32 (hidden / input gradient) or 16 (the last layer,
-// output channel 0 real) outputs; weights: 27 packed taps of NOUT x 32; one
-// output tile (128 x of a row) per TMEM accumulator, staging shared between
-// neighbouring output rows.  A work item is a run of up to L output
-// rows y0 .. y0 + L - 1 of one column (patch b, plane z, x tile); its tiles
-// read the row-sets Y = y0 - 1 .. y0 + L, a row-set being the strips of input
-// row Y in planes z - 1, z, z + 1.  Each row-set is loaded once into a ring of
-// W_R slots and serves the up to three tiles that read it, so an input row is
-// staged about (L + 2) / L times per plane instead of nine.  A strip outside
-// the patch is loaded from row -1 (zero-filled), so that every tile issues the
-// same 54 MMAs, with descriptors formed as base + compile-time offset.
-//   warp 8 (one lane)  producer: row-sets in order into the ring ("full"),
-//                      after the slot's previous row-set was released;
-//   warp 9 (one lane)  MMA issuer: per tile the row-sets i, i + 1, i + 2 of
-//                      the item, 6 MMAs per valid strip, into accumulator
-//                      lt & 1; row-set i is released (tcgen05.commit to its
-//                      "empty") right after its MMAs -- its last use -- and
-//                      the item's last two after its last tile;
-//   warps 0-3, 4-7     two epilogue groups, group g for the tiles lt with
-//                      lt & 1 == g, so that two epilogues run at once.
+// ---- conv32: bulk copies + tcgen05, walking along y ----------------------------
+// 32 -> 32 channels (hidden layers and their input gradients).  A work item is
+// a run of up to L output rows y0 .. y0 + L - 1 of one column (patch b, planes
+// z and z + 1, x tile of 128).  The item's input rows Y = y0 - 1 .. y0 + L come
+// one after another as row-sets (the strips of row Y in planes z - 1 .. z + 2),
+// and each row-set is used by one step only: the three dy taps are stacked
+// along N, so that one MMA over a strip at row offset dx adds
+//     D[x][(dy, o)] += sum_i a[x0 - 1 + x + dx][i] W[dz][dy][dx][o][i]
+// to the accumulators of the three output rows that read row Y -- rows Y - 1
+// (dy = 2), Y (dy = 1) and Y + 1 (dy = 0), 32 TMEM columns each, side by side:
+// 18 MMAs of M = 128, N = 96, K = 16 per input row and output plane.
+//
+// Two output planes share two of their four strips, and each plane's MMAs are
+// issued by a warp of its own: issued from a one-lane branch the MMAs followed
+// each other 96 - 140 cycles apart whatever their size (N = 32 and N = 96
+// alike: 48 cycles of math at N = 96), with warp-uniform descriptors about 65,
+// with one warp per plane about 35 -- the operand fetch (7 KB of shared memory
+// per N = 96 MMA, 56 cycles) is then the tensor side's limit and the strips'
+// delivery (0.94 ms per clinical layer with the MMAs left out) the next.
+// A hidden layer on 1024 x 512 x 60 voxels: 1.05 - 1.12 ms against 2.46 ms for
+// the form before (dx stacked along N, shifted back in the epilogue by warp
+// shuffles); steps: 2.35 ms with dy stacked, one plane per CTA and tensor-map
+// copies; 1.42 with two planes and bulk copies; 1.18 with warp-wide issue.
+//
+// Accumulators: 8 slots of 32 columns per plane.  Step T (the CTA's steps
+// counted through) works on the window of slots s, s + 1, s + 2, s = T % 6.
+// For s > 0 the last of the three is fresh (its part of the step's first MMA
+// is issued by itself, without accumulation); at s = 0 the window jumps back
+// to slots 0 - 2 and all three are fresh, so that the two rows in the middle
+// of their three steps have their sum in two slots, added by the epilogue.
+// The row that step T starts is "row T" (rows outside the run are computed
+// and not stored): complete after step T + 2, in slot T % 6 + 2 (T % 6 < 4),
+// in slots 6 and 0 (4) or 7 and 1 (5); step T needs row T - 6 read.
+//
+// The dx shift is the strip's row offset (descriptor start + 16 B), so the
+// accumulator rows are output voxels and the epilogue is one TMEM read, bias
+// and ReLU (or mask) and the store.  Strips arrive as plain bulk copies, one
+// contiguous run per 8-channel plane (a tensor-map copy of the same run as two
+// boxes took about 90 cycles per 1 KB box, 2.0 ms per clinical layer by
+// itself); rows outside the patch come from a block of zeros.
+//   warp 4 Y_NG            producer (16 lanes): row-sets into a ring of Y_R slots;
+//   warps 4 Y_NG + 1, + 2  MMA issuers of the two planes (one elected lane each);
+//   groups of four warps   epilogues, group g: plane g & 1 of the rows T with
+//                          T % Y_NT == g >> 1.
 // One CTA per SM (the ring and all 27 taps' weights).  Every wait is bounded
 // and also gives up once another role has aborted; a role that gives up flags
 // NR_FLAG_TIMEOUT and aborts the block.  Before TMEM is released the issuer's
 // MMAs are drained, and the producer waits for every copy it issued.
-// Measured against the previous form (nine strips per tile, two CTAs per SM):
-// L2 traffic falls from 67 % to 8 % of its throughput and the network's
-// forward pass on the clinical volume from 22.6-23.0 to 22.5 ms -- the MMAs'
-// front end (sm__pipe_tc 57 % with the math at 14 %: an N = 32 MMA reads 5 KB
-// of operands for 65 K MACs) paces both.
-constexpr int W_R = 6;                                 // row-set slots
-constexpr int W_SET = 3 * TSTRIP;                      // 26112 bytes
-constexpr int W_THREADS = 320;
-
-struct WalkCtl {
-    uint64_t full[W_R], empty[W_R], accf[2], acce[2], drain;
-    uint32_t tslot;
-    int abort;
-};
+constexpr int W_SET = 3 * TSTRIP;                      // three strips (wgrad_walk_kernel)
+constexpr int Y_SET = 4 * TSTRIP;                      // 34816 bytes
+constexpr int Y_R = 4;                                 // row-set slots
+constexpr int Y_NT = 2;                                // rows in the epilogue at once
+constexpr int Y_NG = 2 * Y_NT;                         // epilogue groups
+constexpr int Y_THREADS = 32 * (4 * Y_NG + 3);
+constexpr int Y_ROWS = 8;                              // row barriers (six rows in use at most)
+constexpr int Y_WBYTES = 27 * C * C * 2;
 
 struct WalkPlan {
     int L, nchunk;
     int tw;  // outputs per tile along x
     int64_t nitems;
 };
+
+struct YCtl {
+    uint64_t full[Y_R], empty[Y_R], accf[Y_ROWS], acce[Y_ROWS], drain;
+    uint32_t tslot;
+    int abort;
+    float bias[C];
+};
+
+// The zeros that rows outside a patch are copied from.
+static __device__ __align__(16) uint4 g_zero_rows[SROWS];
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
+                                          uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(tc::smem_u32(dst)),
+        "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(tc::smem_u32(bar))
+        : "memory");
+}
+
+// K chunk kc of the strip of row `row` (-1: zeros) from x0 - 1, 130 rows of 16
+// bytes: the part inside [0, nx) from the activations, the rest zeros.
+__device__ __forceinline__ void load_chunk(uint8_t* dst, const __nv_bfloat16* in, int nx, int x0,
+                                           int64_t row, int kc, uint64_t* bar) {
+    if (row < 0) {
+        bulk_load(dst, g_zero_rows, SROWS * 16, bar);
+        return;
+    }
+    const int lo = x0 == 0 ? 1 : 0, hi = min(x0 + SROWS - 1, nx) - x0 + 1;  // strip rows [lo, hi)
+    if (lo) bulk_load(dst, g_zero_rows, 16, bar);
+    bulk_load(dst + lo * 16, in + ((row * KCH + kc) * nx + x0 - 1 + lo) * 8, (uint32_t)(hi - lo) * 16,
+              bar);
+    if (hi < SROWS) bulk_load(dst + hi * 16, g_zero_rows, (uint32_t)(SROWS - hi) * 16, bar);
+}
 
 // Column (b, z, x0) and rows y0 .. y0 + ly - 1 of item it.
 __device__ __forceinline__ void item_pos(const Dims& d, const WalkPlan& w, int64_t it, int& b,
@@ -189,15 +221,13 @@ __device__ __forceinline__ void item_pos(const Dims& d, const WalkPlan& w, int64
     ly = min(w.L, d.ny - y0);
 }
 
-// Epilogue of output row `row` (one (patch, z, y) row), voxel x.
+// Epilogue of output row `row` (one (patch, z, y) row), voxel x: bias and ReLU
+// or the ReLU mask of the layer below, stored as BF16.  bias: C floats.
 template <int EPI>
 __device__ __forceinline__ void epilogue_rx(const uint32_t* acc, int64_t row, int x, int nx,
-                                            const float* __restrict__ bias, void* out,
+                                            const float* __restrict__ bias,
+                                            __nv_bfloat16* __restrict__ out,
                                             const __nv_bfloat16* __restrict__ mask) {
-    if (EPI == EPI_RESID) {
-        ((float*)out)[row * nx + x] = __uint_as_float(acc[0]) + bias[0];
-        return;
-    }
     const int64_t o0 = row * KCH * (int64_t)nx * 8 + (int64_t)x * 8;  // chunk q at o0 + q nx 8
     __align__(16) __nv_bfloat16 o[C];
     if (EPI == EPI_RELU) {
@@ -222,232 +252,39 @@ __device__ __forceinline__ void epilogue_rx(const uint32_t* acc, int64_t row, in
     }
 #pragma unroll
     for (int q = 0; q < KCH; q++)
-        *(uint4*)((__nv_bfloat16*)out + o0 + (int64_t)q * nx * 8) = ((const uint4*)o)[q];
+        *(uint4*)(out + o0 + (int64_t)q * nx * 8) = ((const uint4*)o)[q];
 }
 
-template <int NOUT, int EPI>
-__global__ void __launch_bounds__(W_THREADS, 1) conv32_walk_kernel(
-    Dims d, WalkPlan wp, const __grid_constant__ CUtensorMap amap,
-    const __grid_constant__ CUtensorMap amap_hi, const __nv_bfloat16* __restrict__ wpk,
-    const float* __restrict__ bias, void* out, const __nv_bfloat16* __restrict__ mask,
-    int* status) {
-    constexpr int WBYTES = 27 * NOUT * C * 2;
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* ring = smem;
-    uint8_t* sW = smem + W_R * W_SET;
-    WalkCtl* K = (WalkCtl*)(sW + WBYTES);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int k = tid; k < WBYTES / 16; k += W_THREADS)
-        ((uint4*)sW)[k] = __ldg((const uint4*)wpk + k);
-    if (tid == 0) {
-        for (int s = 0; s < W_R; s++) {
-            tc::mbar_init(&K->full[s], 1);
-            tc::mbar_init(&K->empty[s], 1);
-        }
-        for (int a = 0; a < 2; a++) {
-            tc::mbar_init(&K->accf[a], 1);
-            tc::mbar_init(&K->acce[a], 4);
-        }
-        tc::mbar_init(&K->drain, 1);
-        K->abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) tc::tmem_alloc(&K->tslot, 64);
-    tc::fence_async_smem();
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = K->tslot;
-    volatile int* abort = &K->abort;
-    auto fail = [&]() {
-        if (!*abort) atomicOr(status, NR_FLAG_TIMEOUT);
-        *abort = 1;
-        __threadfence_block();
-    };
-    auto strip_ok = [&](int zz, int yy) { return zz >= 0 && zz < d.nz && yy >= 0 && yy < d.ny; };
-    if (warp == 8) {
-        if (lane == 0) {
-            // producer
-            int64_t G = 0, issued = 0;
-            bool stop = false;
-            for (int64_t it = blockIdx.x; it < wp.nitems && !stop && !*abort; it += gridDim.x) {
-                int b, z, x0, y0, ly;
-                item_pos(d, wp, it, b, z, x0, y0, ly);
-                for (int j = 0; j < ly + 2; j++, G++) {
-                    const int s = (int)(G % W_R);
-                    if (G >= W_R &&
-                        !wait_live(&K->empty[s], (uint32_t)((G / W_R - 1) & 1), abort)) {
-                        fail();
-                        stop = true;
-                        break;
-                    }
-                    const int Y = y0 - 1 + j;
-                    mbar_arrive_tx(&K->full[s], 3 * STRIP_TX);
-                    for (int dz = 0; dz < 3; dz++)
-                        load_strip(ring + s * W_SET + dz * TSTRIP, PLANE, &amap, &amap_hi, x0,
-                                   strip_ok(z + dz - 1, Y) ? (b * d.nz + z + dz - 1) * d.ny + Y : -1,
-                                   &K->full[s]);
-                    issued = G + 1;
-                }
-            }
-            // no copy may be in flight when the block exits
-            for (int64_t k = issued > W_R ? issued - W_R : 0; k < issued; k++) {
-                uint64_t* bar = &K->full[k % W_R];
-                if (!tc::mbar_wait(bar, (uint32_t)((k / W_R) & 1), WAIT_LIMIT))
-                    tc::mbar_wait(bar, (uint32_t)((k / W_R) & 1), WAIT_LIMIT);
-            }
-        }
-    } else if (warp == 9) {
-        if (lane == 0) {
-            // MMA issuer
-            constexpr uint32_t idesc = tc::idesc_bf16(TM, NOUT);
-            const uint64_t ad0 = tc::sdesc(tc::smem_u32(ring), PLANE, 128);
-            const uint64_t bd0 = tc::sdesc(tc::smem_u32(sW), 128, 512);
-            int64_t G = 0;
-            int lt = 0;
-            bool stop = false;
-            for (int64_t it = blockIdx.x; it < wp.nitems && !stop && !*abort; it += gridDim.x) {
-                int b, z, x0, y0, ly;
-                item_pos(d, wp, it, b, z, x0, y0, ly);
-                for (int i = 0; i < ly && !stop; i++, lt++) {
-                    const int a = lt & 1;
-                    if (lt >= 2 &&
-                        !wait_live(&K->acce[a], (uint32_t)(((lt >> 1) - 1) & 1), abort)) {
-                        fail();
-                        stop = true;
-                        break;
-                    }
-                    tc::fence_after();
-                    const uint32_t dacc = tmem + (uint32_t)(a * 32);
-#pragma unroll
-                    for (int dy = 0; dy < 3; dy++) {
-                        const int64_t gs = G + i + dy;
-                        const int s = (int)(gs % W_R);
-                        if ((i == 0 || dy == 2) &&
-                            !wait_live(&K->full[s], (uint32_t)((gs / W_R) & 1), abort)) {
-                            fail();
-                            stop = true;
-                            break;
-                        }
-                        tc::fence_after();
-                        // descriptors are linear in the address: base + offset / 16
-                        const uint64_t adr = ad0 + (uint64_t)((s * W_SET) >> 4);
-#pragma unroll
-                        for (int dz = 0; dz < 3; dz++)
-#pragma unroll
-                            for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                                for (int j = 0; j < 2; j++) {
-                                    const int tap = dz * 9 + dy * 3 + dx;
-                                    tc::mma_bf16(
-                                        dacc,
-                                        adr + (uint64_t)((dz * TSTRIP + dx * 16 + j * 2 * PLANE) >> 4),
-                                        bd0 + (uint64_t)((tap * NOUT * C * 2 + j * 256) >> 4), idesc,
-                                        (dy | dz | dx | j) ? 1u : 0u);
-                                }
-                        // row-set i is not read after this tile; the last tile
-                        // of the item also frees row-sets ly and ly + 1
-                        if (dy == 0 || i == ly - 1) tc::commit(&K->empty[s]);
-                    }
-                    if (stop) break;
-                    tc::commit(&K->accf[a]);
-                }
-                G += ly + 2;
-            }
-        }
-    } else {
-        // epilogue group g = warp / 4: TMEM lanes 32 (warp % 4) .. + 31 of the
-        // tiles lt with lt & 1 == g.  Test hook: the workspace's second status
-        // word k + 1 > 0 makes the wait for this CTA's tile k report giving up
-        // once it has in fact succeeded.
-        const int g = warp >> 2, wq = warp & 3;
-        const int force_at = status[1] - 1;
-        int lt = 0;
-        bool stop = false;
-        for (int64_t it = blockIdx.x; it < wp.nitems && !stop; it += gridDim.x) {
-            int b, z, x0, y0, ly;
-            item_pos(d, wp, it, b, z, x0, y0, ly);
-            for (int i = 0; i < ly; i++, lt++) {
-                if ((lt & 1) != g) continue;
-                bool got = wait_live(&K->accf[g], (uint32_t)((lt >> 1) & 1), abort);
-                if (lt == force_at) got = false;
-                if (!got) {
-                    if (lane == 0) fail();
-                    stop = true;
-                    break;
-                }
-                tc::fence_after();
-                uint32_t acc[32];
-                tc::ld32(tmem, (uint32_t)(wq * 32), (uint32_t)(g * 32), acc);
-                tc::fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&K->acce[g]);
-                const int x = x0 + wq * 32 + lane;
-                if (x < d.nx)
-                    epilogue_rx<EPI>(acc, ((int64_t)b * d.nz + z) * d.ny + y0 + i, x, d.nx, bias,
-                                     out, mask);
-            }
-        }
-    }
-    // drain: every MMA issued has completed before TMEM is released
-    __syncthreads();
-    if (warp == 9 && lane == 0) tc::commit(&K->drain);
-    if (!tc::mbar_wait(&K->drain, 0, WAIT_LIMIT)) tc::mbar_wait(&K->drain, 0, WAIT_LIMIT);
-    tc::fence_before();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 64);
+// Column (b, z, x0) and rows y0 .. y0 + ly - 1 of item it: z the first of two planes.
+__device__ __forceinline__ void item_pos2(const Dims& d, const WalkPlan& w, int64_t it, int& b,
+                                          int& z, int& x0, int& y0, int& ly) {
+    item_pos(Dims{d.nx, d.ny, (d.nz + 1) / 2, d.nb}, w, it, b, z, x0, y0, ly);
+    z *= 2;
 }
 
-// ---- conv32 with the three dx taps in one MMA -------------------------------
-// The walk of conv32_walk_kernel with N = 3 NOUT: the weights of the three dx
-// taps of a strip are adjacent in the packed buffer (512-byte row groups), so
-// one MMA over the unshifted strip (A rows r = input x0 - 1 + r) computes
-// D[r][(dx, o)] = sum_i a[x0 - 1 + r][i] W[dz][dy][dx][o][i] for all three dx:
-// 18 MMAs per tile instead of 54, and each A row is fetched once per strip
-// instead of three times.  Output x0 - 1 + r (r = 1 .. 126: 126 outputs per
-// tile, tiles 126 apart) is D[r - 1][dx 0] + D[r][dx 1] + D[r + 1][dx 2]: the
-// dx = 0 and dx = 2 columns are moved one TMEM lane by warp shuffles, and
-// across the four warps' lane quarters through shared memory (each warp
-// publishes lane 31's dx-0 and lane 0's dx-2 columns, double-buffered by
-// tile; a named barrier per epilogue group orders the exchange, the group
-// having voted on the accumulator wait first, so that its warps stop
-// together or not at all).  TMEM: two accumulators of 3 NOUT columns (at 0 and 128).
-constexpr int W3_TW = TM - 2;  // 126 outputs per tile
-constexpr int W3_NG = 4;       // epilogue groups = TMEM accumulators
-constexpr int W3_THREADS = 32 * (4 * W3_NG + 2);
-
-struct W3Ctl {
-    uint64_t full[W_R], empty[W_R], accf[W3_NG], acce[W3_NG], drain;
-    uint32_t tslot;
-    int abort;
-    float xb[W3_NG][2][4][2][C];  // [group][tile parity][warp][lane 31 dx 0 | lane 0 dx 2][o]
-};
-
-template <int NOUT, int EPI>
-__global__ void __launch_bounds__(W3_THREADS, 1) conv32_w3_kernel(
-    Dims d, WalkPlan wp, const __grid_constant__ CUtensorMap amap,
-    const __grid_constant__ CUtensorMap amap_hi, const __nv_bfloat16* __restrict__ wpk,
-    const float* __restrict__ bias, void* out, const __nv_bfloat16* __restrict__ mask,
-    int* status) {
-    constexpr int WBYTES = 27 * NOUT * C * 2;
-    constexpr int NO = EPI == EPI_RESID ? 1 : NOUT;  // output channels the epilogue needs
+template <int EPI>
+__global__ void __launch_bounds__(Y_THREADS, 1) conv32_ys_kernel(
+    Dims d, WalkPlan wp, const __nv_bfloat16* __restrict__ in,
+    const __nv_bfloat16* __restrict__ wpk, const float* __restrict__ bias,
+    __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ mask, int* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* ring = smem;
-    uint8_t* sW = smem + W_R * W_SET;
-    W3Ctl* K = (W3Ctl*)(sW + WBYTES);
+    uint8_t* sW = smem + Y_R * Y_SET;
+    YCtl* K = (YCtl*)(sW + Y_WBYTES);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int k = tid; k < WBYTES / 16; k += W3_THREADS)
+    for (int k = tid; k < Y_WBYTES / 16; k += Y_THREADS)
         ((uint4*)sW)[k] = __ldg((const uint4*)wpk + k);
+    if (EPI == EPI_RELU && tid < C) K->bias[tid] = bias[tid];
     if (tid == 0) {
-        for (int s = 0; s < W_R; s++) {
+        for (int s = 0; s < Y_R; s++) {
             tc::mbar_init(&K->full[s], 1);
-            tc::mbar_init(&K->empty[s], 1);
+            tc::mbar_init(&K->empty[s], 2);
         }
-        for (int a = 0; a < W3_NG; a++) {
-            tc::mbar_init(&K->accf[a], 1);
-            tc::mbar_init(&K->acce[a], 4);
+        for (int a = 0; a < Y_ROWS; a++) {
+            tc::mbar_init(&K->accf[a], 2);
+            tc::mbar_init(&K->acce[a], 8);
         }
-        tc::mbar_init(&K->drain, 1);
+        tc::mbar_init(&K->drain, 2);
         K->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -463,154 +300,184 @@ __global__ void __launch_bounds__(W3_THREADS, 1) conv32_w3_kernel(
         *abort = 1;
         __threadfence_block();
     };
-    auto strip_ok = [&](int zz, int yy) { return zz >= 0 && zz < d.nz && yy >= 0 && yy < d.ny; };
-    if (warp == 4 * W3_NG) {
-        if (lane == 0) {
-            // producer (as in conv32_walk_kernel)
-            int64_t G = 0, issued = 0;
-            bool stop = false;
-            for (int64_t it = blockIdx.x; it < wp.nitems && !stop && !*abort; it += gridDim.x) {
-                int b, z, x0, y0, ly;
-                item_pos(d, wp, it, b, z, x0, y0, ly);
-                for (int j = 0; j < ly + 2; j++, G++) {
-                    const int s = (int)(G % W_R);
-                    if (G >= W_R &&
-                        !wait_live(&K->empty[s], (uint32_t)((G / W_R - 1) & 1), abort)) {
-                        fail();
-                        stop = true;
-                        break;
-                    }
-                    const int Y = y0 - 1 + j;
-                    mbar_arrive_tx(&K->full[s], 3 * STRIP_TX);
-                    for (int dz = 0; dz < 3; dz++)
-                        load_strip(ring + s * W_SET + dz * TSTRIP, PLANE, &amap, &amap_hi, x0,
-                                   strip_ok(z + dz - 1, Y) ? (b * d.nz + z + dz - 1) * d.ny + Y : -1,
-                                   &K->full[s]);
-                    issued = G + 1;
-                }
-            }
-            for (int64_t k = issued > W_R ? issued - W_R : 0; k < issued; k++) {
-                uint64_t* bar = &K->full[k % W_R];
-                if (!tc::mbar_wait(bar, (uint32_t)((k / W_R) & 1), WAIT_LIMIT))
-                    tc::mbar_wait(bar, (uint32_t)((k / W_R) & 1), WAIT_LIMIT);
-            }
-        }
-    } else if (warp == 4 * W3_NG + 1) {
-        if (lane == 0) {
-            // MMA issuer: per strip (dz, dy) two MMAs of K = 16, N = 3 NOUT
-            constexpr uint32_t idesc = tc::idesc_bf16(TM, 3 * NOUT);
-            const uint64_t ad0 = tc::sdesc(tc::smem_u32(ring), PLANE, 128);
-            const uint64_t bd0 = tc::sdesc(tc::smem_u32(sW), 128, 512);
-            int64_t G = 0;
-            int lt = 0;
-            bool stop = false;
-            for (int64_t it = blockIdx.x; it < wp.nitems && !stop && !*abort; it += gridDim.x) {
-                int b, z, x0, y0, ly;
-                item_pos(d, wp, it, b, z, x0, y0, ly);
-                for (int i = 0; i < ly && !stop; i++, lt++) {
-                    const int a = lt % W3_NG;
-                    if (lt >= W3_NG &&
-                        !wait_live(&K->acce[a], (uint32_t)((lt / W3_NG - 1) & 1), abort)) {
-                        fail();
-                        stop = true;
-                        break;
-                    }
-                    tc::fence_after();
-                    const uint32_t dacc = tmem + (uint32_t)(a * 128);
-#pragma unroll
-                    for (int dy = 0; dy < 3; dy++) {
-                        const int64_t gs = G + i + dy;
-                        const int s = (int)(gs % W_R);
-                        if ((i == 0 || dy == 2) &&
-                            !wait_live(&K->full[s], (uint32_t)((gs / W_R) & 1), abort)) {
-                            fail();
-                            stop = true;
-                            break;
-                        }
-                        tc::fence_after();
-                        const uint64_t adr = ad0 + (uint64_t)((s * W_SET) >> 4);
-#pragma unroll
-                        for (int dz = 0; dz < 3; dz++)
-#pragma unroll
-                            for (int j = 0; j < 2; j++)
-                                tc::mma_bf16(
-                                    dacc, adr + (uint64_t)((dz * TSTRIP + j * 2 * PLANE) >> 4),
-                                    bd0 + (uint64_t)(((dz * 9 + dy * 3) * NOUT * C * 2 + j * 256) >> 4),
-                                    idesc, (dy | dz | j) ? 1u : 0u);
-                        if (dy == 0 || i == ly - 1) tc::commit(&K->empty[s]);
-                    }
-                    if (stop) break;
-                    tc::commit(&K->accf[a]);
-                }
-                G += ly + 2;
-            }
-        }
-    } else {
-        // epilogue group g = warp / 4 (tiles lt with lt % W3_NG == g); TMEM lane
-        // 32 wq + lane = tile row r.  Test hook as in conv32_walk_kernel.
-        const int g = warp >> 2, wq = warp & 3;
-        const int force_at = status[1] - 1;
-        int lt = 0, kg = 0;
+    if (warp == 4 * Y_NG) {
+        // producer: lane = (strip, K chunk)
+        const int sp = lane >> 2, kc = lane & 3;
+        int T = 0;
         bool stop = false;
         for (int64_t it = blockIdx.x; it < wp.nitems && !stop; it += gridDim.x) {
             int b, z, x0, y0, ly;
-            item_pos(d, wp, it, b, z, x0, y0, ly);
-            for (int i = 0; i < ly; i++, lt++) {
-                if (lt % W3_NG != g) continue;
-                bool got = wait_live(&K->accf[g], (uint32_t)((lt / W3_NG) & 1), abort);
-                if (lt == force_at) got = false;
-                if (!group_all(got, 1 + g, 128)) {  // the group stops together
+            item_pos2(d, wp, it, b, z, x0, y0, ly);
+            const int zz = z - 1 + sp;
+            for (int j = 0; j < ly + 2; j++, T++) {
+                const int s = T % Y_R;
+                bool go = !*abort;
+                if (go && T >= Y_R) go = wait_live(&K->empty[s], (uint32_t)((T / Y_R - 1) & 1), abort);
+                if (!__all_sync(0xffffffffu, go)) {
+                    if (lane == 0) fail();
+                    stop = true;
+                    break;
+                }
+                if (lane == 0) mbar_arrive_tx(&K->full[s], 4 * KCH * SROWS * 16);
+                __syncwarp();
+                const int Y = y0 - 1 + j;
+                const bool ok = zz >= 0 && zz < d.nz && Y >= 0 && Y < d.ny;
+                if (lane < 4 * KCH)
+                    load_chunk(ring + s * Y_SET + sp * TSTRIP + kc * PLANE, in, d.nx, x0,
+                               ok ? ((int64_t)b * d.nz + zz) * d.ny + Y : -1, kc, &K->full[s]);
+            }
+        }
+        // no copy may be in flight when the block exits (T row-sets were issued)
+        if (lane == 0)
+            for (int k = T > Y_R ? T - Y_R : 0; k < T; k++) {
+                uint64_t* bar = &K->full[k % Y_R];
+                if (!tc::mbar_wait(bar, (uint32_t)((k / Y_R) & 1), WAIT_LIMIT))
+                    tc::mbar_wait(bar, (uint32_t)((k / Y_R) & 1), WAIT_LIMIT);
+            }
+    } else if (warp > 4 * Y_NG) {
+        // MMA issuer of plane p: the whole warp runs the loop, one elected lane issues
+        const int p = warp - (4 * Y_NG + 1);
+        const uint64_t ad0 = tc::sdesc(tc::smem_u32(ring), PLANE, 128);
+        const uint64_t bd0 = tc::sdesc(tc::smem_u32(sW), 128, 512);
+        const uint32_t ahi = (uint32_t)(ad0 >> 32), bhi = (uint32_t)(bd0 >> 32);
+        // K step m = (dz, dx, j): N = 32 n accumulator columns from window row k
+        // on (row 0 = output row Y - 1, whose weights come first in the packed
+        // block of (dz, dx))
+        auto mma = [&](uint32_t alo, uint32_t win, int m, int k, int n, uint32_t acc) {
+            const int dz = m / 6, dx = (m / 2) % 3, j = m & 1;
+            tc::mma_bf16_warp(
+                win + (uint32_t)(k * 32),
+                alo + (uint32_t)((dz * TSTRIP + dx * 16 + j * 2 * PLANE) >> 4), ahi,
+                (uint32_t)bd0 + (uint32_t)((((dz * 3 + dx) * 3 + k) * C * C * 2 + j * 256) >> 4),
+                bhi, tc::idesc_bf16(TM, 32 * n), acc);
+        };
+        int T = 0, w = 0;  // step, T % 6
+        bool stop = false;
+        for (int64_t it = blockIdx.x; it < wp.nitems && !stop; it += gridDim.x) {
+            int b, z, x0, y0, ly;
+            item_pos2(d, wp, it, b, z, x0, y0, ly);
+            for (int i = 0; i < ly + 2; i++, T++) {
+                const int s = T % Y_R;
+                const bool go =
+                    (T < 6 || wait_live(&K->acce[(T - 6) % Y_ROWS],
+                                        (uint32_t)(((T - 6) / Y_ROWS) & 1), abort)) &&
+                    wait_live(&K->full[s], (uint32_t)((T / Y_R) & 1), abort);
+                if (!__all_sync(0xffffffffu, go)) {
                     if (lane == 0) fail();
                     stop = true;
                     break;
                 }
                 tc::fence_after();
-                // columns: dx 0 at col, dx 1 at col + NOUT, dx 2 at col + 2 NOUT.
-                // First publish the lane-quarter edges (lane 31's dx 0, lane 0's
-                // dx 2), then, after the group barrier, read the columns again
-                // into a running sum: at most 64 accumulator values live.
-                const uint32_t col = (uint32_t)(g * 128), l0 = (uint32_t)(wq * 32);
-                float* xb = &K->xb[g][kg & 1][0][0][0];
-                uint32_t c[32];
-                tc::ld32(tmem, l0, col, c);
-                if (lane == 31)
-                    for (int o = 0; o < NO; o++) xb[(wq * 2 + 0) * C + o] = __uint_as_float(c[o]);
-                tc::ld32(tmem, l0, col + 2 * NOUT, c);
-                if (lane == 0)
-                    for (int o = 0; o < NO; o++) xb[(wq * 2 + 1) * C + o] = __uint_as_float(c[o]);
-                group_sync(1 + g, 128);
-                kg++;
-                float sum[NO];
-                tc::ld32(tmem, l0, col, c);
-#pragma unroll
-                for (int o = 0; o < NO; o++) {
-                    float up = __shfl_up_sync(0xffffffffu, __uint_as_float(c[o]), 1);
-                    if (lane == 0) up = wq > 0 ? xb[((wq - 1) * 2 + 0) * C + o] : 0.f;
-                    sum[o] = up;
+                const uint32_t alo = (uint32_t)ad0 + (uint32_t)((s * Y_SET + p * TSTRIP) >> 4);
+                const uint32_t win = tmem + (uint32_t)(p * 256 + w * 32);
+                if (w == 0) {
+                    mma(alo, win, 0, 0, 3, 0u);
+                } else {
+                    mma(alo, win, 0, 0, 2, 1u);
+                    mma(alo, win, 0, 2, 1, 0u);
                 }
-                tc::ld32(tmem, l0, col + NOUT, c);
 #pragma unroll
-                for (int o = 0; o < NO; o++) sum[o] = sum[o] + __uint_as_float(c[o]);
-                tc::ld32(tmem, l0, col + 2 * NOUT, c);
-                tc::fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&K->acce[g]);
-                uint32_t acc[32];
+                for (int m = 1; m < 18; m++) mma(alo, win, m, 0, 3, 1u);
+                tc::commit_warp(&K->empty[s]);
+                if (T >= 2) tc::commit_warp(&K->accf[(T - 2) % Y_ROWS]);
+                if (++w == 6) w = 0;
+            }
+        }
+        // the last two rows lie outside the last run: nothing more is added
+        if (!stop)
+            for (int r = max(T - 2, 0); r < T; r++) tc::commit_warp(&K->accf[r % Y_ROWS]);
+        __syncwarp();
+    } else {
+        // epilogue: TMEM lanes 32 (warp % 4) .. + 31.  Test hook: the workspace's
+        // second status word k + 1 > 0 makes the wait for this CTA's row k report
+        // giving up once it has in fact succeeded.
+        const int p = (warp >> 2) & 1, tset = warp >> 3, wq = warp & 3;
+        const int force_at = status[1] - 1;
+        const int64_t qs = (int64_t)d.nx * 8, rs = KCH * qs;  // elements per chunk and per row
+        const uint32_t l0 = (uint32_t)(wq * 32);
+        int T = 0, w = 0;
+        bool stop = false;
+        for (int64_t it = blockIdx.x; it < wp.nitems && !stop; it += gridDim.x) {
+            int b, z, x0, y0, ly;
+            item_pos2(d, wp, it, b, z, x0, y0, ly);
+            const int x = x0 + wq * 32 + lane;
+            const bool in_vol = x < d.nx && z + p < d.nz;
+            const int64_t o00 =
+                (((int64_t)b * d.nz + z + p) * d.ny + y0) * rs + (int64_t)x * 8;  // chunk q: + q qs
+            for (int i = 0; i < ly + 2; i++, T++) {
+                const int wt = w;
+                if (++w == 6) w = 0;
+                if (T % Y_NT != tset) continue;
+                const bool on = in_vol && i < ly;
+                const int64_t o0 = o00 + i * rs;
+                __align__(16) uint4 m4[EPI == EPI_MASK ? KCH : 1];
+                if (EPI == EPI_MASK && on) {
 #pragma unroll
-                for (int o = 0; o < NO; o++) {
-                    float dn = __shfl_down_sync(0xffffffffu, __uint_as_float(c[o]), 1);
-                    if (lane == 31) dn = wq < 3 ? xb[((wq + 1) * 2 + 1) * C + o] : 0.f;
-                    acc[o] = __float_as_uint(sum[o] + dn);
+                    for (int q = 0; q < KCH; q++) m4[q] = __ldg((const uint4*)(mask + o0 + q * qs));
                 }
-                const int r = wq * 32 + lane, x = x0 - 1 + r;
-                if (r >= 1 && r <= W3_TW && x < d.nx)
-                    epilogue_rx<EPI>(acc, ((int64_t)b * d.nz + z) * d.ny + y0 + i, x, d.nx, bias,
-                                     out, mask);
+                bool got = wait_live(&K->accf[T % Y_ROWS], (uint32_t)((T / Y_ROWS) & 1), abort);
+                if (T == force_at) got = false;
+                if (!__all_sync(0xffffffffu, got)) {
+                    if (lane == 0) fail();
+                    stop = true;
+                    break;
+                }
+                if (i < ly) {
+                    tc::fence_after();
+                    uint32_t acc[32];
+                    tc::ld32(tmem, l0, (uint32_t)(p * 256 + (wt + 2) * 32), acc);
+                    if (wt >= 4) {
+                        uint32_t a2[32];
+                        tc::ld32(tmem, l0, (uint32_t)(p * 256 + (wt - 4) * 32), a2);
+#pragma unroll
+                        for (int c = 0; c < C; c++)
+                            acc[c] = __float_as_uint(__uint_as_float(acc[c]) + __uint_as_float(a2[c]));
+                    }
+                    tc::fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&K->acce[T % Y_ROWS]);
+                    if (on) {
+                        __align__(16) __nv_bfloat162 o[C / 2];
+                        if (EPI == EPI_RELU) {
+                            // the bias in FP32, then BF16 pairs and the ReLU on the pairs
+                            // (rounding is monotone, so max(round(v), 0) =
+                            // round(max(v, 0)) up to a zero's sign)
+                            const __nv_bfloat162 zero2 = __float2bfloat162_rn(0.f);
+#pragma unroll
+                            for (int c = 0; c < C; c += 4) {
+                                const float4 b4 = *(const float4*)(K->bias + c);
+                                o[c / 2] = __hmax2(
+                                    __floats2bfloat162_rn(__uint_as_float(acc[c]) + b4.x,
+                                                          __uint_as_float(acc[c + 1]) + b4.y),
+                                    zero2);
+                                o[c / 2 + 1] = __hmax2(
+                                    __floats2bfloat162_rn(__uint_as_float(acc[c + 2]) + b4.z,
+                                                          __uint_as_float(acc[c + 3]) + b4.w),
+                                    zero2);
+                            }
+                        } else {
+                            const __nv_bfloat16* m = (const __nv_bfloat16*)m4;
+#pragma unroll
+                            for (int c = 0; c < C; c += 2)
+                                o[c / 2] = __floats2bfloat162_rn(
+                                    __bfloat162float(m[c]) > 0.f ? __uint_as_float(acc[c]) : 0.f,
+                                    __bfloat162float(m[c + 1]) > 0.f ? __uint_as_float(acc[c + 1])
+                                                                     : 0.f);
+                        }
+#pragma unroll
+                        for (int q = 0; q < KCH; q++)
+                            *(uint4*)(out + o0 + q * qs) = ((const uint4*)o)[q];
+                    }
+                } else {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&K->acce[T % Y_ROWS]);
+                }
             }
         }
     }
+    // drain: every MMA issued has completed before TMEM is released
     __syncthreads();
-    if (warp == 4 * W3_NG + 1 && lane == 0) tc::commit(&K->drain);
+    if (warp > 4 * Y_NG) tc::commit_warp(&K->drain);
     if (!tc::mbar_wait(&K->drain, 0, WAIT_LIMIT)) tc::mbar_wait(&K->drain, 0, WAIT_LIMIT);
     tc::fence_before();
     __syncthreads();
@@ -628,7 +495,7 @@ __global__ void __launch_bounds__(W3_THREADS, 1) conv32_w3_kernel(
 // (zero outside the patch), nine coalesced loads in a fixed order.  Pass 1:
 // a producer lane loads the strips into a ring of LR_STAGE stages, an issuer
 // lane runs the MMAs into one of two TMEM accumulators, four epilogue warps
-// store the nine planes of q; waits bounded as in conv32_walk_kernel.
+// store the nine planes of q; waits bounded as in conv32_ys_kernel.
 constexpr int LR_STAGE = 6;
 constexpr int LR_THREADS = 192;
 
@@ -817,7 +684,8 @@ template <int EPI>
 __global__ void __launch_bounds__(128) conv1_kernel(Dims d, WalkPlan wp, const float* __restrict__ in,
                                                     float scale,
                                                     const __nv_bfloat16* __restrict__ wpk,
-                                                    const float* __restrict__ bias, void* out,
+                                                    const float* __restrict__ bias,
+                                                    __nv_bfloat16* __restrict__ out,
                                                     const __nv_bfloat16* __restrict__ mask,
                                                     int* status) {
     __shared__ __align__(1024) uint8_t sW[C * C * 2];
@@ -837,8 +705,8 @@ __global__ void __launch_bounds__(128) conv1_kernel(Dims d, WalkPlan wp, const f
     int ntile = 0;
     int ncommit = 0;
     bool ok = true;
-    const int force_at = status[1] - 1;  // test hook, as in conv32_walk_kernel
-    // Tiles in runs of rows along y (the items of conv32_walk_kernel), so
+    const int force_at = status[1] - 1;  // test hook, as in conv32_ys_kernel
+    // Tiles in runs of rows along y (the items of conv32_ys_kernel), so
     // that consecutive tiles of a CTA share six of their nine input rows.
     struct Pos {
         int64_t it;
@@ -1278,7 +1146,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgrad_tc_kernel(
 // outside the row), so that with K = x' the input strips are B unshifted (rows
 // (strip, i)) and A (M = 128) is the gradient strip in three copies, copy c
 // staged from x0 + 1 - c (rows (c, o); copy 3 is zeros): D[(dx, o)][(strip, i)].
-// The staging is shared between neighbouring rows, as in conv32_walk_kernel: a CTA takes runs of L rows y of
+// The staging is shared between neighbouring rows, as in conv32_ys_kernel: a CTA takes runs of L rows y of
 // one (patch, z, x tile) column; the input strips come as row-sets (the strips
 // of one input row in planes z - 1, z, z + 1) through a ring of GW_R slots, each
 // row-set loaded once for the three K blocks (output rows) that read it.  Per
@@ -1565,6 +1433,13 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
 // mode 4: forward of the 1-output layer in row passes: per dx one 16 x 32
 //         block, row n = (dz, dy) = 3 dz + dy (n < 9), k = i, from
 //         W[9 dz + 3 dy + dx][0][i].
+// The 27 taps t = 9 dz + 3 dy + dx of modes 0 and 1 stand in the order of
+// conv32_ys_kernel: per (dz, dx) the taps dy = 2, 1, 0 one after another.
+__host__ __device__ inline int hid_tap(int t) {
+    const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
+    return (dz * 3 + dx) * 3 + (2 - dy);
+}
+
 __global__ void pack_kernel(const float* __restrict__ w, int mode, int NI, int NO, int NOUT,
                             __nv_bfloat16* __restrict__ out) {
     const int per_tap = NOUT * C;
@@ -1575,11 +1450,11 @@ __global__ void pack_kernel(const float* __restrict__ w, int mode, int NI, int N
         if (mode == 0) {
             const int t = e / per_tap, r = e % per_tap, n = r / C, k = r % C;
             if (n < NO && k < NI) v = w[((int64_t)t * NO + n) * NI + k];
-            dst = t * per_tap + bpk_index(n, k);
+            dst = hid_tap(t) * per_tap + bpk_index(n, k);
         } else if (mode == 1) {
             const int t = e / per_tap, r = e % per_tap, n = r / C, k = r % C;
             if (n < NI && k < NO) v = w[((int64_t)(26 - t) * NO + k) * NI + n];
-            dst = t * per_tap + bpk_index(n, k);
+            dst = hid_tap(t) * per_tap + bpk_index(n, k);
         } else if (mode == 2) {
             const int n = e / C, k = e % C;
             if (k < 27 && n < NO) v = w[((int64_t)k * NO + n) * NI + 0];
@@ -1758,56 +1633,40 @@ static bool act_maps(const Dims& d, const __nv_bfloat16* in, ActMaps* m) {
     return one(&m->lo, box_lo) && one(&m->hi, box_hi);
 }
 
-template <int NOUT, int EPI>
+template <int EPI>
 static nr_status launch_conv32(const Dims& d, const __nv_bfloat16* in, const __nv_bfloat16* wpk,
-                               const float* bias, void* out, const __nv_bfloat16* mask,
+                               const float* bias, __nv_bfloat16* out, const __nv_bfloat16* mask,
                                int* status, cudaStream_t s) {
-    ActMaps map;
-    if (!act_maps(d, in, &map)) return NR_ERR_CUDA;  // the input cannot be described for TMA
-    // runs of L rows: about eight items per SM, L in [4, 32]
-    const int nsm = sm_count();
-    const int64_t ncols = (int64_t)d.nb * d.nz * xtiles(d);
-    int64_t L = ((int64_t)d.ny * ncols + 8LL * nsm - 1) / (8LL * nsm);
-    L = L < 4 ? 4 : (L > 32 ? 32 : L);
-    if (L > d.ny) L = d.ny;
+    // Runs of L rows, each L + 2 steps: the number of runs per column whose
+    // busiest CTA has the fewest steps (few columns want short runs that fill
+    // the GPU, many want long ones).
+    const int64_t nsm = sm_count();
+    const int64_t ncols = (int64_t)d.nb * ((d.nz + 1) / 2) * xtiles(d);
     WalkPlan wp;
-    wp.L = (int)L;
-    wp.nchunk = (int)((d.ny + L - 1) / L);
-    const int grid_max = nsm;
-    // The dx-stacked kernel costs about 0.6 of the other per row of tiles
-    // (whole network on 512 x 60 planes: 1.46 against 2.36 ms at one tile per
-    // row, nx = 126 / 128; 2.73 against 4.60 ms at two, nx = 252 / 256) but
-    // needs ceil(nx / 126) tiles per row: it is used when that is cheaper
-    // (not for nx = 128, where two of its tiles cost 2.73 ms against 2.36).
-    const int t126 = (d.nx + W3_TW - 1) / W3_TW, t128 = (d.nx + TM - 1) / TM;
-    if (60 * t126 < 100 * t128) {
-        wp.tw = W3_TW;
-        wp.nitems = (int64_t)d.nb * d.nz * t126 * wp.nchunk;
-        const size_t smem = (size_t)W_R * W_SET + 27 * NOUT * C * 2 + sizeof(W3Ctl);
-        if (cudaFuncSetAttribute(conv32_w3_kernel<NOUT, EPI>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return NR_ERR_CUDA;
-        const int grid = (int)(wp.nitems < (int64_t)grid_max ? wp.nitems : (int64_t)grid_max);
-        conv32_w3_kernel<NOUT, EPI><<<grid, W3_THREADS, smem, s>>>(d, wp, map.lo, map.hi, wpk,
-                                                                   bias, out, mask, status);
-        return launch_status();
+    int64_t best = INT64_MAX;
+    for (int nchunk = 1; nchunk <= d.ny && nchunk <= 64; nchunk++) {
+        const int64_t L = (d.ny + nchunk - 1) / nchunk, n = (d.ny + L - 1) / L;
+        const int64_t steps = (ncols * n + nsm - 1) / nsm * (L + 2);
+        if (steps < best) {
+            best = steps;
+            wp.L = (int)L;
+            wp.nchunk = (int)n;
+        }
     }
     wp.tw = TM;
-    wp.nitems = (int64_t)d.nb * d.nz * t128 * wp.nchunk;
-    const size_t smem = (size_t)W_R * W_SET + 27 * NOUT * C * 2 + sizeof(WalkCtl);
-    if (cudaFuncSetAttribute(conv32_walk_kernel<NOUT, EPI>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    wp.nitems = ncols * wp.nchunk;
+    const size_t smem = (size_t)Y_R * Y_SET + Y_WBYTES + sizeof(YCtl);
+    if (cudaFuncSetAttribute(conv32_ys_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess)
         return NR_ERR_CUDA;
-    const int grid = (int)(wp.nitems < (int64_t)grid_max ? wp.nitems : (int64_t)grid_max);
-    conv32_walk_kernel<NOUT, EPI><<<grid, W_THREADS, smem, s>>>(d, wp, map.lo, map.hi, wpk, bias,
-                                                                out, mask, status);
+    const int grid = (int)(wp.nitems < nsm ? wp.nitems : nsm);
+    conv32_ys_kernel<EPI><<<grid, Y_THREADS, smem, s>>>(d, wp, in, wpk, bias, out, mask, status);
     return launch_status();
 }
 
 template <int EPI>
 static nr_status launch_conv1(const Dims& d, const float* in, float scale,
-                              const __nv_bfloat16* wpk, const float* bias, void* out,
+                              const __nv_bfloat16* wpk, const float* bias, __nv_bfloat16* out,
                               const __nv_bfloat16* mask, int* status, cudaStream_t s) {
     // four CTAs per SM (nine, as many as fit, measured 2.7x slower on the
     // clinical volume), each walking runs of L rows: about eight runs per CTA
@@ -1873,7 +1732,7 @@ static nr_status forward(const Dims& d, const float* params, const float* x, flo
     if ((e = launch_conv1<EPI_RELU>(d, x, s, pkf(0), params + bo[0], act(0), nullptr, status, st)) != NR_OK)
         return e;
     for (int l = 1; l < 5; l++)
-        if ((e = launch_conv32<C, EPI_RELU>(d, act(l - 1), pkf(l), params + bo[l], act(l), nullptr,
+        if ((e = launch_conv32<EPI_RELU>(d, act(l - 1), pkf(l), params + bo[l], act(l), nullptr,
                                             status, st)) != NR_OK)
             return e;
     // q of the last layer: a buffer idle by now (the gradient buffer when the
@@ -1976,7 +1835,7 @@ static nr_status loss_grad(const Dims& d, const float* params, const float* x, c
     // layers 5..2: dpre_l lives in dpre(l-1)
     for (int l = 4; l >= 1; l--) {
         if ((e = wgrad(d, l, dpre(l), act(l - 1), 1.f, ws, L, grad, status, st)) != NR_OK) return e;
-        if ((e = launch_conv32<C, EPI_MASK>(d, dpre(l), pkb(l), nullptr, dpre(l - 1), act(l - 1),
+        if ((e = launch_conv32<EPI_MASK>(d, dpre(l), pkb(l), nullptr, dpre(l - 1), act(l - 1),
                                             status, st)) != NR_OK)
             return e;
     }

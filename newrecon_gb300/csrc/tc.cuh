@@ -86,6 +86,31 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// The same issued by a whole (converged) warp, of which one elected lane -- the
+// same one each time -- performs it.  With warp-uniform operands the
+// descriptors stay in uniform registers: issued from inside a one-lane branch
+// they are moved there one word at a time, about 96 cycles per MMA in a
+// sequence with compile-time offsets.  Descriptors as two words: an offset in
+// bytes / 16 adds to the low one.
+__device__ __forceinline__ void mma_bf16_warp(uint32_t tmem_d, uint32_t alo, uint32_t ahi,
+                                              uint32_t blo, uint32_t bhi, uint32_t idesc,
+                                              uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n .reg .b64 a, b;\n elect.sync _|q, 0xffffffff;\n"
+        " setp.ne.b32 p, %6, 0;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n}\n" ::"r"(tmem_d),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate));
+}
+
+// commit() by the elected lane of a whole warp.
+__device__ __forceinline__ void commit_warp(uint64_t* bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(
+            smem_u32(bar))
+        : "memory");
+}
+
 // Arrives on the barrier once every tensor-core operation issued so far by
 // this thread has completed.
 __device__ __forceinline__ void commit(uint64_t* bar) {
