@@ -148,7 +148,8 @@ typedef struct nr_ostr_params {
     float beta;                /* penalty weight                                 */
     float delta;               /* potential scale (1/mm), > 0 unless Q2          */
     int32_t fp_batch;          /* Siddon steps per gather round: 2, 4, 8 (0 = 4) */
-    int32_t upd_planes;        /* z planes per update block: 8, 16, 32 (0 = 16) */
+    int32_t upd_planes;        /* z planes per update block: 8, 16, 32 (0: 16, or
+                                  fewer for a volume that would not fill the GPU) */
     int32_t fp_stage;          /* NR_STAGE_OFF (default): the projection gathers
                                   the volume through L1/L2; NR_STAGE_TMA: it stages
                                   the volume slab by slab in shared memory by TMA
@@ -156,16 +157,13 @@ typedef struct nr_ostr_params {
                                   4, x 16-byte aligned; fp_batch 2 or 4).  Same
                                   result either way; on the clinical workload the
                                   staged form is slower (0.255 vs 0.162 ms).     */
-    int32_t upd_tile;          /* NR_TILE_1 (default): the update gives each thread
-                                  one voxel of a 32 x 8-column tile; NR_TILE_2: two
-                                  voxels side by side in x of a 64 x 8-column tile
-                                  (one-view subsets; others use NR_TILE_1).  Same
-                                  result bit for bit; fewer instructions per voxel,
-                                  fewer resident blocks.  NR_TILE_TMA: the
-                                  one-voxel tile with its planes streamed by TMA
-                                  through a shared-memory ring by a producer warp
-                                  (IMGSIZx a multiple of 4 and x 16-byte aligned,
-                                  else NR_TILE_1); same result bit for bit.       */
+    int32_t upd_tile;          /* NR_TILE_1 (default) and NR_TILE_2: each thread of
+                                  the update owns two voxels, one above the other
+                                  in y, of a 32 x 8-column tile.  NR_TILE_TMA: one
+                                  voxel per thread, the planes streamed by TMA
+                                  through a shared-memory ring (IMGSIZx a multiple
+                                  of 4 and x 16-byte aligned, else NR_TILE_1); same
+                                  result bit for bit.                             */
 } nr_ostr_params;
 
 enum {
@@ -479,7 +477,7 @@ typedef struct nr_sart_params {
     int32_t use_cos;           /* 1: the _cos projector, 0: plain line integrals */
     int32_t regularized;       /* 1: prior_GPU_SART + backprj_OSSART_R           */
     int32_t fp_batch;          /* Siddon steps per gather round: 2, 4, 8 (0 = 4) */
-    int32_t upd_planes;        /* z planes per update block: 8, 16, 32 (0 = 16) */
+    int32_t upd_planes;        /* z planes per update block: 8, 16, 32 (0: by size) */
     float lambda;              /* relaxation                                     */
     float beta;                /* prior weight (regularized only; see the sign note above) */
     float delta;               /* hyperbola scale, != 0 (regularized only)      */

@@ -9,13 +9,11 @@ computes the same result, bit for bit):
   volume staged slab by slab in shared memory by TMA (``fp_stage``), where
   the geometry allows it;
 * ``upd_planes`` -- z planes walked per block by the fused update (8, 16, 32):
-  deeper slabs amortise the halo planes, shallower ones give more blocks;
-  tried with each update tile (``upd_tile``: one voxel per thread; two side
-  by side in x, with fewer instructions per voxel but fewer resident blocks,
-  when the subsets hold one view each; or one voxel per thread with the
-  planes streamed by TMA through a ring filled by a producer warp, where the
-  volume's rows allow TMA); a tile other than the default one voxel per
-  thread must win by ``TILE_MARGIN``.
+  deeper slabs amortise the planes beside the slab, shallower ones give more
+  blocks; tried with each update tile (``upd_tile``: two voxels per thread
+  walking the planes in registers; or one voxel per thread with the planes
+  streamed by TMA through a ring, where the volume's rows allow TMA); a tile
+  other than the default must win by ``TILE_MARGIN``.
 
 The tuner times each variant on the plan's own geometry (CUDA events on the
 launching stream, best of a few repetitions over all subsets) and keeps the
@@ -36,11 +34,11 @@ FP_BATCHES = (2, 4, 8)
 # batch, TMA-staged slabs for 2 and 4
 FP_VARIANTS = ((2, 0), (4, 0), (8, 0), (2, 1), (4, 1))
 UPD_PLANES = (8, 16, 32)
-UPD_TILES = (0, 1, 2)  # NR_TILE_1, NR_TILE_2, NR_TILE_TMA
-TILE_NAMES = {0: "", 1: "-x2", 2: "-tma"}
-# A tile other than the default one-voxel tile is kept only when it beats the
-# best one-voxel variant by this fraction: near a tie the choice would
-# otherwise follow the timing noise from run to run.
+UPD_TILES = (0, 2)  # NR_TILE_1, NR_TILE_TMA (NR_TILE_2 runs NR_TILE_1's kernel)
+TILE_NAMES = {0: "", 2: "-tma"}
+# A tile other than the default is kept only when it beats the default's best
+# variant by this fraction: near a tie the choice would otherwise follow the
+# timing noise from run to run.
 TILE_MARGIN = 0.02
 
 
@@ -54,7 +52,7 @@ def signature(plan) -> str:
     p = plan.params
     dev = torch.cuda.get_device_name(plan.ws.device)
     return (f"{dev}|{g.nx}x{g.ny}x{g.nz}|{g.nbx}x{g.nby}|A{g.n_angles}|M{p.subset_num}"
-            f"|pot{p.potential}|scat{p.has_scatter}|v4")
+            f"|pot{p.potential}|scat{p.has_scatter}|v5")
 
 
 def _load() -> Dict[str, dict]:
@@ -95,8 +93,8 @@ def _time(fn, reps: int) -> float:
 
 def choose_update(up_ms: Dict[Tuple[int, int], float]) -> Tuple[int, int]:
     """(upd_tile, upd_planes) from the timings of the update variants: the
-    fastest, except that a tile other than the one-voxel tile (0) must beat
-    the fastest one-voxel variant by TILE_MARGIN."""
+    fastest, except that a tile other than the default (0) must beat the
+    default's fastest variant by TILE_MARGIN."""
     best_t, best_z = min(up_ms, key=up_ms.get)
     if best_t != 0:
         z1 = min((z for t, z in up_ms if t == 0), key=lambda z: up_ms[(0, z)])
@@ -110,7 +108,7 @@ def apply_cached(plan) -> Optional[dict]:
     None (and the plan unchanged) when the cache holds none."""
     hit = _load().get(signature(plan))
     if not (hit and hit.get("fp_batch") in FP_BATCHES and hit.get("upd_planes") in UPD_PLANES
-            and hit.get("fp_stage", 0) in (0, 1) and hit.get("upd_tile", 0) in UPD_TILES):
+            and hit.get("fp_stage", 0) in (0, 1) and hit.get("upd_tile", 0) in (0, 1, 2)):
         return None
     plan.params.fp_batch = int(hit["fp_batch"])
     plan.params.upd_planes = int(hit["upd_planes"])
@@ -133,7 +131,6 @@ def tune(plan, x: Optional[torch.Tensor] = None, reps: int = 3,
     xo = torch.empty_like(x)
     M = plan.params.subset_num
     saved = (plan.params.fp_batch, plan.params.upd_planes, plan.params.fp_stage)
-    one_view = plan.geom.n_angles == M  # the two-voxel tile serves one-view subsets
     fp_ms, up_ms = {}, {}
     for k, st in FP_VARIANTS:
         plan.params.fp_batch = k
@@ -142,7 +139,7 @@ def tune(plan, x: Optional[torch.Tensor] = None, reps: int = 3,
         fp_ms[(k, st)] = _time(lambda: [plan.project(x, a) for a in range(M)], reps)
     plan.params.fp_batch, plan.params.fp_stage = saved[0], saved[2]
     plan.project(x, 0)  # h of subset 0 for the update timings
-    for t in (UPD_TILES if one_view else (0, 2)):
+    for t in UPD_TILES:
         for z in UPD_PLANES:
             plan.params.upd_tile = t
             plan.params.upd_planes = z

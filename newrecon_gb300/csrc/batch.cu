@@ -25,11 +25,9 @@
 // 64 cases: ~19 KB, inside the 32 KB parameter limit).  The item decode then
 // runs on block-uniform constant-bank values and the tile reads its case's
 // geometry from the constant bank as the single-case kernels do, instead of
-// from a shared-memory copy that costs registers: the one-voxel one-view
-// update fits 32 registers (8 resident blocks per SM; 8 bytes spill).
+// from a shared-memory copy that costs registers.
 #include <cstdint>
 #include <cstring>
-#include <type_traits>
 
 #include "project.cuh"
 #include "update.cuh"
@@ -38,9 +36,7 @@ namespace nr {
 
 constexpr int BATCH_MAX = 64;
 constexpr int N_ZC = 3;                      // update slab depths 8, 16, 32 planes
-// update forms: several views per subset; one view, one voxel per thread;
-// one view, two voxels per thread (the case's upd_tile)
-constexpr int N_FORM = 3;
+constexpr int N_FORM = 2;                    // several views per subset; one view
 constexpr int N_CLASSES = 4 * N_FORM * N_ZC; // potential x form x slab depth
 
 struct CaseDev {
@@ -56,16 +52,13 @@ struct CaseDev {
     int* status;
     BpTab T;               // the case's back-projection tables
     int fp_tx, fp_ty;      // detector tiles of 32 x 4 bins
-    int up_tx, up_ty;      // volume tiles of 32 x 8 columns (64 x 8 in form 2)
+    int up_tx, up_ty;      // volume tiles of 32 x 8 columns
     int form;              // update form (N_FORM)
     int zc;                // z planes per update item (the plan's upd_planes)
     int64_t N;
 };
 
 __host__ __device__ constexpr int zc_index(int zc) { return zc == 8 ? 0 : (zc == 32 ? 2 : 1); }
-__host__ __device__ constexpr int upd_form(bool one_view, int tile) {
-    return one_view ? (tile == NR_TILE_2 ? 2 : 1) : 0;
-}
 __host__ __device__ constexpr int upd_class(int pot, int form, int zc) {
     return (N_FORM * pot + form) * N_ZC + zc_index(zc);
 }
@@ -109,45 +102,33 @@ __global__ void __launch_bounds__(128, 12) fp_batch_kernel(const __grid_constant
     }
 }
 
-// Update items [lo, hi) of one (potential, NV, ZC, X2) class.  NV = 1 serves
-// the cases whose subsets hold one view (the compile-time view count of
-// update_tile: 32 registers, 8 resident blocks per SM); NV = 0 the others
-// (no block minimum, as update_kernel: 40 registers).  X2: the one-view
-// cases that take two voxels per thread (update_tile_x2, 5 blocks per SM as
-// update_x2_kernel).  ZC is the case's slab depth (planes per item), as the
-// autotuner picked it.
-template <int POT, int NV, int ZC, bool X2>
-__global__ void __launch_bounds__(256, NV ? (X2 ? 5 : 8) : 0) update_batch_kernel(
-    const __grid_constant__ BatchTable P, int step, int lo, int hi) {
-    __shared__ typename std::conditional<X2, UpdSmem2, UpdSmem>::type sm;
-    for (int it = lo + blockIdx.x; it < hi; it += gridDim.x) {
-        const int c = find_case(P.up_off, P.n, it);
-        const CaseDev& cd = P.c[c];
-        __syncthreads();  // previous item's readers of sm are done
-        if (step >= cd.total_sub) continue;
-        const int local = it - P.up_off[c];
-        const int bx = local % cd.up_tx;
-        const int by = (local / cd.up_tx) % cd.up_ty;
-        const int bz = local / (cd.up_tx * cd.up_ty);
-        const int a0 = (step % (int)cd.M) * cd.Vs;
-        const float* cur = (step & 1) ? cd.xtmp : cd.x;
-        float* nxt = (step & 1) ? cd.x : cd.xtmp;
-        // The tile reads its case's values from locals copied once per item:
-        // read through the runtime case index, they were fetched again on
-        // every plane (8 % more instructions than the single-case kernel,
-        // whose fixed constant-bank offsets are free operands).
-        const Geo G = cd.G;
-        const PriorW5 W = cd.W;
-        const BpTab T = cd.T;
-        if constexpr (X2)
-            update_tile_x2<POT, ZC, UPD_OSTR, NV>(G, W, cur, nxt, cd.d, cd.h, cd.angles, cd.index,
-                                                  T, a0, cd.Vs, cd.M, cd.beta, cd.delta,
-                                                  cd.status, bx, by, bz, sm);
-        else
-            update_tile<POT, ZC, UPD_OSTR, NV>(G, W, cur, nxt, cd.d, cd.h, cd.angles, cd.index, T,
-                                                a0, cd.Vs, cd.M, cd.beta, cd.delta, cd.status, bx,
-                                                by, bz, sm);
-    }
+// Update items [lo, hi) of one (potential, NV, ZC) class.  NV = 1 serves the
+// cases whose subsets hold one view (the compile-time view count of
+// update_tile), NV = 0 the others.  ZC is the case's slab depth (planes per
+// item), as the autotuner picked it.
+template <int POT, int NV, int ZC>
+__global__ void __launch_bounds__(UNT, UPD_BLOCKS) update_batch_kernel(
+    const __grid_constant__ BatchTable P, int step, int lo) {
+    const int it = lo + blockIdx.x;
+    const int c = find_case(P.up_off, P.n, it);
+    const CaseDev& cd = P.c[c];
+    if (step >= cd.total_sub) return;
+    const int local = it - P.up_off[c];
+    const int bx = local % cd.up_tx;
+    const int by = (local / cd.up_tx) % cd.up_ty;
+    const int bz = local / (cd.up_tx * cd.up_ty);
+    const int a0 = (step % (int)cd.M) * cd.Vs;
+    const float* cur = (step & 1) ? cd.xtmp : cd.x;
+    float* nxt = (step & 1) ? cd.x : cd.xtmp;
+    // The tile reads its case's values from locals copied once per item: read
+    // through the runtime case index, they were fetched again on every plane
+    // (8 % more instructions than the single-case kernel, whose fixed
+    // constant-bank offsets are free operands).
+    const Geo G = cd.G;
+    const PriorW5 W = cd.W;
+    const BpTab T = cd.T;
+    update_tile<POT, ZC, UPD_OSTR, NV>(G, W, cur, nxt, cd.d, cd.h, T, a0, cd.Vs, cd.M, cd.beta,
+                                       cd.delta, cd.status, bx, by, bz);
 }
 
 // Cases whose sub-iteration count is odd end in xtmp: copy them back to x.
@@ -219,8 +200,7 @@ NR_API nr_status nr_batch_prepare(const nr_batch_case* cases, int32_t n_cases, v
     auto zc_of = [&](int c) { return cases[c].p.upd_planes == 0 ? UZC : cases[c].p.upd_planes; };
     auto cls_of = [&](int c) {
         const nr_batch_case& k = cases[c];
-        return upd_class(k.p.potential, upd_form(k.g.n_angles == k.p.subset_num, k.p.upd_tile),
-                         zc_of(c));
+        return upd_class(k.p.potential, k.g.n_angles == k.p.subset_num ? 1 : 0, zc_of(c));
     };
     // case order: by class, then by sub-iteration count, longest first (stable)
     int order[BATCH_MAX];
@@ -260,8 +240,8 @@ NR_API nr_status nr_batch_prepare(const nr_batch_case* cases, int32_t n_cases, v
         d.x = k.x;
         d.fp_tx = (int)cdiv(g.nbx, 32);
         d.fp_ty = (int)cdiv(g.nby, 4);
-        d.form = upd_form(d.Vs == 1, k.p.upd_tile);
-        d.up_tx = (int)cdiv(g.nx, d.form == 2 ? U2X : UTX);
+        d.form = d.Vs == 1 ? 1 : 0;
+        d.up_tx = (int)cdiv(g.nx, UTX);
         d.up_ty = (int)cdiv(g.ny, UTY);
         d.zc = zc_of(order[c]);
         d.N = (int64_t)g.nx * g.ny * g.nz;
@@ -308,24 +288,22 @@ NR_API nr_status nr_batch_prepare(const nr_batch_case* cases, int32_t n_cases, v
 
 namespace {
 
-template <int POT, int NV, int ZC, bool X2>
-void launch_class_t(const BatchTable& P, int32_t k, int lo, int hi, cudaStream_t s) {
-    update_batch_kernel<POT, NV, ZC, X2><<<hi - lo, dim3(UTX, UTY), 0, s>>>(P, k, lo, hi);
-}
-
-template <int POT, int NV, bool X2>
+template <int POT, int NV>
 void launch_class_z(int zi, const BatchTable& P, int32_t k, int lo, int hi, cudaStream_t s) {
-    if (zi == 0) return launch_class_t<POT, NV, 8, X2>(P, k, lo, hi, s);
-    if (zi == 2) return launch_class_t<POT, NV, 32, X2>(P, k, lo, hi, s);
-    return launch_class_t<POT, NV, 16, X2>(P, k, lo, hi, s);
+    const dim3 blk(UTX, UTY / 2);
+    if (zi == 0)
+        update_batch_kernel<POT, NV, 8><<<hi - lo, blk, 0, s>>>(P, k, lo);
+    else if (zi == 2)
+        update_batch_kernel<POT, NV, 32><<<hi - lo, blk, 0, s>>>(P, k, lo);
+    else
+        update_batch_kernel<POT, NV, 16><<<hi - lo, blk, 0, s>>>(P, k, lo);
 }
 
 template <int POT>
 void launch_class_form(int form, int zi, const BatchTable& P, int32_t k, int lo, int hi,
                        cudaStream_t s) {
-    if (form == 2) return launch_class_z<POT, 1, true>(zi, P, k, lo, hi, s);
-    if (form == 1) return launch_class_z<POT, 1, false>(zi, P, k, lo, hi, s);
-    return launch_class_z<POT, 0, false>(zi, P, k, lo, hi, s);
+    if (form == 1) return launch_class_z<POT, 1>(zi, P, k, lo, hi, s);
+    return launch_class_z<POT, 0>(zi, P, k, lo, hi, s);
 }
 
 void launch_class(int cls, const BatchTable& P, int32_t k, int lo, int hi, cudaStream_t s) {

@@ -30,15 +30,14 @@ nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const f
 nr_status launch_bp(const nr_geom& g, bool ji, float* vol, const float* prj, const float* angles,
                     const int32_t* index, int a0, int nv, cudaStream_t st);
 nr_status launch_update(const nr_geom& g, int pot, int zc, int tile, const float* x, float* x_out,
-                        const float* d, const float* h, const float* angles, const int32_t* index,
-                        const BpTab& T, int a0, int nv, float M, float beta, float delta,
+                        const float* d, const float* h, const BpTab& T, int a0, int nv, float M, float beta, float delta,
                         int* status, const CUtensorMap* map, cudaStream_t st);
 bool volume_map_nan(const nr_geom& g, const float* x, int bx, int by, int bz, CUtensorMap* map);
 
 // The TMA descriptor the update's NR_TILE_TMA form reads volume x through
 // (its planes with halo, NaN outside the volume); false when the volume
 // cannot be described (IMGSIZx not a multiple of 4, x not 16-byte aligned),
-// and the update then runs the one-voxel tile instead.
+// and the update then runs the default tile instead.
 static bool update_map(const nr_geom& g, const nr_ostr_params& p, const float* x,
                        CUtensorMap* map) {
     return p.upd_tile == NR_TILE_TMA && volume_map_nan(g, x, UTW, USH, 1, map);
@@ -289,8 +288,7 @@ NR_API nr_status nr_ostr_update(const nr_geom* g, const nr_ostr_params* p, const
     const int M = p->subset_num, Vs = g->n_angles / M;
     CUtensorMap map;
     const bool mapped = update_map(*g, *p, x, &map);
-    return launch_update(*g, p->potential, p->upd_planes, p->upd_tile, x, x_out, w.d, w.h,
-                         w.angles, w.index, w.tab(), subset * Vs, Vs, (float)M, p->beta, p->delta,
+    return launch_update(*g, p->potential, p->upd_planes, p->upd_tile, x, x_out, w.d, w.h, w.tab(), subset * Vs, Vs, (float)M, p->beta, p->delta,
                          w.status, mapped ? &map : nullptr, as_stream(stream));
 }
 
@@ -330,8 +328,7 @@ NR_API nr_status nr_ostr_subiter(const nr_geom* g, const nr_ostr_params* p, floa
         return st;
     CUtensorMap map;
     const bool mapped = update_map(*g, *p, x, &map);
-    if ((st = launch_update(*g, p->potential, p->upd_planes, p->upd_tile, x, w.xtmp, w.d, w.h,
-                            w.angles, w.index, w.tab(), a0, Vs, (float)M, p->beta, p->delta,
+    if ((st = launch_update(*g, p->potential, p->upd_planes, p->upd_tile, x, w.xtmp, w.d, w.h, w.tab(), a0, Vs, (float)M, p->beta, p->delta,
                             w.status, mapped ? &map : nullptr, s)) != NR_OK)
         return st;
     if (cudaMemcpyAsync(x, w.xtmp, N * sizeof(float), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -362,7 +359,7 @@ static nr_status enqueue_iterations(const nr_geom* g, const nr_ostr_params* p, f
                 NR_OK)
                 return st;
             if ((st = launch_update(*g, p->potential, p->upd_planes, p->upd_tile, cur, nxt, w.d,
-                                    w.h, w.angles, w.index, w.tab(), a0, Vs, (float)M, p->beta,
+                                    w.h, w.tab(), a0, Vs, (float)M, p->beta,
                                     p->delta, w.status,
                                     umapped ? &umaps[cur == x ? 0 : 1] : nullptr, s)) != NR_OK)
                 return st;

@@ -154,13 +154,14 @@ __global__ void __launch_bounds__(128) bp_table_kernel(const __grid_constant__ G
     const float z1 = vox_z(g, z);
     const float tt = bp_tt(g, src, z1);
     const float inv_bx = 1.f / g.bx, inv_by = 1.f / g.by;
+    const float k = __fdiv_rn(1.f, g.vz * src.s2);
     const int64_t row = (int64_t)a * g.nz + z;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.nx + g.ny;
          q += gridDim.x * blockDim.x) {
         if (q < g.nx)
-            tx[row * g.nx + q] = bp_entry_x(g, src, tt, q, inv_bx);
+            tx[row * g.nx + q] = bp_entry_x(g, src, tt, q, inv_bx, k);
         else
-            ty[row * g.ny + (q - g.nx)] = bp_entry_y(g, src, z1, tt, q - g.nx, inv_by);
+            ty[row * g.ny + (q - g.nx)] = bp_entry_y(g, src, z1, tt, q - g.nx, inv_by, k);
     }
 }
 
@@ -177,70 +178,71 @@ nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t*
 
 template <int POT, int ZC>
 static nr_status launch_update_t(const nr_geom& g, int tile, const float* x, float* x_out, const float* d,
-                                 const float* h, const float* angles, const int32_t* index,
-                                 const BpTab& T, int a0, int nv, float M, float beta,
+                                 const float* h, const BpTab& T, int a0, int nv, float M, float beta,
                                  float delta, int* status, const CUtensorMap* map,
                                  cudaStream_t st) {
-    dim3 blk(UTX, UTY), grd(cdiv(g.nx, UTX), cdiv(g.ny, UTY), cdiv(g.nz, ZC));
+    dim3 grd(cdiv(g.nx, UTX), cdiv(g.ny, UTY), cdiv(g.nz, ZC));
     const Geo G = make_geo(g);
     const PriorW5 W = make_w5(g.vz / g.vx, delta);
     if (tile == NR_TILE_TMA && map) {
+        dim3 blk(UTX, UTY);
         if (nv == 1)
-            update_tma_kernel<POT, ZC, 1><<<grd, blk, 0, st>>>(
-                G, W, *map, x_out, d, h, angles, index, T, a0, nv, M, beta, delta, status);
+            update_tma_kernel<POT, ZC, 1><<<grd, blk, 0, st>>>(G, W, *map, x_out, d, h, T, a0, nv, M,
+                                                               beta, delta, status);
         else
-            update_tma_kernel<POT, ZC, 0><<<grd, blk, 0, st>>>(
-                G, W, *map, x_out, d, h, angles, index, T, a0, nv, M, beta, delta, status);
-    } else if (nv == 1 && tile == NR_TILE_2) {
-        dim3 g2(cdiv(g.nx, U2X), cdiv(g.ny, UTY), cdiv(g.nz, ZC));
-        update_x2_kernel<POT, ZC, 1><<<g2, blk, 0, st>>>(G, W, x, x_out, d, h, angles, index, T, a0,
-                                                       nv, M, beta, delta, status);
-    } else if (nv == 1)
-        update_kernel<POT, ZC, 1><<<grd, blk, 0, st>>>(G, W, x, x_out, d, h, angles, index, T, a0,
-                                                       nv, M, beta, delta, status);
+            update_tma_kernel<POT, ZC, 0><<<grd, blk, 0, st>>>(G, W, *map, x_out, d, h, T, a0, nv, M,
+                                                               beta, delta, status);
+        return launch_status();
+    }
+    dim3 blk(UTX, UTY / 2);
+    if (nv == 1)
+        update_kernel<POT, ZC, 1><<<grd, blk, 0, st>>>(G, W, x, x_out, d, h, T, a0, nv, M, beta,
+                                                       delta, status);
     else
-        update_kernel<POT, ZC, 0><<<grd, blk, 0, st>>>(G, W, x, x_out, d, h, angles, index, T, a0,
-                                                       nv, M, beta, delta, status);
+        update_kernel<POT, ZC, 0><<<grd, blk, 0, st>>>(G, W, x, x_out, d, h, T, a0, nv, M, beta,
+                                                       delta, status);
     return launch_status();
 }
 
 template <int POT>
 static nr_status launch_update_z(const nr_geom& g, int zc, int tile, const float* x, float* x_out,
-                                 const float* d, const float* h, const float* angles,
-                                 const int32_t* index, const BpTab& T, int a0, int nv, float M,
-                                 float beta, float delta, int* status, const CUtensorMap* map,
-                                 cudaStream_t st) {
-    switch (zc) {
+                                 const float* d, const float* h, const BpTab& T, int a0, int nv,
+                                 float M, float beta, float delta, int* status,
+                                 const CUtensorMap* map, cudaStream_t st) {
+    switch (zc ? zc : upd_planes_auto(g)) {
+    case 4:
+        return launch_update_t<POT, 4>(g, tile, x, x_out, d, h, T, a0, nv, M, beta, delta, status,
+                                       map, st);
     case 8:
-        return launch_update_t<POT, 8>(g, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta, delta,
-                                       status, map, st);
+        return launch_update_t<POT, 8>(g, tile, x, x_out, d, h, T, a0, nv, M, beta, delta, status,
+                                       map, st);
     case 32:
-        return launch_update_t<POT, 32>(g, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta, delta,
-                                        status, map, st);
+        return launch_update_t<POT, 32>(g, tile, x, x_out, d, h, T, a0, nv, M, beta, delta, status,
+                                        map, st);
     default:
-        return launch_update_t<POT, 16>(g, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta, delta,
-                                        status, map, st);
+        return launch_update_t<POT, 16>(g, tile, x, x_out, d, h, T, a0, nv, M, beta, delta, status,
+                                        map, st);
     }
 }
 
 nr_status launch_update(const nr_geom& g, int pot, int zc, int tile, const float* x, float* x_out,
-                        const float* d, const float* h, const float* angles, const int32_t* index,
-                        const BpTab& T, int a0, int nv, float M, float beta, float delta,
-                        int* status, const CUtensorMap* map, cudaStream_t st) {
-    if (nv > UPD_VIEWS_SMEM) return NR_ERR_BAD_ARGUMENT;
+                        const float* d, const float* h, const BpTab& T, int a0, int nv, float M,
+                        float beta, float delta, int* status, const CUtensorMap* map,
+                        cudaStream_t st) {
+    if (nv > UPD_MAX_VIEWS) return NR_ERR_BAD_ARGUMENT;
     switch (pot) {
     case NR_POT_Q2:
-        return launch_update_z<NR_POT_Q2>(g, zc, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta,
-                                          delta, status, map, st);
+        return launch_update_z<NR_POT_Q2>(g, zc, tile, x, x_out, d, h, T, a0, nv, M, beta, delta,
+                                          status, map, st);
     case NR_POT_LANGE:
-        return launch_update_z<NR_POT_LANGE>(g, zc, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta,
-                                             delta, status, map, st);
+        return launch_update_z<NR_POT_LANGE>(g, zc, tile, x, x_out, d, h, T, a0, nv, M, beta, delta,
+                                             status, map, st);
     case NR_POT_HYPERBOLA:
-        return launch_update_z<NR_POT_HYPERBOLA>(g, zc, tile, x, x_out, d, h, angles, index, T, a0, nv, M,
-                                                 beta, delta, status, map, st);
+        return launch_update_z<NR_POT_HYPERBOLA>(g, zc, tile, x, x_out, d, h, T, a0, nv, M, beta,
+                                                 delta, status, map, st);
     case NR_POT_HUBER:
-        return launch_update_z<NR_POT_HUBER>(g, zc, tile, x, x_out, d, h, angles, index, T, a0, nv, M, beta,
-                                             delta, status, map, st);
+        return launch_update_z<NR_POT_HUBER>(g, zc, tile, x, x_out, d, h, T, a0, nv, M, beta, delta,
+                                             status, map, st);
     default: return NR_ERR_BAD_ARGUMENT;
     }
 }

@@ -17,7 +17,7 @@
 //                        projector) against their mean chord
 //   sart_update_kernel   the fused update tile of update.cuh in its OS-SART
 //                        kinds: sensitivity-normalised back projection, the
-//                        hyperbola prior from the 3-plane ring, the step and
+//                        hyperbola prior, the step and
 //                        the clamp, written to the second volume buffer
 // normprj -- the in-volume chord of each ray -- does not depend on x, so it
 // is traced once at set-up (the reference re-traces it with every FP).
@@ -103,7 +103,7 @@ nr_status sart_check_params(const nr_geom* g, const nr_sart_params* p) {
     if (!geom_ok(g)) return NR_ERR_BAD_GEOMETRY;
     if (!p) return NR_ERR_BAD_ARGUMENT;
     if (p->subset_num <= 0 || g->n_angles % p->subset_num != 0) return NR_ERR_BAD_GEOMETRY;
-    if (g->n_angles / p->subset_num > UPD_VIEWS_SMEM) return NR_ERR_BAD_ARGUMENT;
+    if (g->n_angles / p->subset_num > UPD_MAX_VIEWS) return NR_ERR_BAD_ARGUMENT;
     if (!(fabsf(p->lambda) < INFINITY) || !(fabsf(p->beta) < INFINITY)) return NR_ERR_BAD_ARGUMENT;
     if (p->regularized && (p->delta == 0.f || !(fabsf(p->delta) < INFINITY)))
         return NR_ERR_BAD_ARGUMENT;  // prior_GPU_SART exits on delta == 0 (Tomo_OSTR.cu:2260)
@@ -243,16 +243,14 @@ __global__ void __launch_bounds__(256) sart_fp_diff_4r_kernel(
 }
 
 template <int KIND, int ZC, int NV>
-__global__ void __launch_bounds__(256, NV == 1 ? 8 : 0) sart_update_kernel(
+__global__ void __launch_bounds__(UNT, UPD_BLOCKS) sart_update_kernel(
     const __grid_constant__ Geo G, const __grid_constant__ PriorW5 W,
     const float* __restrict__ x, float* __restrict__ x_out, const float* __restrict__ diff,
-    const float* __restrict__ angles, const int32_t* __restrict__ index,
     const __grid_constant__ BpTab T, int a0, int nv, float lambda, float beta, float delta,
     int* __restrict__ status) {
-    __shared__ UpdSmem sm;
-    update_tile<NR_POT_HYPERBOLA, ZC, KIND, NV>(G, W, x, x_out, nullptr, diff, angles, index, T,
-                                                a0, nv, lambda, beta, delta, status, blockIdx.x,
-                                                blockIdx.y, blockIdx.z, sm);
+    update_tile<NR_POT_HYPERBOLA, ZC, KIND, NV>(G, W, x, x_out, nullptr, diff, T, a0, nv, lambda,
+                                                beta, delta, status, blockIdx.x, blockIdx.y,
+                                                blockIdx.z);
 }
 
 namespace {
@@ -283,27 +281,26 @@ nr_status launch_fp_diff_c(const nr_geom& g, int k, const float* x, const SartWS
 template <int KIND, int ZC>
 nr_status launch_sart_update_t(const nr_geom& g, const nr_sart_params& p, const float* x,
                                float* x_out, const SartWS& w, int a0, int nv, cudaStream_t s) {
-    dim3 blk(UTX, UTY), grd(cdiv(g.nx, UTX), cdiv(g.ny, UTY), cdiv(g.nz, ZC));
+    dim3 blk(UTX, UTY / 2), grd(cdiv(g.nx, UTX), cdiv(g.ny, UTY), cdiv(g.nz, ZC));
     // unit neighbour distances: G_Huber_prior has no z ratio (Tomo_OSTR.cu:303)
     const float delta = p.regularized ? p.delta : 1.f;
     const Geo G = make_geo(g);
     const PriorW5 W = make_w5(1.f, delta);
     const BpTab T{w.bpx, w.bpy};
     if (nv == 1)
-        sart_update_kernel<KIND, ZC, 1><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, w.angles,
-                                                            w.index, T, a0, nv, p.lambda, p.beta,
-                                                            delta, w.status);
+        sart_update_kernel<KIND, ZC, 1><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, a0, nv,
+                                                            p.lambda, p.beta, delta, w.status);
     else
-        sart_update_kernel<KIND, ZC, 0><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, w.angles,
-                                                            w.index, T, a0, nv, p.lambda, p.beta,
-                                                            delta, w.status);
+        sart_update_kernel<KIND, ZC, 0><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, a0, nv,
+                                                            p.lambda, p.beta, delta, w.status);
     return launch_status();
 }
 
 template <int KIND>
 nr_status launch_sart_update_z(const nr_geom& g, const nr_sart_params& p, const float* x,
                                float* x_out, const SartWS& w, int a0, int nv, cudaStream_t s) {
-    switch (p.upd_planes) {
+    switch (p.upd_planes ? p.upd_planes : upd_planes_auto(g)) {
+    case 4: return launch_sart_update_t<KIND, 4>(g, p, x, x_out, w, a0, nv, s);
     case 8: return launch_sart_update_t<KIND, 8>(g, p, x, x_out, w, a0, nv, s);
     case 32: return launch_sart_update_t<KIND, 32>(g, p, x, x_out, w, a0, nv, s);
     default: return launch_sart_update_t<KIND, 16>(g, p, x, x_out, w, a0, nv, s);

@@ -8,16 +8,31 @@
 #pragma once
 
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tma.cuh"
 
 namespace nr {
 
-constexpr int UPD_VIEWS_SMEM = 32;
+constexpr int UPD_MAX_VIEWS = 32;               // views per subset
 constexpr int UTX = 32, UTY = 8, UZC = 16;      // tile: 32 x 8 columns, 16 planes per block
-constexpr int USW = UTX + 2, USH = UTY + 2;     // plane tile with a 1-voxel halo
-constexpr int UPLANE = USW * USH;
+constexpr int UNT = UTX * UTY / 2;              // threads of a block: two voxels each
+// Resident blocks per SM.  96 registers hold the walk without spills; per
+// sub-iteration of the clinical workload 5 blocks took 0.236 ms, 6 blocks (80
+// registers) 0.243, 4 blocks 0.246, 8 blocks (64 registers, 300 bytes of
+// spills) 0.27: fewer instructions win over more warps.
+constexpr int UPD_BLOCKS = 5;
+
+// Planes per block when the caller leaves the choice open: 16, or fewer when
+// that leaves SMs without their UPD_BLOCKS blocks (a 256 x 128 x 24 volume makes
+// 256 blocks of 16 planes, 768 of 4).
+__host__ inline int upd_planes_auto(const nr_geom& g) {
+    const int64_t tiles = (int64_t)((g.nx + UTX - 1) / UTX) * ((g.ny + UTY - 1) / UTY);
+    for (int zc = UZC; zc > 4; zc /= 2)
+        if (tiles * ((g.nz + zc - 1) / zc) >= 152 * UPD_BLOCKS) return zc;
+    return 4;
+}
 
 // The five distinct neighbour weights 1/sqrt(dx^2+dy^2+(dz zr)^2) of the
 // 26-neighbourhood (in-plane face, in-plane diagonal, z face, z edge, z
@@ -99,21 +114,12 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     return r;
 }
 
-// Weight class of neighbour K = ((dz+1)*3 + (dy+1))*3 + (dx+1).
-template <int K>
-__device__ __forceinline__ constexpr int nb_class() {
-    constexpr int dz = K / 9 - 1, dy = (K / 3) % 3 - 1, dx = K % 3 - 1;
-    constexpr int nxy = (dx != 0) + (dy != 0);
-    return dz == 0 ? (nxy == 1 ? W_FACE : W_DIAG)
-                   : (nxy == 0 ? W_ZFACE : (nxy == 1 ? W_ZEDGE : W_ZCORNER));
-}
-
-// The penalty terms of a packed pair of differences t2 of one weight class:
-// each lane adds w omega(t) to sdd and w omega(t) t to sd.  EDGE: a
-// difference with an out-of-volume cell (NaN) counts as t = 0.
-template <int POT, bool EDGE, int CLS>
-__device__ __forceinline__ void nb_terms(f32x2 t2, const PriorW5& W, float delta, float inv_delta,
-                                         f32x2& sdd, f32x2& sd) {
+// omega(t) of two differences of one potential, divided by delta for Huber
+// (min(1, delta/|t|) = delta / max(|t|, delta): the class factor carries the
+// delta).  EDGE: a difference with an out-of-volume cell (NaN) counts as t = 0.
+template <int POT, bool EDGE>
+__device__ __forceinline__ f32x2 omega2(f32x2& t2, const PriorW5& W, float delta,
+                                        float inv_delta) {
     float ta, tb;
     upk2(t2, ta, tb);
     if (EDGE) {
@@ -121,90 +127,69 @@ __device__ __forceinline__ void nb_terms(f32x2 t2, const PriorW5& W, float delta
         tb = (tb == tb) ? tb : 0.f;
         t2 = pk2(ta, tb);
     }
-    const f32x2 w2 = ld2(W.w[CLS]);
-    f32x2 wo2;
-    if (POT == NR_POT_Q2) {
-        wo2 = w2;
-    } else if (POT == NR_POT_LANGE) {
-        wo2 = mul2(w2, pk2(rcp_approx(__fmaf_rn(fabsf(ta), inv_delta, 1.f)),
-                           rcp_approx(__fmaf_rn(fabsf(tb), inv_delta, 1.f))));
-    } else if (POT == NR_POT_HYPERBOLA) {
+    if (POT == NR_POT_Q2) return ld2(W.one);
+    if (POT == NR_POT_LANGE)
+        return pk2(rcp_approx(__fmaf_rn(fabsf(ta), inv_delta, 1.f)),
+                   rcp_approx(__fmaf_rn(fabsf(tb), inv_delta, 1.f)));
+    if (POT == NR_POT_HYPERBOLA) {
         const f32x2 u2 = mul2(t2, ld2(W.inv_delta));
         float qa, qb;
         upk2(fma2(u2, u2, ld2(W.one)), qa, qb);
-        wo2 = mul2(w2, pk2(rsqrt_approx(qa), rsqrt_approx(qb)));
-    } else {
-        wo2 = mul2(ld2(W.wd[CLS]), pk2(rcp_approx(fmaxf(fabsf(ta), delta)),
-                                       rcp_approx(fmaxf(fabsf(tb), delta))));
+        return pk2(rsqrt_approx(qa), rsqrt_approx(qb));
     }
-    sdd = add2(sdd, wo2);
-    sd = fma2(wo2, t2, sd);
+    return pk2(rcp_approx(fmaxf(fabsf(ta), delta)), rcp_approx(fmaxf(fabsf(tb), delta)));
 }
 
-// Neighbours KA and KB (same weight class) of the centre at offset `base` in
-// the shared-memory planes, in one packed step: lane 0 accumulates KA's
-// terms, lane 1 KB's.  Against one neighbour per step this saves the
-// difference, the weight product and both accumulations of every second
-// neighbour (5 instead of 7 instructions per Huber term, 5.5 instead of 8 per
-// hyperbola term; measured 5 % / 8 % off the update).
-template <int POT, bool EDGE, int KA, int KB, int RW = USW>
-__device__ __forceinline__ void nb_pair(const float* __restrict__ pb, const float* __restrict__ pc,
-                                        const float* __restrict__ pa, int base, f32x2 xc2,
-                                        const PriorW5& W, float delta, float inv_delta,
-                                        f32x2& sdd, f32x2& sd) {
-    constexpr int dza = KA / 9 - 1, dya = (KA / 3) % 3 - 1, dxa = KA % 3 - 1;
-    constexpr int dzb = KB / 9 - 1, dyb = (KB / 3) % 3 - 1, dxb = KB % 3 - 1;
-    static_assert(nb_class<KA>() == nb_class<KB>(), "one weight class");
-    const float* pla = dza < 0 ? pb : (dza == 0 ? pc : pa);
-    const float* plb = dzb < 0 ? pb : (dzb == 0 ? pc : pa);
-    const f32x2 t2 = sub2(xc2, pk2(pla[base + dya * RW + dxa], plb[base + dyb * RW + dxb]));
-    nb_terms<POT, EDGE, nb_class<KA>()>(t2, W, delta, inv_delta, sdd, sd);
+// The factor of weight class CLS on omega2's values.
+template <int POT>
+__device__ __forceinline__ const float2& class_factor(const PriorW5& W, int cls) {
+    return POT == NR_POT_HUBER ? W.wd[cls] : W.w[cls];
 }
 
-// The 26 neighbours as 13 equal-weight pairs: (dx = -1, dx = +1) of each
-// (dy, dz) row, and the dx = 0 cells paired across dy or dz.  RW: floats per
-// row of the staged planes.
-template <int POT, bool EDGE, int RW>
-__device__ __forceinline__ void prior_pairs_w(const float* __restrict__ pb,
-                                              const float* __restrict__ pc,
-                                              const float* __restrict__ pa, int base, float xc,
-                                              const PriorW5& W, float delta, float inv_delta,
-                                              float* rdd, float* rd) {
-    const f32x2 xc2 = pk2(xc, xc);
-    f32x2 sdd = pk2(0.f, 0.f), sd = pk2(0.f, 0.f);
-#define NR_PAIR(a, b) \
-    nb_pair<POT, EDGE, a, b, RW>(pb, pc, pa, base, xc2, W, delta, inv_delta, sdd, sd)
-    NR_PAIR(0, 2); NR_PAIR(3, 5); NR_PAIR(6, 8);      // dz = -1 rows
-    NR_PAIR(9, 11); NR_PAIR(12, 14); NR_PAIR(15, 17); // dz = 0 rows
-    NR_PAIR(18, 20); NR_PAIR(21, 23); NR_PAIR(24, 26);  // dz = +1 rows
-    NR_PAIR(1, 7); NR_PAIR(19, 25); NR_PAIR(4, 22); NR_PAIR(10, 16);
-#undef NR_PAIR
-    float a0, a1, b0, b1;
-    upk2(sdd, a0, a1);
-    upk2(sd, b0, b1);
-    *rdd = a0 + a1;
-    *rd = b0 + b1;
+// Two neighbour pairs na, nb of one weight class: each lane sums its two terms
+// omega and omega t first and scales the sums once, sdd += w sum omega, sd +=
+// w sum omega t (one multiplication less per class than scaling each term).
+template <int POT, bool EDGE, int CLS>
+__device__ __forceinline__ void nb_class2(f32x2 xc2, f32x2 na, f32x2 nb, const PriorW5& W,
+                                          float delta, float inv_delta, f32x2& sdd, f32x2& sd) {
+    f32x2 ta = sub2(xc2, na), tb = sub2(xc2, nb);
+    const f32x2 oa = omega2<POT, EDGE>(ta, W, delta, inv_delta);
+    const f32x2 ob = omega2<POT, EDGE>(tb, W, delta, inv_delta);
+    const f32x2 f = ld2(class_factor<POT>(W, CLS));
+    sdd = fma2(f, add2(oa, ob), sdd);
+    sd = fma2(f, fma2(ob, tb, mul2(oa, ta)), sd);
 }
 
-template <int POT, bool EDGE>
-__device__ __forceinline__ void prior_pairs(const float* __restrict__ pb,
-                                            const float* __restrict__ pc,
-                                            const float* __restrict__ pa, int base, float xc,
-                                            const PriorW5& W, float delta, float inv_delta,
-                                            float* rdd, float* rd) {
-    prior_pairs_w<POT, EDGE, USW>(pb, pc, pa, base, xc, W, delta, inv_delta, rdd, rd);
+// The z-face neighbours na, nb of two voxels (one each): lane `LANE` of each
+// voxel's sums takes its term.
+template <int POT, bool EDGE, int LANE>
+__device__ __forceinline__ void nb_zface(f32x2 xc2, f32x2 n2, const PriorW5& W, float delta,
+                                         float inv_delta, f32x2& sdda, f32x2& sda, f32x2& sddb,
+                                         f32x2& sdb) {
+    f32x2 t2 = sub2(xc2, n2);
+    const f32x2 o2 = omega2<POT, EDGE>(t2, W, delta, inv_delta);
+    float oa, ob, pa, pb, v[2];
+    upk2(o2, oa, ob);
+    upk2(mul2(o2, t2), pa, pb);
+    const float f = class_factor<POT>(W, W_ZFACE).x;
+    upk2(sdda, v[0], v[1]);
+    v[LANE] = __fmaf_rn(f, oa, v[LANE]);
+    sdda = pk2(v[0], v[1]);
+    upk2(sda, v[0], v[1]);
+    v[LANE] = __fmaf_rn(f, pa, v[LANE]);
+    sda = pk2(v[0], v[1]);
+    upk2(sddb, v[0], v[1]);
+    v[LANE] = __fmaf_rn(f, ob, v[LANE]);
+    sddb = pk2(v[0], v[1]);
+    upk2(sdb, v[0], v[1]);
+    v[LANE] = __fmaf_rn(f, pb, v[LANE]);
+    sdb = pk2(v[0], v[1]);
 }
 
 // Kinds of fused update (template argument KIND of update_tile).
 constexpr int UPD_OSTR = 0;     // OSTR step above
 constexpr int UPD_SART = 1;     // OS-SART, backprj_OSSART_gpu_manyviews (Tomo_OSTR.cu:1737-1936)
 constexpr int UPD_SART_R = 2;   // OS-SART with the hyperbola prior, backprj_OSSART_R (:1938-2143)
-
-// Shared memory of one update tile: the 3-plane ring and the subset's sources.
-struct UpdSmem {
-    float tile[3][UPLANE];
-    ViewSrc sv[UPD_VIEWS_SMEM];
-};
 
 // The back projection of a voxel onto one view's detector is separable: on a
 // plane z, the detector column (ilb, fracI) of a voxel depends only on its x
@@ -214,8 +199,10 @@ struct UpdSmem {
 // per reconstruction, per view (subset order), plane and column / row, with
 // the arithmetic of bp.cu's sbp_term in reciprocal-multiply form, as a tap
 // pair and its weights:
-//   x[(a nz + z) nx + i] = {c, w0, w1, (x0 - x1)^2}
-//   y[(a nz + z) ny + j] = {r * BINSx, v0, v1, (y0 - y1)^2 + (z0 - z1)^2}
+//   x[(a nz + z) nx + i] = {c, w0, w1, k (x0 - x1)^2}
+//   y[(a nz + z) ny + j] = {r * BINSx, v0, v1, k ((y0 - y1)^2 + (z0 - z1)^2)}
+// with k = 1 / (Vsize_z |source|^2), so that the depth weight times Vsize_z is
+// the reciprocal of the entries' sum.
 // The bilinear stencil's columns are ilb, ilb + 1 with weights 1 - fracI,
 // fracI; a column off the detector gets weight 0 (the rules of
 // Tomo_OSTR.cu:1684-1715), and c is ilb clamped to [0, BINSx - 2] with the
@@ -268,7 +255,7 @@ __device__ __forceinline__ void bp_pair(int lb, float w0, float w1, int n, int& 
 }
 
 __device__ __forceinline__ float4 bp_entry_x(const nr_geom& g, const ViewSrc& vs, float tt,
-                                             int i, float inv_bx) {
+                                             int i, float inv_bx, float k) {
     const float x1 = vox_x(g, i);
     const float ddx = vs.x0 - x1;
     const float x2 = vs.x0 + (x1 - vs.x0) * tt;
@@ -281,11 +268,11 @@ __device__ __forceinline__ float4 bp_entry_x(const nr_geom& g, const ViewSrc& vs
     int c;
     float p0, p1;
     bp_pair(ilb, i0 ? 1.f - fracI : 0.f, i1 ? fracI : 0.f, g.nbx, c, p0, p1);
-    return make_float4(__int_as_float(c), p0, p1, ddx * ddx);
+    return make_float4(__int_as_float(c), p0, p1, k * (ddx * ddx));
 }
 
 __device__ __forceinline__ float4 bp_entry_y(const nr_geom& g, const ViewSrc& vs, float z1,
-                                             float tt, int j, float inv_by) {
+                                             float tt, int j, float inv_by, float k) {
     const bool valid = z1 != vs.z0;
     const float y1 = vox_y(g, j);
     const float ddy = vs.y0 - y1, ddz = vs.z0 - z1;
@@ -299,29 +286,52 @@ __device__ __forceinline__ float4 bp_entry_y(const nr_geom& g, const ViewSrc& vs
     int r;
     float p0, p1;
     bp_pair(jlb, j0 ? 1.f - fracJ : 0.f, j1 ? fracJ : 0.f, g.nby, r, p0, p1);
-    return make_float4(__int_as_float(r * g.nbx), p0, p1, ddy * ddy + ddz * ddz);
+    return make_float4(__int_as_float(r * g.nbx), p0, p1, k * (ddy * ddy + ddz * ddz));
 }
 
 // One view's back-projection term of one voxel, added to capL (and, for the
-// OS-SART kinds, the sensitivity): the tap pair (c, c + 1) x rows (r, r + 1)
-// of its table entries ex, ey on the view's h section p, off-detector taps
-// weighted 0 and their loads kept in bounds by the tables.
+// OS-SART kinds, the sensitivity), from its table entries ex, ey and the taps
+// q of its pair (c, c + 1) x rows (r, r + 1); off-detector taps are weighted 0
+// and their loads kept in bounds by the tables.
 template <int KIND>
 __device__ __forceinline__ void bp_view(const float* __restrict__ p, const float4 ex,
-                                        const float4 ey, float s2, const nr_geom& g, float& capL,
+                                        const float4 ey, const nr_geom& g, float& capL,
                                         float& sens) {
-    const float dw = __fdividef(s2, ex.w + ey.w);
     const float* q0 = p + (__float_as_int(ey.x) + __float_as_int(ex.x));
     const float* q1 = q0 + g.nbx;
-    float d1 = ex.y * __ldg(q0);
-    d1 = d1 + ex.z * __ldg(q0 + 1);
-    float d2 = ex.y * __ldg(q1);
-    d2 = d2 + ex.z * __ldg(q1 + 1);
-    capL = capL + (ey.y * d1 + ey.z * d2) * g.vz * dw;
+    const float dw = rcp_approx(ex.w + ey.w);
+    const float d1 = __fmaf_rn(ex.z, __ldg(q0 + 1), __fmul_rn(ex.y, __ldg(q0)));
+    const float d2 = __fmaf_rn(ex.z, __ldg(q1 + 1), __fmul_rn(ex.y, __ldg(q1)));
+    capL = __fmaf_rn(__fmaf_rn(ey.z, d2, __fmul_rn(ey.y, d1)), dw, capL);
     if (KIND != UPD_OSTR) {  // sensitivity: the same weights on ones
         const float s1 = ex.y + ex.z;
-        sens = sens + (ey.y * s1 + ey.z * s1) * g.vz * dw;
+        sens = __fmaf_rn(__fmaf_rn(ey.z, s1, __fmul_rn(ey.y, s1)), dw, sens);
     }
+}
+
+// The value of the OSTR step, xc - (M capL + beta rd) / (dv + 2 beta rdd).
+__device__ __forceinline__ float ostr_step(float xc, float capL, float rd, float rdd, float dv,
+                                           float M, float beta) {
+    const float num = __fmaf_rn(-M, capL, __fmul_rn(-beta, rd));
+    const float den = __fmaf_rn(2.f * beta, rdd, dv);
+    return __fmaf_rn(num, rcp_approx(den), xc);
+}
+
+// The value of the OS-SART step (Tomo_OSTR.cu:2193-2205: u / sens and beta
+// prior / sens, 0 without sensitivity); lambda in M.
+template <int KIND>
+__device__ __forceinline__ float sart_step(float xc, float capL, float sens, float rd, float M,
+                                           float beta) {
+    float ut = 0.f, bt = 0.f;
+    if (sens != 0.f) {
+        ut = __fdiv_rn(capL, sens);
+        if (KIND == UPD_SART_R) bt = __fdiv_rn(beta * rd, sens);
+    }
+    return xc + M * (ut + bt);
+}
+
+__device__ __forceinline__ bool not_finite(float v) {
+    return !(fabsf(v) < __int_as_float(0x7f800000));
 }
 
 // The update of one voxel from its sums, stored at out (non-finite values
@@ -330,31 +340,149 @@ template <int KIND>
 __device__ __forceinline__ void upd_store(float xc, float capL, float sens, float rd, float rdd,
                                           float dv, float M, float beta, float* __restrict__ out,
                                           int* __restrict__ status) {
-    float xn;
-    if (KIND == UPD_OSTR) {
-        capL = M * capL;
-        xn = xc - __fdividef(capL + beta * rd, dv + 2.f * beta * rdd);
-    } else {
-        // Tomo_OSTR.cu:2193-2205: u/sens and beta*prior/sens, 0 without sensitivity
-        float ut = 0.f, bt = 0.f;
-        if (sens != 0.f) {
-            ut = __fdiv_rn(capL, sens);
-            if (KIND == UPD_SART_R) bt = __fdiv_rn(beta * rd, sens);
-        }
-        xn = xc + M * (ut + bt);
-    }
-    if (!(fabsf(xn) < __int_as_float(0x7f800000))) atomicOr(status, NR_FLAG_NONFINITE);
+    const float xn = KIND == UPD_OSTR ? ostr_step(xc, capL, rd, rdd, dv, M, beta)
+                                      : sart_step<KIND>(xc, capL, sens, rd, M, beta);
+    if (not_finite(xn)) atomicOr(status, NR_FLAG_NONFINITE);
     *out = xn < 0.f ? 0.f : xn;
+}
+
+// One view's back projection onto the voxels A = (ix, iy) and B = (ix, iy + 1)
+// of a thread, in the steps its loads come in: the table entries (the column
+// entry serves both), then the four taps of each, then bp_view's sums, packed
+// (lane 0: A, lane 1: B; each lane rounded as there).
+struct UpdView {
+    float4 ex, ea, eb;
+    float qa[4], qb[4];
+    __device__ __forceinline__ void entries(const BpTab& T, int tix, int tiy, int jb) {
+        ex = __ldg(T.x + tix);
+        ea = __ldg(T.y + tiy);
+        eb = __ldg(T.y + (tiy + jb));
+    }
+    __device__ __forceinline__ void taps(const float* __restrict__ p, int nbx) {
+        const float* a = p + (__float_as_int(ea.x) + __float_as_int(ex.x));
+        const float* b = p + (__float_as_int(eb.x) + __float_as_int(ex.x));
+        qa[0] = __ldg(a);
+        qa[1] = __ldg(a + 1);
+        qb[0] = __ldg(b);
+        qb[1] = __ldg(b + 1);
+        a += nbx;
+        b += nbx;
+        qa[2] = __ldg(a);
+        qa[3] = __ldg(a + 1);
+        qb[2] = __ldg(b);
+        qb[3] = __ldg(b + 1);
+    }
+    template <int KIND>
+    __device__ __forceinline__ void add(f32x2& cap, f32x2& sens) const {
+        const f32x2 dw = pk2(rcp_approx(ex.w + ea.w), rcp_approx(ex.w + eb.w));
+        const f32x2 w0 = pk2(ex.y, ex.y), w1 = pk2(ex.z, ex.z);
+        const f32x2 v0 = pk2(ea.y, eb.y), v1 = pk2(ea.z, eb.z);
+        const f32x2 d1 = fma2(w1, pk2(qa[1], qb[1]), mul2(w0, pk2(qa[0], qb[0])));
+        const f32x2 d2 = fma2(w1, pk2(qa[3], qb[3]), mul2(w0, pk2(qa[2], qb[2])));
+        cap = fma2(fma2(v1, d2, mul2(v0, d1)), dw, cap);
+        if (KIND != UPD_OSTR) {
+            const float s = ex.y + ex.z;
+            const f32x2 s2 = pk2(s, s);
+            sens = fma2(fma2(v1, s2, mul2(v0, s2)), dw, sens);
+        }
+    }
+};
+
+// The voxels a thread of the update reads of one plane, around its voxels A =
+// (ix, iy) and B = (ix, iy + 1): rows iy - 1 .. iy + 2, per row the cells x -
+// 1, x + 1 and x.  Each neighbour class of A or B is then two packed pairs --
+// (x - 1, x + 1) of two rows, or of one row with the centre cells above and
+// below -- and every value read serves both voxels.
+struct UpdRows {
+    float l[4], e[4], c[4];
+    __device__ __forceinline__ f32x2 lr(int r) const { return pk2(l[r], e[r]); }
+};
+
+// Plane z's rows, `at` the offset of (ix, iy) in plane 0; a plane outside the
+// volume reads as zeros.  EDGE: cells outside the volume in x or y read as NaN.
+template <bool EDGE>
+__device__ __forceinline__ void upd_rows(const nr_geom& g, const float* __restrict__ x, int z,
+                                         int at, int ix, int iy, UpdRows& R) {
+    const int v = z * (g.nx * g.ny) + at;
+    const float qnan = __int_as_float(0x7fc00000);
+    const bool zin = z >= 0 && z < g.nz;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const float* q = x + (v + (r - 1) * g.nx);
+        R.c[r] = R.l[r] = R.e[r] = 0.f;
+        if (EDGE) {
+            const bool on = iy + r - 1 >= 0 && iy + r - 1 < g.ny;
+            if (zin) {
+                R.c[r] = on ? __ldg(q) : qnan;
+                R.l[r] = on && ix > 0 ? __ldg(q - 1) : qnan;
+                R.e[r] = on && ix + 1 < g.nx ? __ldg(q + 1) : qnan;
+            }
+        } else if (zin) {
+            R.c[r] = __ldg(q);
+            R.l[r] = __ldg(q - 1);
+            R.e[r] = __ldg(q + 1);
+        }
+    }
+}
+
+// The penalty sums of voxels A and B, one packed accumulator pair each (the
+// voxel's sum is the sum of the lanes).
+struct UpdSums {
+    f32x2 sdda, sda, sddb, sdb;
+};
+
+// The nine neighbours of both voxels (cells ca, cb) in the plane below (LANE
+// 0) or above (LANE 1).
+template <int POT, bool EDGE, int LANE>
+__device__ __forceinline__ void upd_far_plane(const UpdRows& R, float ca, float cb,
+                                              const PriorW5& W, float delta, float inv_delta,
+                                              UpdSums& S) {
+    const f32x2 a2 = pk2(ca, ca), b2 = pk2(cb, cb);
+    nb_class2<POT, EDGE, W_ZCORNER>(a2, R.lr(0), R.lr(2), W, delta, inv_delta, S.sdda, S.sda);
+    nb_class2<POT, EDGE, W_ZCORNER>(b2, R.lr(1), R.lr(3), W, delta, inv_delta, S.sddb, S.sdb);
+    nb_class2<POT, EDGE, W_ZEDGE>(a2, R.lr(1), pk2(R.c[0], R.c[2]), W, delta, inv_delta, S.sdda,
+                                  S.sda);
+    nb_class2<POT, EDGE, W_ZEDGE>(b2, R.lr(2), pk2(R.c[1], R.c[3]), W, delta, inv_delta, S.sddb,
+                                  S.sdb);
+    nb_zface<POT, EDGE, LANE>(pk2(ca, cb), pk2(R.c[1], R.c[2]), W, delta, inv_delta, S.sdda, S.sda,
+                              S.sddb, S.sdb);
+}
+
+// The eight in-plane neighbours of both voxels.
+template <int POT, bool EDGE>
+__device__ __forceinline__ void upd_own_plane(const UpdRows& R, const PriorW5& W, float delta,
+                                              float inv_delta, UpdSums& S) {
+    const f32x2 a2 = pk2(R.c[1], R.c[1]), b2 = pk2(R.c[2], R.c[2]);
+    nb_class2<POT, EDGE, W_FACE>(a2, R.lr(1), pk2(R.c[0], R.c[2]), W, delta, inv_delta, S.sdda,
+                                 S.sda);
+    nb_class2<POT, EDGE, W_FACE>(b2, R.lr(2), pk2(R.c[1], R.c[3]), W, delta, inv_delta, S.sddb,
+                                 S.sdb);
+    nb_class2<POT, EDGE, W_DIAG>(a2, R.lr(0), R.lr(2), W, delta, inv_delta, S.sdda, S.sda);
+    nb_class2<POT, EDGE, W_DIAG>(b2, R.lr(1), R.lr(3), W, delta, inv_delta, S.sddb, S.sdb);
 }
 
 // One sub-iteration's update, fused: SBP of h (subset views, [view][j][i]),
 // the penalty, and the update_est step.  Each block owns a 32 x 8 tile of
-// (x, y) columns and walks UZC planes in z, keeping planes z-1, z, z+1 of x
-// (with halo) in a 3-slot shared-memory ring, so every neighbour read is a
-// shared-memory load at a fixed offset.  The global loads of plane z+2 are
-// issued before plane z is computed (register prefetch), so they overlap the
-// arithmetic.  The back projection reads the separable tables (BpTab).
-// Writes x_out; flags non-finite values.
+// (x, y) columns and walks ZC planes in z; a thread owns two voxels of each
+// plane, one above the other in y, and carries the plane's rows in registers:
+// plane z - 1 and its voxels' unfinished sums (own plane and the one below)
+// wait there until plane z arrives, whose rows finish them and start plane z's.
+// There is no shared memory and no barrier, so warps run independently of
+// each other; the rows come through L1, where the tile's threads share them,
+// and are brought into L2 three planes ahead.  The order of a step gives each
+// load some arithmetic to hide behind: the next plane's rows and the taps of h
+// the own-plane neighbours, d and the table entries the nine below.  The back
+// projection reads the separable tables (BpTab).  Writes x_out; flags
+// non-finite values.
+//
+// The update is bound by instruction issue (DRAM traffic is at the algorithmic
+// bytes).  The form before -- one voxel per thread, three planes with halo in
+// a shared-memory ring, 26 shared loads and two barriers per voxel and plane --
+// issued 251 instructions per voxel at 77 % issue-active, 0.262 ms per
+// clinical sub-iteration; this one 188 at 64 %, 0.236 ms (full resolution
+// 1.20 -> 1.08 ms).  Measured beside it: the rows through a cp.async ring of
+// each warp's own (235 instructions, 0.250 ms at 74 %), the next plane's rows
+// a whole step ahead (spills, 0.31 ms).
 //
 // KIND = UPD_SART / UPD_SART_R turn the same tile into the OS-SART update:
 // h is the normalised projection difference of the subset, the back
@@ -365,306 +493,163 @@ __device__ __forceinline__ void upd_store(float xc, float capL, float sens, floa
 // z ratio 1) for UPD_SART_R, and d unused.
 //
 // NV > 0 fixes the subset's view count at compile time (nv is then NV): with
-// one view per subset the per-view loop disappears, which saves ~40
-// instructions per voxel and 8 registers.
+// one view per subset the per-view loop disappears.
 template <int POT, int ZC = UZC, int KIND = UPD_OSTR, int NV = 0>
 __device__ __forceinline__ void update_tile(
     const Geo& G, const PriorW5& W, const float* __restrict__ x, float* __restrict__ x_out,
-    const float* __restrict__ d, const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const BpTab& T, int a0, int nv, float M, float beta,
-    float delta, int* __restrict__ status, int bx, int by, int bz, UpdSmem& sm) {
-    float (*tile)[UPLANE] = sm.tile;
-    ViewSrc* sv = sm.sv;
+    const float* __restrict__ d, const float* __restrict__ h, const BpTab& T, int a0, int nv,
+    float M, float beta, float delta, int* __restrict__ status, int bx, int by, int bz) {
     const nr_geom& g = G.g;
-    const int tid = threadIdx.y * UTX + threadIdx.x;
-    for (int t = tid; t < (NV ? NV : nv); t += UTX * UTY)
-        sv[t] = view_source(g, angles[index[a0 + t]]);
     const int x0t = bx * UTX, y0t = by * UTY;
+    const int ix = x0t + threadIdx.x, iy = y0t + 2 * threadIdx.y;
+    if (ix >= g.nx || iy >= g.ny) return;
+    const bool has_b = iy + 1 < g.ny;   // voxel B is in the volume
     const int zb = bz * ZC, ze = min(zb + ZC, g.nz);
     // voxel and table indices in 32 bits: volumes hold fewer than 2^31 voxels
     // (geom_ok) and the tables fewer than 2^31 entries (bp_tables_fit)
     const int plane = g.nx * g.ny;
-    // This thread's (at most two) cells of a halo plane tile.
-    constexpr int NT = UTX * UTY;
-    static_assert(UPLANE <= 2 * NT, "two cells per thread");
-    const int e1 = tid + NT;
-    const bool has1 = e1 < UPLANE;
-    auto cell_off = [&](int k, bool& ok) -> int {
-        const int r = k / USW, c = k - r * USW;
-        const int gx = x0t - 1 + c, gy = y0t - 1 + r;
-        ok = gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny;
-        return ok ? gy * g.nx + gx : 0;
-    };
-    bool ok0, ok1 = false;
-    const int off0 = cell_off(tid, ok0);
-    const int off1 = has1 ? cell_off(e1, ok1) : 0;
-    const float qnan = __int_as_float(0x7fc00000);  // outside the volume
-    auto fetch = [&](int z, float& v0, float& v1) {
-        const bool zin = z >= 0 && z < g.nz;
-        v0 = (zin && ok0) ? __ldg(x + (z * plane + off0)) : qnan;
-        v1 = (zin && ok1) ? __ldg(x + (z * plane + off1)) : qnan;
-    };
-    float* pb = tile[0];
-    float* pc = tile[1];
-    float* pa = tile[2];
-    {
-        float v0, v1;
-        fetch(zb - 1, v0, v1);
-        pb[tid] = v0;
-        if (has1) pb[e1] = v1;
-        fetch(zb, v0, v1);
-        pc[tid] = v0;
-        if (has1) pc[e1] = v1;
-    }
-    float n0, n1;
-    fetch(zb + 1, n0, n1);
-    const int ix = x0t + threadIdx.x, iy = y0t + threadIdx.y;
-    const bool active = ix < g.nx && iy < g.ny;
-    const bool edge_xy = x0t == 0 || x0t + UTX >= g.nx || y0t == 0 || y0t + UTY >= g.ny;
+    const int at = iy * g.nx + ix;
+    const int jb = has_b ? 1 : 0;       // B's offsets, kept in bounds
     const float inv_delta = 1.f / delta;
     const int64_t B = (int64_t)g.nbx * g.nby;
-    const int r = threadIdx.y + 1, c = threadIdx.x + 1;
-    for (int z = zb; z < ze; z++) {
-        pa[tid] = n0;
-        if (has1) pa[e1] = n1;
-        __syncthreads();
-        if (z + 1 < ze) fetch(z + 2, n0, n1);
-        if (active) {
-            const int v = z * plane + iy * g.nx + ix;
-            const float dv = KIND == UPD_OSTR ? __ldg(d + v) : 0.f;
-            const float xc = pc[r * USW + c];
-            // M * SBP(h) from the plane's tables: the taps and weights of
-            // bp.cu's sbp_term on the [j][i] layout.
-            float capL = 0.f, sens = 0.f;
+    UpdSums S;
+    UpdView V;
+    float dva = 0.f, dvb = 0.f;
+    // d and the first view's table entries of plane z's voxels
+    auto fetch = [&](int z) {
+        const int v = z * plane + at;
+        if (KIND == UPD_OSTR) {
+            dva = __ldg(d + v);
+            dvb = __ldg(d + (v + jb * g.nx));
+        }
+        V.entries(T, (a0 * g.nz + z) * g.nx + ix, (a0 * g.nz + z) * g.ny + iy, jb);
+    };
+    // The update of plane z's voxels ca, cb from their sums (d and the first
+    // view's taps are loaded): upd_store's steps, packed for the OSTR kind.
+    auto finish = [&](int z, float ca, float cb) {
+        const int v = z * plane + at;
+        f32x2 cap = pk2(0.f, 0.f), sens = cap;
+        V.add<KIND>(cap, sens);
+        if (NV != 1) {
             const float* p = h;
             int tix = (a0 * g.nz + z) * g.nx + ix;
             int tiy = (a0 * g.nz + z) * g.ny + iy;
             const int sx = g.nz * g.nx, sy = g.nz * g.ny;
-            for (int t = 0; t < (NV ? NV : nv); t++, p += B, tix += sx, tiy += sy)
-                bp_view<KIND>(p, __ldg(T.x + tix), __ldg(T.y + tiy), sv[t].s2, g, capL, sens);
-            float rdd = 0.f, rd = 0.f;
-            const int base = r * USW + c;
-            if (KIND != UPD_SART) {
-                if (edge_xy || z == 0 || z == g.nz - 1)
-                    prior_pairs<POT, true>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
-                else
-                    prior_pairs<POT, false>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
+            for (int t = 1; t < (NV ? NV : nv); t++) {
+                p += B;
+                tix += sx;
+                tiy += sy;
+                V.entries(T, tix, tiy, jb);
+                V.taps(p, g.nbx);
+                V.add<KIND>(cap, sens);
             }
-            upd_store<KIND>(xc, capL, sens, rd, rdd, dv, M, beta, x_out + v, status);
         }
-        __syncthreads();
-        float* t = pb;
-        pb = pc;
-        pc = pa;
-        pa = t;
+        float u, w, rdda, rda, rddb, rdb, xa, xb;
+        upk2(S.sdda, u, w);
+        rdda = u + w;
+        upk2(S.sda, u, w);
+        rda = u + w;
+        upk2(S.sddb, u, w);
+        rddb = u + w;
+        upk2(S.sdb, u, w);
+        rdb = u + w;
+        if (KIND == UPD_OSTR) {
+            const f32x2 num = fma2(pk2(-M, -M), cap, mul2(pk2(-beta, -beta), pk2(rda, rdb)));
+            const f32x2 den =
+                fma2(pk2(2.f * beta, 2.f * beta), pk2(rdda, rddb), pk2(dva, dvb));
+            upk2(den, u, w);
+            upk2(fma2(num, pk2(rcp_approx(u), rcp_approx(w)), pk2(ca, cb)), xa, xb);
+        } else {
+            float sa, sb;
+            upk2(cap, u, w);
+            upk2(sens, sa, sb);
+            xa = sart_step<KIND>(ca, u, sa, rda, M, beta);
+            xb = sart_step<KIND>(cb, w, sb, rdb, M, beta);
+        }
+        if (not_finite(xa) || (has_b && not_finite(xb))) atomicOr(status, NR_FLAG_NONFINITE);
+        x_out[v] = xa < 0.f ? 0.f : xa;
+        if (has_b) x_out[v + g.nx] = xb < 0.f ? 0.f : xb;
+    };
+    S.sdda = S.sda = S.sddb = S.sdb = pk2(0.f, 0.f);
+    if (KIND == UPD_SART) {
+        fetch(zb);
+        for (int z = zb; z < ze; z++) {
+            const int v = z * plane + at;
+            const float ca = __ldg(x + v), cb = __ldg(x + (v + jb * g.nx));
+            V.taps(h, g.nbx);
+            const UpdView U = V;
+            if (z + 1 < ze) fetch(z + 1);   // the next plane's entries while the taps come
+            const UpdView F = V;
+            V = U;
+            finish(z, ca, cb);
+            V = F;
+        }
+        return;
     }
-}
-
-// ---- Two voxels per thread ----------------------------------------------
-// The x2 tile: 64 x 8 columns, thread (tx, ty) owning voxels x0 + 2 tx and
-// x0 + 2 tx + 1 of row y0 + ty.  The neighbour terms of its two voxels at one
-// offset form a packed pair whose operands lie side by side in shared
-// memory, so one 64-bit load brings both.  In a plane row with its halo the
-// two voxels sit at cells 2 tx + 1 and 2 tx + 2: the dx = -1 and dx = +1
-// pairs start at the even cells 2 tx and 2 tx + 2; the dx = 0 pairs (odd
-// start) are read from a second copy of the plane stored one float later.
-// Per voxel this halves the shared-memory loads of the penalty and shares
-// the row table entry of the back projection.
-constexpr int U2X = 2 * UTX;           // 64 columns
-constexpr int U2W = U2X + 2;           // cells per row with the halo (even)
-constexpr int U2PLANE = U2W * USH;     // cells per plane
-constexpr int U2COPY = U2PLANE + 2;    // floats per copy (the shifted copy ends one later)
-static_assert(U2W % 2 == 0 && U2COPY % 2 == 0, "8-byte aligned rows and copies");
-
-struct UpdSmem2 {
-    alignas(16) float tile[3][2 * U2COPY];  // per ring slot: copy 0 (cell k at k), copy 1 (at k + 1)
-    ViewSrc sv[UPD_VIEWS_SMEM];
-};
-
-// Neighbour K of both voxels (base: the first voxel's cell in copy 0).
-template <int POT, bool EDGE, int K>
-__device__ __forceinline__ void nb_x2(const float* __restrict__ pb, const float* __restrict__ pc,
-                                      const float* __restrict__ pa, int base, f32x2 xc2,
-                                      const PriorW5& W, float delta, float inv_delta, f32x2& sdd,
-                                      f32x2& sd) {
-    constexpr int dz = K / 9 - 1, dy = (K / 3) % 3 - 1, dx = K % 3 - 1;
-    const float* pl = dz < 0 ? pb : (dz == 0 ? pc : pa);
-    const int at = dx == 0 ? U2COPY + base + 1 + dy * U2W : base + dy * U2W + dx;
-    const f32x2 n2 = *reinterpret_cast<const f32x2*>(pl + at);
-    nb_terms<POT, EDGE, nb_class<K>()>(sub2(xc2, n2), W, delta, inv_delta, sdd, sd);
-}
-
-// The penalty sums of both voxels.  Each voxel's neighbours are summed in
-// the order and grouping of prior_pairs (its two partial sums, then their
-// sum), so every voxel gets the bits the one-voxel tile gives it.
-template <int POT, bool EDGE>
-__device__ __forceinline__ void prior_x2(const float* __restrict__ pb,
-                                         const float* __restrict__ pc,
-                                         const float* __restrict__ pa, int base, f32x2 xc2,
-                                         const PriorW5& W, float delta, float inv_delta,
-                                         f32x2& rdd2, f32x2& rd2) {
-    const f32x2 zero = pk2(0.f, 0.f);
-    f32x2 dda = zero, da = zero, ddb = zero, db = zero;
-#define NR_X2(ka, kb)                                                              \
-    nb_x2<POT, EDGE, ka>(pb, pc, pa, base, xc2, W, delta, inv_delta, dda, da);    \
-    nb_x2<POT, EDGE, kb>(pb, pc, pa, base, xc2, W, delta, inv_delta, ddb, db)
-    NR_X2(0, 2); NR_X2(3, 5); NR_X2(6, 8);
-    NR_X2(9, 11); NR_X2(12, 14); NR_X2(15, 17);
-    NR_X2(18, 20); NR_X2(21, 23); NR_X2(24, 26);
-    NR_X2(1, 7); NR_X2(19, 25); NR_X2(4, 22); NR_X2(10, 16);
-#undef NR_X2
-    rdd2 = add2(dda, ddb);
-    rd2 = add2(da, db);
-}
-
-// update_tile on the x2 tile: the same sums and update, bit for bit, for the
-// two voxels of each thread.  A voxel past the volume's last column is
-// computed from out-of-volume cells and not stored.
-template <int POT, int ZC = UZC, int KIND = UPD_OSTR, int NV = 0>
-__device__ __forceinline__ void update_tile_x2(
-    const Geo& G, const PriorW5& W, const float* __restrict__ x, float* __restrict__ x_out,
-    const float* __restrict__ d, const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const BpTab& T, int a0, int nv, float M, float beta,
-    float delta, int* __restrict__ status, int bx, int by, int bz, UpdSmem2& sm) {
-    ViewSrc* sv = sm.sv;
-    const nr_geom& g = G.g;
-    const int tid = threadIdx.y * UTX + threadIdx.x;
-    for (int t = tid; t < (NV ? NV : nv); t += UTX * UTY)
-        sv[t] = view_source(g, angles[index[a0 + t]]);
-    const int x0t = bx * U2X, y0t = by * UTY;
-    const int zb = bz * ZC, ze = min(zb + ZC, g.nz);
-    const int plane = g.nx * g.ny;
-    // This thread's (two or three) cells of a halo plane tile.
-    constexpr int NT = UTX * UTY;
-    static_assert(2 * NT <= U2PLANE && U2PLANE <= 3 * NT, "two or three cells per thread");
-    const int e1 = tid + NT, e2 = tid + 2 * NT;
-    const bool has2 = e2 < U2PLANE;
-    auto cell_off = [&](int k, bool& ok) -> int {
-        const int r = k / U2W, c = k - r * U2W;
-        const int gx = x0t - 1 + c, gy = y0t - 1 + r;
-        ok = gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny;
-        return ok ? gy * g.nx + gx : 0;
+    // Lanes 0-7: one end of a row of the warp, of x (lanes 0-3) or d (4-7).
+    const int pl = threadIdx.x & 7;
+    const float* pf = (pl < 4 || KIND != UPD_OSTR ? x : d) +
+                      ((iy + ((pl >> 1) & 1) * jb) * g.nx + min(x0t + (pl & 1) * (UTX - 1), g.nx - 1));
+    auto prefetch = [&](int z) {
+        if (threadIdx.x < 8 && z < g.nz)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                __cvta_generic_to_global(pf + (int64_t)z * plane)));
     };
-    bool ok0, ok1, ok2 = false;
-    const int off0 = cell_off(tid, ok0);
-    const int off1 = cell_off(e1, ok1);
-    const int off2 = has2 ? cell_off(e2, ok2) : 0;
-    const float qnan = __int_as_float(0x7fc00000);  // outside the volume
-    auto fetch = [&](int z, float& v0, float& v1, float& v2) {
-        const bool zin = z >= 0 && z < g.nz;
-        v0 = (zin && ok0) ? __ldg(x + (z * plane + off0)) : qnan;
-        v1 = (zin && ok1) ? __ldg(x + (z * plane + off1)) : qnan;
-        v2 = (zin && ok2) ? __ldg(x + (z * plane + off2)) : qnan;
-    };
-    auto put = [&](float* pl, float v0, float v1, float v2) {
-        pl[tid] = v0;
-        pl[U2COPY + tid + 1] = v0;
-        pl[e1] = v1;
-        pl[U2COPY + e1 + 1] = v1;
-        if (has2) {
-            pl[e2] = v2;
-            pl[U2COPY + e2 + 1] = v2;
+    auto walk = [&](auto edge_c) {
+        constexpr bool EDGE = decltype(edge_c)::value;
+        // Starts plane z's voxels (rows N; P holds plane z - 1), then loads plane
+        // z + 1 into P.
+        auto start = [&](UpdRows& P, const UpdRows& N, int z) {
+            fetch(z);
+            S.sdda = S.sda = S.sddb = S.sdb = pk2(0.f, 0.f);
+            // a plane outside the volume (zeros) against zeros: t = 0
+            upd_far_plane<POT, EDGE, 0>(P, z > 0 ? N.c[1] : 0.f, z > 0 ? N.c[2] : 0.f, W, delta,
+                                        inv_delta, S);
+            upd_rows<EDGE>(g, x, z + 1, at, ix, iy, P);
+            V.taps(h, g.nbx);
+            prefetch(z + 3);
+            upd_own_plane<POT, EDGE>(N, W, delta, inv_delta, S);
+        };
+        // Plane z + 1 is in F: finishes plane z's voxels ca, cb.
+        auto end = [&](const UpdRows& F, float ca, float cb, int z) {
+            const bool in = z + 1 < g.nz;
+            upd_far_plane<POT, EDGE, 1>(F, in ? ca : 0.f, in ? cb : 0.f, W, delta, inv_delta, S);
+            finish(z, ca, cb);
+        };
+        UpdRows A, C;
+        prefetch(zb + 1);
+        prefetch(zb + 2);
+        upd_rows<EDGE>(g, x, zb - 1, at, ix, iy, A);
+        upd_rows<EDGE>(g, x, zb, at, ix, iy, C);
+        for (int z = zb;; z += 2) {
+            start(A, C, z);
+            end(A, C.c[1], C.c[2], z);
+            if (z + 1 == ze) break;
+            start(C, A, z + 1);
+            end(C, A.c[1], A.c[2], z + 1);
+            if (z + 2 == ze) break;
         }
     };
-    float* pb = sm.tile[0];
-    float* pc = sm.tile[1];
-    float* pa = sm.tile[2];
-    float n0, n1, n2;
-    fetch(zb - 1, n0, n1, n2);
-    put(pb, n0, n1, n2);
-    fetch(zb, n0, n1, n2);
-    put(pc, n0, n1, n2);
-    fetch(zb + 1, n0, n1, n2);
-    const int ix = x0t + 2 * threadIdx.x, iy = y0t + threadIdx.y;
-    const bool active = ix < g.nx && iy < g.ny;
-    const bool has_b = ix + 1 < g.nx;   // the second voxel is in the volume
-    const bool edge_xy = x0t == 0 || x0t + U2X >= g.nx || y0t == 0 || y0t + UTY >= g.ny;
-    const float inv_delta = 1.f / delta;
-    const int64_t B = (int64_t)g.nbx * g.nby;
-    const int base = (threadIdx.y + 1) * U2W + 2 * threadIdx.x + 1;
-    for (int z = zb; z < ze; z++) {
-        put(pa, n0, n1, n2);
-        __syncthreads();
-        if (z + 1 < ze) fetch(z + 2, n0, n1, n2);
-        if (active) {
-            const int v = z * plane + iy * g.nx + ix;
-            const float dva = KIND == UPD_OSTR ? __ldg(d + v) : 0.f;
-            const float dvb = (KIND == UPD_OSTR && has_b) ? __ldg(d + v + 1) : 0.f;
-            const f32x2 xc2 = *reinterpret_cast<const f32x2*>(pc + U2COPY + base + 1);
-            float capa = 0.f, capb = 0.f, sensa = 0.f, sensb = 0.f;
-            const float* p = h;
-            int tix = (a0 * g.nz + z) * g.nx + ix;
-            int tiy = (a0 * g.nz + z) * g.ny + iy;
-            const int sx = g.nz * g.nx, sy = g.nz * g.ny;
-            const int db = has_b ? 1 : 0;   // the second voxel's column entry (kept in bounds)
-            for (int t = 0; t < (NV ? NV : nv); t++, p += B, tix += sx, tiy += sy) {
-                const float4 ey = __ldg(T.y + tiy);
-                const float s2 = sv[t].s2;
-                bp_view<KIND>(p, __ldg(T.x + tix), ey, s2, g, capa, sensa);
-                bp_view<KIND>(p, __ldg(T.x + tix + db), ey, s2, g, capb, sensb);
-            }
-            f32x2 rdd2 = pk2(0.f, 0.f), rd2 = pk2(0.f, 0.f);
-            if (KIND != UPD_SART) {
-                if (edge_xy || z == 0 || z == g.nz - 1)
-                    prior_x2<POT, true>(pb, pc, pa, base, xc2, W, delta, inv_delta, rdd2, rd2);
-                else
-                    prior_x2<POT, false>(pb, pc, pa, base, xc2, W, delta, inv_delta, rdd2, rd2);
-            }
-            float xa, xb, rdda, rddb, rda, rdb;
-            upk2(xc2, xa, xb);
-            upk2(rdd2, rdda, rddb);
-            upk2(rd2, rda, rdb);
-            upd_store<KIND>(xa, capa, sensa, rda, rdda, dva, M, beta, x_out + v, status);
-            if (has_b)
-                upd_store<KIND>(xb, capb, sensb, rdb, rddb, dvb, M, beta, x_out + v + 1, status);
-        }
-        __syncthreads();
-        float* t = pb;
-        pb = pc;
-        pc = pa;
-        pa = t;
-    }
+    if (x0t == 0 || x0t + UTX >= g.nx || y0t == 0 || y0t + UTY >= g.ny)
+        walk(std::integral_constant<bool, true>());
+    else
+        walk(std::integral_constant<bool, false>());
 }
 
-// One block per (x, y) tile and chunk of ZC planes; NV as in update_tile.
-// One-view kernels are held to 32 registers (8 resident blocks per SM: the
-// paired prior would otherwise take 35-38).  The others carry no block
-// minimum (40-44 registers, no spills); a minimum of 1 lets ptxas take 80-119
-// and one of 5 spills 80 bytes.
+// One block of 32 x 4 threads per (x, y) tile and chunk of ZC planes; NV as in
+// update_tile.
 template <int POT, int ZC, int NV>
-__global__ void __launch_bounds__(256, NV == 1 ? 8 : 0) update_kernel(
+__global__ void __launch_bounds__(UNT, UPD_BLOCKS) update_kernel(
     const __grid_constant__ Geo G, const __grid_constant__ PriorW5 W,
     const float* __restrict__ x, float* __restrict__ x_out, const float* __restrict__ d,
-    const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const __grid_constant__ BpTab T, int a0, int nv,
+    const float* __restrict__ h, const __grid_constant__ BpTab T, int a0, int nv,
     float M, float beta, float delta, int* __restrict__ status) {
-    __shared__ UpdSmem sm;
-    update_tile<POT, ZC, UPD_OSTR, NV>(G, W, x, x_out, d, h, angles, index, T, a0, nv, M, beta,
-                                       delta, status, blockIdx.x, blockIdx.y, blockIdx.z, sm);
+    update_tile<POT, ZC, UPD_OSTR, NV>(G, W, x, x_out, d, h, T, a0, nv, M, beta, delta, status,
+                                       blockIdx.x, blockIdx.y, blockIdx.z);
 }
-
-// The same update on x2 tiles (64 x 8 columns per block), five resident
-// blocks per SM (48 registers, no spills).  Measured per 25 updates at 16
-// planes, clinical / full resolution: 5 blocks 6.54 / 17.42 ms, 6 blocks (40
-// registers) 6.71 / 17.46 ms, 4 blocks (64 registers) 6.82 / 18.51 ms; held
-// to 8 blocks (32 registers) it spills 20 bytes (0.275 ms per update).
-template <int POT, int ZC, int NV>
-__global__ void __launch_bounds__(256, NV == 1 ? 5 : 0) update_x2_kernel(
-    const __grid_constant__ Geo G, const __grid_constant__ PriorW5 W,
-    const float* __restrict__ x, float* __restrict__ x_out, const float* __restrict__ d,
-    const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const __grid_constant__ BpTab T, int a0, int nv,
-    float M, float beta, float delta, int* __restrict__ status) {
-    __shared__ UpdSmem2 sm;
-    update_tile_x2<POT, ZC, UPD_OSTR, NV>(G, W, x, x_out, d, h, angles, index, T, a0, nv, M,
-                                          beta, delta, status, blockIdx.x, blockIdx.y,
-                                          blockIdx.z, sm);
-}
-
 
 // ---- TMA-fed ring -----------------------------------------------------------
-// The one-voxel tile with its planes streamed by TMA instead of through the
-// threads' registers: lane 0 of warp 0 loads each plane of the tile with its
+// One voxel per thread, the planes streamed by TMA: lane 0 of warp 0 loads each plane of the tile with its
 // halo (one cp.async.bulk.tensor.3d box of UTW x USH voxels starting 4 voxels
 // left of the tile, so that the box's x coordinate is a multiple of 4 floats;
 // out-of-volume voxels read as NaN, the ring's convention for "outside") into
@@ -686,6 +671,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 5 : 0) update_x2_kernel(
 // is released.  A first version with a ninth, producer-only warp held 7
 // blocks per SM instead of 8 and ran 11 % slower on the clinical workload.
 constexpr int UTW = UTX + 8;            // columns of a staged row: x0 - 4 .. x0 + 35
+constexpr int USH = UTY + 2;            // rows of a staged plane
 constexpr int UT_SLOT = 416;            // floats per slot: UTW x USH = 400, rounded to 128 B
 constexpr int UT_SLOTS = 6;
 constexpr uint32_t UT_BYTES = UTW * USH * 4;
@@ -696,20 +682,54 @@ struct UpdSmemT {
     alignas(128) float ring[UT_SLOTS][UT_SLOT];
     alignas(8) uint64_t full[UT_SLOTS];
     uint64_t empty[UT_SLOTS];
-    ViewSrc sv[UPD_VIEWS_SMEM];
 };
+
+// One z-face neighbour n of a voxel, as nb_zface forms it: lane LANE of the sums.
+template <int POT, bool EDGE, int LANE>
+__device__ __forceinline__ void nb_zface1(float xc, float n, const PriorW5& W, float delta,
+                                          float inv_delta, f32x2& sdd, f32x2& sd) {
+    f32x2 zdd = pk2(0.f, 0.f), zd = pk2(0.f, 0.f);
+    nb_zface<POT, EDGE, LANE>(pk2(xc, xc), pk2(n, n), W, delta, inv_delta, sdd, sd, zdd, zd);
+}
+
+// The penalty sums of the voxel at `base` of the ring's planes below (pb), its
+// own (pc) and above (pa): the terms of update_tile in its order and grouping.
+template <int POT, bool EDGE>
+__device__ __forceinline__ void prior_ring(const float* __restrict__ pb,
+                                           const float* __restrict__ pc,
+                                           const float* __restrict__ pa, int base, float xc,
+                                           const PriorW5& W, float delta, float inv_delta,
+                                           float* rdd, float* rd) {
+    const f32x2 c2 = pk2(xc, xc);
+    f32x2 sdd = pk2(0.f, 0.f), sd = pk2(0.f, 0.f);
+    auto lr = [&](const float* p, int dy) {
+        return pk2(p[base + dy * UTW - 1], p[base + dy * UTW + 1]);
+    };
+    auto ud = [&](const float* p) { return pk2(p[base - UTW], p[base + UTW]); };
+    nb_class2<POT, EDGE, W_ZCORNER>(c2, lr(pb, -1), lr(pb, 1), W, delta, inv_delta, sdd, sd);
+    nb_class2<POT, EDGE, W_ZEDGE>(c2, lr(pb, 0), ud(pb), W, delta, inv_delta, sdd, sd);
+    nb_zface1<POT, EDGE, 0>(xc, pb[base], W, delta, inv_delta, sdd, sd);
+    nb_class2<POT, EDGE, W_FACE>(c2, lr(pc, 0), ud(pc), W, delta, inv_delta, sdd, sd);
+    nb_class2<POT, EDGE, W_DIAG>(c2, lr(pc, -1), lr(pc, 1), W, delta, inv_delta, sdd, sd);
+    nb_class2<POT, EDGE, W_ZCORNER>(c2, lr(pa, -1), lr(pa, 1), W, delta, inv_delta, sdd, sd);
+    nb_class2<POT, EDGE, W_ZEDGE>(c2, lr(pa, 0), ud(pa), W, delta, inv_delta, sdd, sd);
+    nb_zface1<POT, EDGE, 1>(xc, pa[base], W, delta, inv_delta, sdd, sd);
+    float u, w;
+    upk2(sdd, u, w);
+    *rdd = u + w;
+    upk2(sd, u, w);
+    *rd = u + w;
+}
 
 template <int POT, int ZC = UZC, int KIND = UPD_OSTR, int NV = 0>
 __device__ __forceinline__ void update_tile_tma(
     const Geo& G, const PriorW5& W, const CUtensorMap* map, float* __restrict__ x_out,
-    const float* __restrict__ d, const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const BpTab& T, int a0, int nv, float M, float beta,
-    float delta, int* __restrict__ status, int bx, int by, int bz, UpdSmemT& sm) {
+    const float* __restrict__ d, const float* __restrict__ h, const BpTab& T, int a0, int nv,
+    float M, float beta, float delta, int* __restrict__ status, int bx, int by, int bz,
+    UpdSmemT& sm) {
     const nr_geom& g = G.g;
     const int warp = threadIdx.y, lane = threadIdx.x;
     const int tid = warp * UTX + lane;
-    for (int t = tid; t < (NV ? NV : nv); t += UTX * UTY)
-        sm.sv[t] = view_source(g, angles[index[a0 + t]]);
     const int x0t = bx * UTX, y0t = by * UTY;
     const int zb = bz * ZC, ze = min(zb + ZC, g.nz);
     const int np = ze - zb + 2;  // planes zb - 1 .. ze; plane k is z = zb - 1 + k
@@ -770,15 +790,13 @@ __device__ __forceinline__ void update_tile_tma(
             int tiy = (a0 * g.nz + z) * g.ny + iy;
             const int sx = g.nz * g.nx, sy = g.nz * g.ny;
             for (int t = 0; t < (NV ? NV : nv); t++, p += B, tix += sx, tiy += sy)
-                bp_view<KIND>(p, __ldg(T.x + tix), __ldg(T.y + tiy), sm.sv[t].s2, g, capL, sens);
+                bp_view<KIND>(p, __ldg(T.x + tix), __ldg(T.y + tiy), g, capL, sens);
             float rdd = 0.f, rd = 0.f;
             if (KIND != UPD_SART) {
                 if (edge_xy || z == 0 || z == g.nz - 1)
-                    prior_pairs_w<POT, true, UTW>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd,
-                                                  &rd);
+                    prior_ring<POT, true>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
                 else
-                    prior_pairs_w<POT, false, UTW>(pb, pc, pa, base, xc, W, delta, inv_delta,
-                                                   &rdd, &rd);
+                    prior_ring<POT, false>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
             }
             upd_store<KIND>(xc, capL, sens, rd, rdd, dv, M, beta, x_out + v, status);
         }
@@ -816,19 +834,16 @@ __device__ __forceinline__ void update_tile_tma(
     }
 }
 
-// One block per (x, y) tile and chunk of ZC planes, 8 warps (one row each);
-// one-view kernels held to 32 registers (8 resident blocks per SM).
+// One block per (x, y) tile and chunk of ZC planes, 8 warps (one row each).
 template <int POT, int ZC, int NV>
-__global__ void __launch_bounds__(256, NV == 1 ? 8 : 0) update_tma_kernel(
+__global__ void __launch_bounds__(256, NV == 1 ? 6 : 0) update_tma_kernel(
     const __grid_constant__ Geo G, const __grid_constant__ PriorW5 W,
     const __grid_constant__ CUtensorMap map, float* __restrict__ x_out,
-    const float* __restrict__ d, const float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const __grid_constant__ BpTab T, int a0, int nv,
-    float M, float beta, float delta, int* __restrict__ status) {
+    const float* __restrict__ d, const float* __restrict__ h, const __grid_constant__ BpTab T,
+    int a0, int nv, float M, float beta, float delta, int* __restrict__ status) {
     __shared__ UpdSmemT sm;
-    update_tile_tma<POT, ZC, UPD_OSTR, NV>(G, W, &map, x_out, d, h, angles, index, T, a0, nv, M,
-                                           beta, delta, status, blockIdx.x, blockIdx.y,
-                                           blockIdx.z, sm);
+    update_tile_tma<POT, ZC, UPD_OSTR, NV>(G, W, &map, x_out, d, h, T, a0, nv, M, beta, delta,
+                                           status, blockIdx.x, blockIdx.y, blockIdx.z, sm);
 }
 
 }  // namespace nr

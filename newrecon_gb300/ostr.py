@@ -370,13 +370,13 @@ class OSTR:
                  stage: bool = False, upd_tile: int = 0):
         """stage=True stages the projection's volume slab by slab in shared
         memory by TMA instead of gathering it through L1/L2 (same result;
-        slower on the clinical workload).  upd_tile=1 gives each thread of the
-        update two voxels side by side in x (one-view subsets); upd_tile=2
-        streams the update's planes by TMA through a shared-memory ring filled
-        by a producer warp (where IMGSIZx is a multiple of 4).  Every variant
-        gives the same result bit for bit.  autotune() picks them per geometry."""
+        slower on the clinical workload).  upd_tile=0 and 1 give each thread of
+        the update two voxels of a plane; upd_tile=2 streams the update's planes
+        by TMA through a shared-memory ring (where IMGSIZx is a multiple of 4).
+        Every variant gives the same result bit for bit.  autotune() picks them
+        per geometry."""
         if upd_tile not in (0, 1, 2):
-            raise ValueError("upd_tile must be 0 (one voxel per thread), 1 (two) or 2 (TMA ring)")
+            raise ValueError("upd_tile must be 0 or 1 (two voxels per thread) or 2 (TMA ring)")
         geom.validate(subset_num)
         self.geom = geom
         self.params = NrOstrParams(int(subset_num), int(POTENTIALS[potential]),
