@@ -47,8 +47,8 @@ struct CaseDev {
     float* x;
     float* xtmp;
     float* h;
-    const float *d, *y, *b, *r, *angles;
-    const int32_t* index;
+    const float *d, *y, *b, *r;
+    const ProjView* views;
     int* status;
     BpTab T;               // the case's back-projection tables
     int fp_tx, fp_ty;      // detector tiles of 32 x 4 bins
@@ -82,10 +82,11 @@ __device__ __forceinline__ int find_case(const int* off, int n, int it) {
 }
 
 // Projection items [0, hi) of step `step` (hi: the active prefix).  12 resident
-// blocks per SM, as fp_h_kernel.
+// blocks per SM: at fp_h_kernel's 16 the runtime case index spills (four mixed
+// cases: 6.86 against 6.47 ms).
 __global__ void __launch_bounds__(128, 12) fp_batch_kernel(const __grid_constant__ BatchTable P,
                                                            int step, int hi) {
-    __shared__ ViewSrc src;
+    __shared__ float2 rows[4][WALK_ROWS];
     for (int it = blockIdx.x; it < hi; it += gridDim.x) {
         const int p = find_case(P.fp_off, P.n, it);
         const CaseDev& cd = P.c[P.fp_case[p]];
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(128, 12) fp_batch_kernel(const __grid_constant
         const int a0 = (step % (int)cd.M) * cd.Vs;
         const float* cur = (step & 1) ? cd.xtmp : cd.x;
         const Geo G = cd.G;  // copied once per item, as in update_batch_kernel
-        fp_h_tile(G, cur, cd.h, cd.angles, cd.index, a0, cd.y, cd.b, cd.r, bx, by, bz, src);
+        fp_h_tile(G, cur, cd.h, cd.views, a0, cd.y, cd.b, cd.r, bx, by, bz, rows);
     }
 }
 
@@ -146,8 +147,8 @@ __global__ void finish_kernel(const __grid_constant__ BatchTable P) {
 // Workspace section pointers of one case (the layout of ostr.cu).
 nr_status ostr_sections(const nr_geom* g, const nr_ostr_params* p, void* ws, size_t bytes,
                         float** xtmp, float** h, const float** d, const float** y,
-                        const float** b, const float** r, const float** angles,
-                        const int32_t** index, int** status, BpTab* tab);
+                        const float** b, const float** r, const ProjView** views, int** status,
+                        BpTab* tab);
 
 // A table written by nr_batch_prepare: its counts and offsets are consistent
 // (a table from anywhere else is refused).
@@ -223,7 +224,7 @@ NR_API nr_status nr_batch_prepare(const nr_batch_case* cases, int32_t n_cases, v
         const nr_batch_case& k = cases[order[c]];
         CaseDev& d = P->c[c];
         st = ostr_sections(&k.g, &k.p, k.workspace, k.ws_bytes, &d.xtmp, &d.h, &d.d, &d.y, &d.b,
-                           &d.r, &d.angles, &d.index, &d.status, &d.T);
+                           &d.r, &d.views, &d.status, &d.T);
         if (st != NR_OK) {
             delete P;
             return st;

@@ -4,8 +4,9 @@
 // column j (lanes along i, the detector x axis).  Adjacent lanes trace nearly
 // parallel rays 1 bin apart in x, so at every step their volume reads fall on
 // the same few 128-byte lines of one volume row (the volume is x-fastest):
-// the gathers coalesce.  Views of a launch run on gridDim.z.  The walk itself
-// is in siddon.cuh.
+// the gathers coalesce.  Views of a launch run on gridDim.z.  The subset loops
+// walk by rows (walk.cuh), the reference-shaped calls ray by ray (siddon.cuh),
+// which keeps their results to the last bit.
 #include <cudaTypedefs.h>
 
 #include "project.cuh"
@@ -112,21 +113,22 @@ __global__ void __launch_bounds__(256) fp_4r_kernel(const __grid_constant__ Geo 
 }
 
 // Fused forward projection + h, one block per 32 x 4 bins of one subset view;
-// K Siddon steps per gather round.  The walk waits on its volume gathers, so
-// residency pays: 12 blocks per SM (40 registers, no spills) run it 5 % faster
-// on the clinical workload than the 10 that 48 registers allow (K = 8 needs
-// more registers and keeps 8).
+// K Siddon steps per gather round.  Clinical workload, per view: 0.163 ms with
+// the three-axis walk of siddon.cuh at 12 blocks per SM (145 M warp
+// instructions, 74 % issue-active), 0.151 with the row lists but each block's
+// view computed by one of its threads (107 M, 59 %: a fifth of the warps' time
+// at that barrier), 0.122 with the views from the workspace (100 M, 69 %) and
+// 0.117 at FP_BLOCKS = 16.
 template <int K>
-__global__ void __launch_bounds__(128, (K >= 8 ? 8 : 12)) fp_h_kernel(const __grid_constant__ Geo G,
+__global__ void __launch_bounds__(128, (K >= 8 ? 8 : FP_BLOCKS)) fp_h_kernel(const __grid_constant__ Geo G,
                                                    const float* __restrict__ vol,
                                                    float* __restrict__ h,
-                                                   const float* __restrict__ angles,
-                                                   const int32_t* __restrict__ index, int a0,
+                                                   const ProjView* __restrict__ views, int a0,
                                                    const float* __restrict__ y,
                                                    const float* __restrict__ b,
                                                    const float* __restrict__ r) {
-    __shared__ ViewSrc src;
-    fp_h_tile<K>(G, vol, h, angles, index, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z, src);
+    __shared__ float2 rows[4][WALK_ROWS];
+    fp_h_tile<K>(G, vol, h, views, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z, rows);
 }
 
 // fp_h_kernel with the subset's FP64 data term: one partial per block in red
@@ -135,15 +137,14 @@ template <int K>
 __global__ void __launch_bounds__(128) fp_h_data_kernel(const __grid_constant__ Geo G,
                                                         const float* __restrict__ vol,
                                                         float* __restrict__ h,
-                                                        const float* __restrict__ angles,
-                                                        const int32_t* __restrict__ index, int a0,
+                                                        const ProjView* __restrict__ views, int a0,
                                                         const float* __restrict__ y,
                                                         const float* __restrict__ b,
                                                         const float* __restrict__ r,
                                                         double* __restrict__ red) {
-    __shared__ ViewSrc src;
-    fp_h_tile<K, true>(G, vol, h, angles, index, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z,
-                       src, red);
+    __shared__ float2 rows[4][WALK_ROWS];
+    fp_h_tile<K, true>(G, vol, h, views, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z, rows,
+                       red);
 }
 
 __global__ void __launch_bounds__(1024) partials_sum_kernel(const double* __restrict__ red,
@@ -161,15 +162,13 @@ __global__ void __launch_bounds__(1024) partials_sum_kernel(const double* __rest
 template <int K, int SZ>
 __global__ void __launch_bounds__(128, (SZ >= 4 ? 6 : 10)) fp_h_slab_kernel(
     const __grid_constant__ Geo G, const __grid_constant__ CUtensorMap map,
-    const float* __restrict__ vol, float* __restrict__ h, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, int a0, const float* __restrict__ y,
-    const float* __restrict__ b, const float* __restrict__ r, int* __restrict__ status) {
+    const float* __restrict__ vol, float* __restrict__ h, const ProjView* __restrict__ views,
+    int a0, const float* __restrict__ y, const float* __restrict__ b,
+    const float* __restrict__ r, int* __restrict__ status) {
     extern __shared__ __align__(128) float sbuf[];
     __shared__ __align__(8) uint64_t bar[2];
-    __shared__ ViewSrc src;
     __shared__ SlabBox box[2];
-    fp_h_slab_tile<K, SZ>(G, &map, vol, h, angles, index, a0, y, b, r, status, sbuf, src, box,
-                          bar);
+    fp_h_slab_tile<K, SZ>(G, &map, vol, h, views, a0, y, b, r, status, sbuf, box, bar);
 }
 
 // gamma * yry for every view in one pass (the d precompute's detector term,
@@ -352,8 +351,7 @@ bool volume_map_nan(const nr_geom& g, const float* x, int bx, int by, int bz, CU
 // premap: x's descriptor when the caller encoded it already (slab_map), else
 // nullptr (encoded here when staging applies).
 nr_status launch_fp_h(const nr_geom& g, int k, int stage, const float* x, float* h,
-                      const float* angles, const int32_t* index, int a0, int nviews,
-                      const float* y, const float* b, const float* r, int* status,
+                      const ProjView* views, int a0, int nviews, const float* y, const float* b, const float* r, int* status,
                       const CUtensorMap* premap, cudaStream_t st) {
     dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), nviews);
     const Geo G = make_geo(g);
@@ -370,39 +368,51 @@ nr_status launch_fp_h(const nr_geom& g, int k, int stage, const float* x, float*
     if (staged) {
         const size_t smem = 2 * SlabCfg<SLAB_Z>::BYTES;
         if (k == 2)
-            fp_h_slab_kernel<2, SLAB_Z><<<grd, blk, smem, st>>>(G, map, x, h, angles, index, a0,
+            fp_h_slab_kernel<2, SLAB_Z><<<grd, blk, smem, st>>>(G, map, x, h, views, a0,
                                                                 y, b, r, status);
         else
-            fp_h_slab_kernel<4, SLAB_Z><<<grd, blk, smem, st>>>(G, map, x, h, angles, index, a0,
+            fp_h_slab_kernel<4, SLAB_Z><<<grd, blk, smem, st>>>(G, map, x, h, views, a0,
                                                                 y, b, r, status);
         return launch_status();
     }
     if (k == 2)
-        fp_h_kernel<2><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r);
+        fp_h_kernel<2><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
     else if (k == 8)
-        fp_h_kernel<8><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r);
+        fp_h_kernel<8><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
     else
-        fp_h_kernel<4><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r);
+        fp_h_kernel<4><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
     return launch_status();
 }
 
 // The fused projection of launch_fp_h (direct gathers, K steps per round)
 // with the subset's FP64 data term into out[0]; red holds red_n partials.
 nr_status launch_fp_h_data(const nr_geom& g, int k, const float* x, float* h,
-                           const float* angles, const int32_t* index, int a0, int nviews,
-                           const float* y, const float* b, const float* r, double* red,
+                           const ProjView* views, int a0, int nviews, const float* y, const float* b, const float* r, double* red,
                            int64_t red_n, double* out, cudaStream_t st) {
     dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), nviews);
     const int64_t n = (int64_t)grd.x * grd.y * grd.z;
     if (n > red_n) return NR_ERR_WORKSPACE;
     const Geo G = make_geo(g);
     if (k == 2)
-        fp_h_data_kernel<2><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r, red);
+        fp_h_data_kernel<2><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r, red);
     else if (k == 8)
-        fp_h_data_kernel<8><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r, red);
+        fp_h_data_kernel<8><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r, red);
     else
-        fp_h_data_kernel<4><<<grd, blk, 0, st>>>(G, x, h, angles, index, a0, y, b, r, red);
+        fp_h_data_kernel<4><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r, red);
     partials_sum_kernel<<<1, 1024, 0, st>>>(red, n, out);
+    return launch_status();
+}
+
+// The views of a plan, subset order (angles[index[a]]).
+__global__ void views_kernel(const __grid_constant__ Geo G, const float* __restrict__ angles,
+                             const int32_t* __restrict__ index, ProjView* __restrict__ views) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a < G.g.n_angles) proj_view(G, angles[index[a]], views[a]);
+}
+
+nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
+                       ProjView* views, cudaStream_t st) {
+    views_kernel<<<cdiv(g.n_angles, 32), 32, 0, st>>>(make_geo(g), angles, index, views);
     return launch_status();
 }
 

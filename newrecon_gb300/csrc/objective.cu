@@ -17,27 +17,26 @@
 #include <utility>
 
 #include "reduce.cuh"
-#include "siddon.cuh"
+#include "walk.cuh"
 
 namespace nr {
 
 __global__ void __launch_bounds__(128) data_term_kernel(
-    const __grid_constant__ Geo G, const float* __restrict__ x, const float* __restrict__ angles,
-    const int32_t* __restrict__ index, const float* __restrict__ y, const float* __restrict__ b,
+    const __grid_constant__ Geo G, const float* __restrict__ x,
+    const ProjView* __restrict__ views, const float* __restrict__ y, const float* __restrict__ b,
     const float* __restrict__ r, double* __restrict__ red) {
-    __shared__ ViewSrc src;
+    __shared__ float2 rows[4][WALK_ROWS];
     const nr_geom& g = G.g;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int a = blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ProjView& view = views[a];
     double term = 0.0;
-    if (i < g.nbx && j < g.nby) {
-        float v;
-        float l = 0.f;
-        if (trace<0>(G, x, src.x0, src.y0, src.z0, bin_x(g, i), bin_y(g, j), -g.detectorR, &v))
-            l = v * src.ct;
+    float v, l = 0.f;
+    const bool on = i < g.nbx && j < g.nby;
+    if (line_integral<4>(G, x, view, bin_x(g, i), bin_y(g, j), on, rows[threadIdx.y], &v))
+        l = v * view.src.ct;
+    if (on) {
         const int64_t o = (int64_t)a * g.nbx * g.nby + (int64_t)j * g.nbx + i;
         const double yb = (double)b[o] * exp(-(double)l);
         const double m = yb + (r ? (double)r[o] : 0.0);
@@ -241,15 +240,14 @@ nr_status launch_penalty(const nr_geom& g, int pot, float delta, const float* x,
 }
 
 nr_status launch_objective(const nr_geom& g, int pot, float delta, const float* x,
-                           const float* angles, const int32_t* index, const float* y,
-                           const float* b, const float* r, double* red, int64_t red_n,
-                           double* out, cudaStream_t st) {
+                           const ProjView* views, const float* y, const float* b, const float* r,
+                           double* red, int64_t red_n, double* out, cudaStream_t st) {
     const int64_t nd = data_blocks(g), np = pen_blocks(g);
     if (nd + np > red_n) return NR_ERR_WORKSPACE;
     const Geo G = make_geo(g);
     {
         dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), g.n_angles);
-        data_term_kernel<<<grd, blk, 0, st>>>(G, x, angles, index, y, b, r, red);
+        data_term_kernel<<<grd, blk, 0, st>>>(G, x, views, y, b, r, red);
     }
     {
         dim3 blk(32, 4), grd(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz);

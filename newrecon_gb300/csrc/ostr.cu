@@ -7,6 +7,7 @@
 //   red      double[red_n]              per-block partial sums of the objective
 //   index    int32[A]                   view order (subset-major)
 //   angles   float[A]
+//   views    ProjView[A]                projection constants, subset order (walk.cuh)
 //   y, b, r  float[A][BINSy][BINSx]     scan in subset order, detector i fastest
 //   d        float[N]                   curvature denominators
 //   xtmp     float[N]                   second volume buffer (ping-pong)
@@ -17,12 +18,13 @@
 #include <cuda.h>
 
 #include "update.cuh"
+#include "walk.cuh"
 
 namespace nr {
 
 nr_status launch_fp_h(const nr_geom& g, int k, int stage, const float* x, float* h,
-                      const float* angles, const int32_t* index, int a0, int nviews,
-                      const float* y, const float* b, const float* r, int* status,
+                      const ProjView* views, int a0, int nviews, const float* y, const float* b,
+                      const float* r, int* status,
                       const CUtensorMap* premap, cudaStream_t st);
 bool slab_map(const nr_geom& g, const float* x, CUtensorMap* map);
 nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const float* angles,
@@ -43,23 +45,25 @@ static bool update_map(const nr_geom& g, const nr_ostr_params& p, const float* x
     return p.upd_tile == NR_TILE_TMA && volume_map_nan(g, x, UTW, USH, 1, map);
 }
 nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t* index,
-                           float4* tx, float4* ty, cudaStream_t st);
+                           float4* tx, float4* ty, bool scaled, cudaStream_t st);
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,
                            int Vs, cudaStream_t st);
+nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
+                       ProjView* views, cudaStream_t st);
 nr_status launch_objective(const nr_geom& g, int pot, float delta, const float* x,
-                           const float* angles, const int32_t* index, const float* y,
+                           const ProjView* views, const float* y,
                            const float* b, const float* r, double* red, int64_t red_n,
                            double* out, cudaStream_t st);
 int64_t objective_partials(const nr_geom& g);
 nr_status launch_fp_h_data(const nr_geom& g, int k, const float* x, float* h,
-                           const float* angles, const int32_t* index, int a0, int nviews,
-                           const float* y, const float* b, const float* r, double* red,
+                           const ProjView* views, int a0, int nviews, const float* y,
+                           const float* b, const float* r, double* red,
                            int64_t red_n, double* out, cudaStream_t st);
 nr_status launch_penalty(const nr_geom& g, int pot, float delta, const float* x, double* red,
                          int64_t red_n, double* out, cudaStream_t st);
 
 struct Layout {
-    size_t status, red, index, angles, y, b, r, d, xtmp, h, bpx, bpy, gc, gr, total;
+    size_t status, red, index, angles, views, y, b, r, d, xtmp, h, bpx, bpy, gc, gr, total;
     int64_t red_n;
 };
 
@@ -81,6 +85,7 @@ static Layout layout(const nr_geom& g, const nr_ostr_params& p) {
     L.red = take((size_t)L.red_n * sizeof(double));
     L.index = take(A * sizeof(int32_t));
     L.angles = take(A * sizeof(float));
+    L.views = take(A * sizeof(ProjView));
     L.y = take(A * B * sizeof(float));
     L.b = take(A * B * sizeof(float));
     L.r = p.has_scatter ? take(A * B * sizeof(float)) : (size_t)-1;
@@ -99,6 +104,7 @@ struct WS {
     int* status;
     double* red;
     int32_t* index;
+    ProjView* views;
     float *angles, *y, *b, *r, *d, *xtmp, *h, *gc, *gr;
     float4 *bpx, *bpy;
     int64_t red_n;
@@ -112,6 +118,7 @@ static WS carve(void* base, const Layout& L) {
     w.red = (double*)(c + L.red);
     w.index = (int32_t*)(c + L.index);
     w.angles = (float*)(c + L.angles);
+    w.views = (ProjView*)(c + L.views);
     w.y = (float*)(c + L.y);
     w.b = (float*)(c + L.b);
     w.r = L.r == (size_t)-1 ? nullptr : (float*)(c + L.r);
@@ -190,8 +197,8 @@ nr_status launch_clear_status(int* status, cudaStream_t s) {
 // Section pointers of a set-up workspace, for the batched path (batch.cu).
 nr_status ostr_sections(const nr_geom* g, const nr_ostr_params* p, void* ws, size_t bytes,
                         float** xtmp, float** h, const float** d, const float** y,
-                        const float** b, const float** r, const float** angles,
-                        const int32_t** index, int** status, BpTab* tab) {
+                        const float** b, const float** r, const ProjView** views, int** status,
+                        BpTab* tab) {
     Layout L;
     nr_status st = check_ws(g, p, ws, bytes, &L);
     if (st != NR_OK) return st;
@@ -202,8 +209,7 @@ nr_status ostr_sections(const nr_geom* g, const nr_ostr_params* p, void* ws, siz
     *y = w.y;
     *b = w.b;
     *r = w.r;
-    *angles = w.angles;
-    *index = w.index;
+    *views = w.views;
     *status = w.status;
     *tab = w.tab();
     return NR_OK;
@@ -243,7 +249,8 @@ NR_API nr_status nr_ostr_setup(const nr_geom* g, const nr_ostr_params* p, const 
     clear_status_kernel<<<1, 64, 0, s>>>(w.status);
     index_kernel<<<1, 256, 0, s>>>(w.index, angles, w.angles, A, M);
     if ((st = launch_status()) != NR_OK) return st;
-    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, s)) != NR_OK) return st;
+    if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
+    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, true, s)) != NR_OK) return st;
     // [view][i][j] original order -> [view][j][i] subset order.
     if ((st = launch_transpose(w.y, prj, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
     if ((st = launch_transpose(w.b, blank, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
@@ -272,7 +279,7 @@ NR_API nr_status nr_ostr_project(const nr_geom* g, const nr_ostr_params* p, cons
     if (!x || subset < 0 || subset >= p->subset_num) return NR_ERR_BAD_ARGUMENT;
     WS w = carve(workspace, L);
     const int Vs = g->n_angles / p->subset_num;
-    return launch_fp_h(*g, p->fp_batch, p->fp_stage, x, w.h, w.angles, w.index, subset * Vs, Vs, w.y, w.b, w.r, w.status, nullptr,
+    return launch_fp_h(*g, p->fp_batch, p->fp_stage, x, w.h, w.views, subset * Vs, Vs, w.y, w.b, w.r, w.status, nullptr,
                        as_stream(stream));
 }
 
@@ -324,7 +331,7 @@ NR_API nr_status nr_ostr_subiter(const nr_geom* g, const nr_ostr_params* p, floa
     const int A = g->n_angles, M = p->subset_num, Vs = A / M;
     const int64_t N = (int64_t)g->nx * g->ny * g->nz;
     const int a0 = subset * Vs;
-    if ((st = launch_fp_h(*g, p->fp_batch, p->fp_stage, x, w.h, w.angles, w.index, a0, Vs, w.y, w.b, w.r, w.status, nullptr, s)) != NR_OK)
+    if ((st = launch_fp_h(*g, p->fp_batch, p->fp_stage, x, w.h, w.views, a0, Vs, w.y, w.b, w.r, w.status, nullptr, s)) != NR_OK)
         return st;
     CUtensorMap map;
     const bool mapped = update_map(*g, *p, x, &map);
@@ -354,7 +361,7 @@ static nr_status enqueue_iterations(const nr_geom* g, const nr_ostr_params* p, f
     for (int it = 0; it < n_iters; it++) {
         for (int a = 0; a < M; a++) {
             const int a0 = a * Vs;
-            if ((st = launch_fp_h(*g, p->fp_batch, p->fp_stage, cur, w.h, w.angles, w.index, a0, Vs, w.y, w.b, w.r, w.status,
+            if ((st = launch_fp_h(*g, p->fp_batch, p->fp_stage, cur, w.h, w.views, a0, Vs, w.y, w.b, w.r, w.status,
                                   staged ? &maps[cur == x ? 0 : 1] : nullptr, s)) !=
                 NR_OK)
                 return st;
@@ -420,7 +427,7 @@ NR_API nr_status nr_ostr_objective(const nr_geom* g, const nr_ostr_params* p, co
     if (st != NR_OK) return st;
     if (!x || !out) return NR_ERR_BAD_ARGUMENT;
     WS w = carve(workspace, L);
-    return launch_objective(*g, p->potential, p->delta, x, w.angles, w.index, w.y, w.b, w.r, w.red,
+    return launch_objective(*g, p->potential, p->delta, x, w.views, w.y, w.b, w.r, w.red,
                             w.red_n, out, as_stream(stream));
 }
 
@@ -433,7 +440,7 @@ NR_API nr_status nr_ostr_project_fp64(const nr_geom* g, const nr_ostr_params* p,
     if (!x || !data_out || subset < 0 || subset >= p->subset_num) return NR_ERR_BAD_ARGUMENT;
     WS w = carve(workspace, L);
     const int Vs = g->n_angles / p->subset_num;
-    return launch_fp_h_data(*g, p->fp_batch, x, w.h, w.angles, w.index, subset * Vs, Vs, w.y,
+    return launch_fp_h_data(*g, p->fp_batch, x, w.h, w.views, subset * Vs, Vs, w.y,
                             w.b, w.r, w.red, w.red_n, data_out, as_stream(stream));
 }
 

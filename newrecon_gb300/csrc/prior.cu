@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128) bp_table_kernel(const __grid_constant__ G
                                                        const float* __restrict__ angles,
                                                        const int32_t* __restrict__ index,
                                                        float4* __restrict__ tx,
-                                                       float4* __restrict__ ty) {
+                                                       float4* __restrict__ ty, bool scaled) {
     __shared__ ViewSrc src;
     const nr_geom& g = G.g;
     const int a = blockIdx.z, z = blockIdx.y;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128) bp_table_kernel(const __grid_constant__ G
     const float z1 = vox_z(g, z);
     const float tt = bp_tt(g, src, z1);
     const float inv_bx = 1.f / g.bx, inv_by = 1.f / g.by;
-    const float k = __fdiv_rn(1.f, g.vz * src.s2);
+    const float k = scaled ? __fdiv_rn(1.f, g.vz * src.s2) : 1.f;
     const int64_t row = (int64_t)a * g.nz + z;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.nx + g.ny;
          q += gridDim.x * blockDim.x) {
@@ -170,9 +170,9 @@ size_t bp_table_bytes(const nr_geom& g) {
 }
 
 nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t* index,
-                           float4* tx, float4* ty, cudaStream_t st) {
+                           float4* tx, float4* ty, bool scaled, cudaStream_t st) {
     dim3 grd(cdiv((int64_t)g.nx + g.ny, 128), g.nz, g.n_angles);
-    bp_table_kernel<<<grd, 128, 0, st>>>(make_geo(g), angles, index, tx, ty);
+    bp_table_kernel<<<grd, 128, 0, st>>>(make_geo(g), angles, index, tx, ty, scaled);
     return launch_status();
 }
 

@@ -4,9 +4,14 @@
 #pragma once
 
 #include "reduce.cuh"
-#include "siddon.cuh"
+#include "walk.cuh"
 
 namespace nr {
+
+// Resident blocks (128 threads) per SM of the projections in the subset loops:
+// the walk waits on its volume gathers, so residency pays (32 registers; 12
+// blocks of 40 registers are 1.5 % slower on the clinical workload).
+constexpr int FP_BLOCKS = 16;
 
 // Detector offset of bin (i, j) of one view: JI -> [j][i] (i fastest, the
 // layout of the fused path and of the scanner files); otherwise [i][j] (the
@@ -22,8 +27,9 @@ __device__ __forceinline__ int64_t bin_off(const nr_geom& g, int i, int j) {
 // volume have line = 0 (the reference zeroes the line buffer every subset,
 // Tomo_OSTR_gold.cpp:843).  h = (y/(b e^-l + r) - 1) b e^-l,
 // Tomo_OSTR_gold.cpp:245-260.
-// One block of 32 x 4 bins (bx, by) of subset view bz.  Every thread of the
-// block must call it (it synchronises once, twice with DATA).
+// One block of 32 x 4 bins (bx, by) of subset view bz, a warp per detector row.
+// Every thread of the block must call it (with DATA it synchronises the block).
+// views: the plan's views in subset order; rows: the warps' lists (walk.cuh).
 //
 // DATA: also the subset's FP64 data term, sum over its bins of
 // ybar + r - y log(ybar + r) with ybar = b exp(-l) -- the data term of the
@@ -32,26 +38,24 @@ __device__ __forceinline__ int64_t bin_off(const nr_geom& g, int i, int j) {
 // then a fixed-order block sum).
 template <int K = 4, bool DATA = false>
 __device__ __forceinline__ void fp_h_tile(const Geo& G, const float* __restrict__ vol,
-                                          float* __restrict__ h, const float* __restrict__ angles,
-                                          const int32_t* __restrict__ index, int a0,
+                                          float* __restrict__ h,
+                                          const ProjView* __restrict__ views, int a0,
                                           const float* __restrict__ y, const float* __restrict__ b,
                                           const float* __restrict__ r, int bx, int by, int bz,
-                                          ViewSrc& src, double* __restrict__ red = nullptr) {
+                                          float2 (*rows)[WALK_ROWS],
+                                          double* __restrict__ red = nullptr) {
     const nr_geom& g = G.g;
     const int a = a0 + bz;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ProjView& view = views[a];
     const int i = bx * 32 + threadIdx.x;
     const int j = by * 4 + threadIdx.y;
     const bool on = i < g.nbx && j < g.nby;
-    if (!DATA && !on) return;
+    if (!DATA && j >= g.nby) return;
     double term = 0.0;
+    float v, l = 0.f;
+    if (line_integral<K>(G, vol, view, bin_x(g, i), bin_y(g, j), on, rows[threadIdx.y], &v))
+        l = v * view.src.ct;
     if (on) {
-        float v = 0.f;
-        float l = 0.f;
-        if (trace<0, K>(G, vol, src.x0, src.y0, src.z0, bin_x(g, i), bin_y(g, j), -g.detectorR,
-                        &v))
-            l = v * src.ct;
         const int64_t B = (int64_t)g.nbx * g.nby;
         const int64_t o = (int64_t)a * B + bin_off<true>(g, i, j);
         const float yb = b[o] * expf(-l);

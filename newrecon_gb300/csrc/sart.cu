@@ -27,6 +27,7 @@
 //   status int32[64]
 //   index  int32[A]                   view order (subset-major)
 //   angles float[A]
+//   views  ProjView[A]                projection constants, subset order (walk.cuh)
 //   p      float[A][BINSy][BINSx]     line integrals, subset order, i fastest
 //   norm   float[A][BINSy][BINSx]     chord lengths, same layout
 //   diff   float[Vs][BINSy][BINSx]    the subset's normalised difference
@@ -42,13 +43,15 @@ nr_status launch_subset_index(int32_t* idx, const float* angles_in, float* angle
 nr_status launch_clear_status(int* status, cudaStream_t s);
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,
                            int Vs, cudaStream_t st);
+nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
+                       ProjView* views, cudaStream_t st);
 nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t* index,
-                           float4* tx, float4* ty, cudaStream_t st);
+                           float4* tx, float4* ty, bool scaled, cudaStream_t st);
 
 namespace {
 
 struct SartLayout {
-    size_t status, index, angles, p, norm, diff, xtmp, bpx, bpy, total;
+    size_t status, index, angles, views, p, norm, diff, xtmp, bpx, bpy, total;
 };
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -67,6 +70,7 @@ SartLayout sart_layout(const nr_geom& g, const nr_sart_params& p) {
     L.status = take(64 * sizeof(int32_t));
     L.index = take(A * sizeof(int32_t));
     L.angles = take(A * sizeof(float));
+    L.views = take(A * sizeof(ProjView));
     L.p = take(A * B * sizeof(float));
     L.norm = take(A * B * sizeof(float));
     L.diff = take((Vs * B + bp_pad(g)) * sizeof(float));  // + zeros the tap pairs may reach
@@ -80,6 +84,7 @@ SartLayout sart_layout(const nr_geom& g, const nr_sart_params& p) {
 struct SartWS {
     int* status;
     int32_t* index;
+    ProjView* views;
     float *angles, *p, *norm, *diff, *xtmp;
     float4 *bpx, *bpy;
 };
@@ -90,6 +95,7 @@ SartWS sart_carve(void* base, const SartLayout& L) {
     w.status = (int*)(c + L.status);
     w.index = (int32_t*)(c + L.index);
     w.angles = (float*)(c + L.angles);
+    w.views = (ProjView*)(c + L.views);
     w.p = (float*)(c + L.p);
     w.norm = (float*)(c + L.norm);
     w.diff = (float*)(c + L.diff);
@@ -132,13 +138,10 @@ nr_status sart_check_ws(const nr_geom* g, const nr_sart_params* p, void* ws, siz
 // that miss the volume (so their difference is 0).
 __global__ void __launch_bounds__(128) sart_norm_kernel(const __grid_constant__ Geo G,
                                                         float* __restrict__ norm,
-                                                        const float* __restrict__ angles,
-                                                        const int32_t* __restrict__ index) {
-    __shared__ ViewSrc src;
+                                                        const ProjView* __restrict__ views) {
     const nr_geom& g = G.g;
     const int a = blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ViewSrc& src = views[a].src;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.nbx || j >= g.nby) return;
@@ -148,18 +151,18 @@ __global__ void __launch_bounds__(128) sart_norm_kernel(const __grid_constant__ 
     norm[(int64_t)a * g.nbx * g.nby + bin_off<true>(g, i, j)] = v;
 }
 
-// diff = (p - FP(x) [cos]) / norm for the subset views [a0, a0 + gridDim.z);
-// 12 resident blocks per SM, as fp_h_kernel.
+// diff = (p - FP(x) [cos]) / norm for the subset views [a0, a0 + gridDim.z); 12
+// resident blocks per SM.  The walk is siddon.cuh's, the one that measured the
+// chord norm: for a ray that cuts a corner of the volume the ratio needs both
+// ends of the two to the last bit.
 template <int K, bool COS>
 __global__ void __launch_bounds__(128, (K >= 8 ? 8 : 12)) sart_fp_diff_kernel(
     const __grid_constant__ Geo G, const float* __restrict__ vol, float* __restrict__ diff,
-    const float* __restrict__ angles, const int32_t* __restrict__ index, int a0,
-    const float* __restrict__ p, const float* __restrict__ norm) {
-    __shared__ ViewSrc src;
+    const ProjView* __restrict__ views, int a0, const float* __restrict__ p,
+    const float* __restrict__ norm) {
     const nr_geom& g = G.g;
     const int a = a0 + blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ViewSrc& src = views[a].src;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.nbx || j >= g.nby) return;
@@ -206,38 +209,33 @@ __device__ __forceinline__ bool sub_ray_merge(const Geo& G, const float* __restr
 
 __global__ void __launch_bounds__(256) sart_norm_4r_kernel(const __grid_constant__ Geo G,
                                                            float* __restrict__ norm,
-                                                           const float* __restrict__ angles,
-                                                           const int32_t* __restrict__ index) {
-    __shared__ ViewSrc src;
+                                                           const ProjView* __restrict__ views) {
     __shared__ float tile[8][33];
     const nr_geom& g = G.g;
     const int a = blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ProjView& view = views[a];
     float m;
     int i, j;
-    if (sub_ray_merge<1>(G, nullptr, src, tile, &m, &i, &j))
+    if (sub_ray_merge<1>(G, nullptr, view.src, tile, &m, &i, &j))
         norm[(int64_t)a * g.nbx * g.nby + bin_off<true>(g, i, j)] = m;
 }
 
 template <bool COS>
 __global__ void __launch_bounds__(256) sart_fp_diff_4r_kernel(
     const __grid_constant__ Geo G, const float* __restrict__ vol, float* __restrict__ diff,
-    const float* __restrict__ angles, const int32_t* __restrict__ index, int a0,
-    const float* __restrict__ p, const float* __restrict__ norm) {
-    __shared__ ViewSrc src;
+    const ProjView* __restrict__ views, int a0, const float* __restrict__ p,
+    const float* __restrict__ norm) {
     __shared__ float tile[8][33];
     const nr_geom& g = G.g;
     const int a = a0 + blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[index[a]]);
-    __syncthreads();
+    const ProjView& view = views[a];
     float m;
     int i, j;
-    if (!sub_ray_merge<0>(G, vol, src, tile, &m, &i, &j)) return;
+    if (!sub_ray_merge<0>(G, vol, view.src, tile, &m, &i, &j)) return;
     const int64_t B = (int64_t)g.nbx * g.nby;
     const int64_t off = bin_off<true>(g, i, j);
     const float nv = norm[(int64_t)a * B + off];
-    const float est = COS ? m * src.ct : m;
+    const float est = COS ? m * view.src.ct : m;
     diff[(int64_t)blockIdx.z * B + off] = nv != 0.f ? __fdiv_rn(p[(int64_t)a * B + off] - est, nv)
                                                     : 0.f;
 }
@@ -246,11 +244,11 @@ template <int KIND, int ZC, int NV>
 __global__ void __launch_bounds__(UNT, UPD_BLOCKS) sart_update_kernel(
     const __grid_constant__ Geo G, const __grid_constant__ PriorW5 W,
     const float* __restrict__ x, float* __restrict__ x_out, const float* __restrict__ diff,
-    const __grid_constant__ BpTab T, int a0, int nv, float lambda, float beta, float delta,
-    int* __restrict__ status) {
+    const __grid_constant__ BpTab T, const ProjView* __restrict__ views, int a0, int nv,
+    float lambda, float beta, float delta, int* __restrict__ status) {
     update_tile<NR_POT_HYPERBOLA, ZC, KIND, NV>(G, W, x, x_out, nullptr, diff, T, a0, nv, lambda,
                                                 beta, delta, status, blockIdx.x, blockIdx.y,
-                                                blockIdx.z);
+                                                blockIdx.z, views);
 }
 
 namespace {
@@ -261,19 +259,19 @@ nr_status launch_fp_diff_c(const nr_geom& g, int k, const float* x, const SartWS
     const Geo G = make_geo(g);
     if (ss) {
         dim3 blk(32, 8), grd(cdiv(2 * (int64_t)g.nbx, 32), cdiv(2 * (int64_t)g.nby, 8), nv);
-        sart_fp_diff_4r_kernel<COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.angles, w.index, a0, w.p,
+        sart_fp_diff_4r_kernel<COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.views, a0, w.p,
                                                          w.norm);
         return launch_status();
     }
     dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), nv);
     if (k == 2)
-        sart_fp_diff_kernel<2, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.angles, w.index, a0, w.p,
+        sart_fp_diff_kernel<2, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.views, a0, w.p,
                                                         w.norm);
     else if (k == 8)
-        sart_fp_diff_kernel<8, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.angles, w.index, a0, w.p,
+        sart_fp_diff_kernel<8, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.views, a0, w.p,
                                                         w.norm);
     else
-        sart_fp_diff_kernel<4, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.angles, w.index, a0, w.p,
+        sart_fp_diff_kernel<4, COS><<<grd, blk, 0, s>>>(G, x, w.diff, w.views, a0, w.p,
                                                         w.norm);
     return launch_status();
 }
@@ -288,11 +286,11 @@ nr_status launch_sart_update_t(const nr_geom& g, const nr_sart_params& p, const 
     const PriorW5 W = make_w5(1.f, delta);
     const BpTab T{w.bpx, w.bpy};
     if (nv == 1)
-        sart_update_kernel<KIND, ZC, 1><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, a0, nv,
-                                                            p.lambda, p.beta, delta, w.status);
+        sart_update_kernel<KIND, ZC, 1><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, w.views, a0,
+                                                            nv, p.lambda, p.beta, delta, w.status);
     else
-        sart_update_kernel<KIND, ZC, 0><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, a0, nv,
-                                                            p.lambda, p.beta, delta, w.status);
+        sart_update_kernel<KIND, ZC, 0><<<grd, blk, 0, s>>>(G, W, x, x_out, w.diff, T, w.views, a0,
+                                                            nv, p.lambda, p.beta, delta, w.status);
     return launch_status();
 }
 
@@ -374,7 +372,8 @@ NR_API nr_status nr_sart_setup(const nr_geom* g, const nr_sart_params* p, const 
     const int A = g->n_angles, M = p->subset_num, Vs = A / M;
     if ((st = launch_clear_status(w.status, s)) != NR_OK) return st;
     if ((st = launch_subset_index(w.index, angles, w.angles, A, M, s)) != NR_OK) return st;
-    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, s)) != NR_OK) return st;
+    if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
+    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, false, s)) != NR_OK) return st;
     if (cudaMemsetAsync(w.diff + (int64_t)Vs * g->nbx * g->nby, 0, bp_pad(*g) * sizeof(float),
                         s) != cudaSuccess)
         return NR_ERR_CUDA;
@@ -382,10 +381,10 @@ NR_API nr_status nr_sart_setup(const nr_geom* g, const nr_sart_params* p, const 
     if ((st = launch_transpose(w.p, line, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
     if (p->supersample) {
         dim3 blk(32, 8), grd(cdiv(2 * (int64_t)g->nbx, 32), cdiv(2 * (int64_t)g->nby, 8), A);
-        sart_norm_4r_kernel<<<grd, blk, 0, s>>>(make_geo(*g), w.norm, w.angles, w.index);
+        sart_norm_4r_kernel<<<grd, blk, 0, s>>>(make_geo(*g), w.norm, w.views);
     } else {
         dim3 blk(32, 4), grd(cdiv(g->nbx, 32), cdiv(g->nby, 4), A);
-        sart_norm_kernel<<<grd, blk, 0, s>>>(make_geo(*g), w.norm, w.angles, w.index);
+        sart_norm_kernel<<<grd, blk, 0, s>>>(make_geo(*g), w.norm, w.views);
     }
     return launch_status();
 }

@@ -14,7 +14,7 @@
 // and are never walked.  A slab whose footprint does not fit the box is read
 // from global memory instead (uniform per block).
 //
-// Each thread's Siddon walk is the one of siddon.cuh, resumed slab by slab:
+// Each thread's walk is the one of walk.cuh (or siddon.cuh), resumed slab by slab:
 // the state (distance, crossing counters, next crossings) carries over, a
 // slab's steps stop where the ray leaves the slab's planes, and the segments
 // are accumulated in the same order with the same arithmetic -- the result is
@@ -158,26 +158,49 @@ __device__ __forceinline__ void walk_slab(const float* __restrict__ vals, int& i
     }
 }
 
+// The three axes of the ray to (x1, y1) in the parametrisation of walk.cuh,
+// its first depth s and the crossings counted by then; R.smax its last depth.
+__device__ __forceinline__ bool depth_axes(const nr_geom& g, const WalkView& V, float x1, float y1,
+                                           RayAxes& R, float& s, float& cx, float& cy, float& cz) {
+    const float ex = V.x.at(x1), ey = V.y.at(y1);
+    const DepthAxis X = depth_axis(ex, V.x.slope(x1)), Y = depth_axis(ey, V.y.slope(y1));
+    float lo, hi, w0, w1;
+    depth_range(X, ex, g.nx, lo, hi);
+    depth_range(Y, ey, g.ny, w0, w1);
+    w0 = fmaxf(w0, 0.f);
+    w1 = fminf(w1, (float)g.nz);
+    s = fmaxf(lo, w0);
+    R.smax = fminf(hi, w1);
+    if (!(w0 < w1) || !(s < R.smax)) return false;
+    R.ax = Axis{X.first, X.step, hi, X.i0, X.dir};
+    R.ay = Axis{Y.first, Y.step, w1, Y.i0, Y.dir};
+    R.az = Axis{1.f, 1.f, (float)g.nz, g.nz - 1, -1};
+    cx = (float)depth_first<false>(X, s);
+    cy = (float)depth_first<false>(Y, s);
+    cz = (float)(int)s;
+    return true;
+}
+
 // The slab-staged body of one block (32 x 4 bins of subset view bz).  Every
 // thread of the block runs it (it synchronises once per slab).
 template <int K, int SZ>
 __device__ __forceinline__ void fp_h_slab_tile(const Geo& G, const CUtensorMap* map,
                                                const float* __restrict__ vol,
                                                float* __restrict__ h,
-                                               const float* __restrict__ angles,
-                                               const int32_t* __restrict__ index, int a0,
+                                               const ProjView* __restrict__ views, int a0,
                                                const float* __restrict__ y,
                                                const float* __restrict__ b,
                                                const float* __restrict__ r,
                                                int* __restrict__ status, float* sbuf,
-                                               ViewSrc& src, SlabBox* box, uint64_t* bar) {
+                                               SlabBox* box, uint64_t* bar) {
     const nr_geom& g = G.g;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int a = a0 + blockIdx.z;
+    const ProjView view = views[a];
+    const ViewSrc& src = view.src;
     const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 4;
     const int i1 = min(i0 + 31, g.nbx - 1), j1 = min(j0 + 3, g.nby - 1);
     if (tid == 0) {
-        src = view_source(g, angles[index[a]]);
         tc::mbar_init(&bar[0], 1);
         tc::mbar_init(&bar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -195,14 +218,21 @@ __device__ __forceinline__ void fp_h_slab_tile(const Geo& G, const CUtensorMap* 
     const bool active = i < g.nbx && j < g.nby;
     RayAxes R;
     bool hit = false;
-    if (active)
+    float s = 0.f, sum = 0.f, tx = 0.f, ty = 0.f, tz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+    float scale = 1.f;
+    if (active && view.w.down) {
+        // the walk of walk.cuh: depth as the parameter, each axis counted from
+        // its cell at depth 0
+        hit = depth_axes(g, view.w, bin_x(g, i), bin_y(g, j), R, s, cx, cy, cz);
+        scale = depth_mm(g, src, bin_x(g, i), bin_y(g, j));
+    } else if (active) {
         hit = ray_axes<false>(G, src.x0, src.y0, src.z0, bin_x(g, i), bin_y(g, j),
                               -g.detectorR, R);
-    float s = 0.f, sum = 0.f, tx = 0.f, ty = 0.f, tz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+    }
     if (hit) {
-        tx = R.ax.first;
-        ty = R.ay.first;
-        tz = R.az.first;
+        tx = R.ax.dir ? __fmaf_rn(cx, R.ax.step, R.ax.first) : NR_FINF;
+        ty = R.ay.dir ? __fmaf_rn(cy, R.ay.step, R.ay.first) : NR_FINF;
+        tz = R.az.dir ? __fmaf_rn(cz, R.az.step, R.az.first) : NR_FINF;
     }
     // staged: the block still reads slabs from shared memory.  It turns false
     // (for every thread at once) when a wait gave up twice in some thread;
@@ -275,7 +305,7 @@ __device__ __forceinline__ void fp_h_slab_tile(const Geo& G, const CUtensorMap* 
                 tc::mbar_wait(&bar[q & 1], (q >> 1) & 1, SLAB_WAIT);
     }
     if (!active) return;
-    const float l = hit ? sum * src.ct : 0.f;
+    const float l = hit ? sum * scale * src.ct : 0.f;
     const int64_t B = (int64_t)g.nbx * g.nby;
     const int64_t o = (int64_t)a * B + bin_off<true>(g, i, j);
     const float yb = b[o] * expf(-l);

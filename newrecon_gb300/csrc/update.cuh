@@ -10,8 +10,8 @@
 #include <cmath>
 #include <type_traits>
 
-#include "common.cuh"
 #include "tma.cuh"
+#include "walk.cuh"
 
 namespace nr {
 
@@ -202,7 +202,7 @@ constexpr int UPD_SART_R = 2;   // OS-SART with the hyperbola prior, backprj_OSS
 //   x[(a nz + z) nx + i] = {c, w0, w1, k (x0 - x1)^2}
 //   y[(a nz + z) ny + j] = {r * BINSx, v0, v1, k ((y0 - y1)^2 + (z0 - z1)^2)}
 // with k = 1 / (Vsize_z |source|^2), so that the depth weight times Vsize_z is
-// the reciprocal of the entries' sum.
+// the reciprocal of the entries' sum (OS-SART: k = 1).
 // The bilinear stencil's columns are ilb, ilb + 1 with weights 1 - fracI,
 // fracI; a column off the detector gets weight 0 (the rules of
 // Tomo_OSTR.cu:1684-1715), and c is ilb clamped to [0, BINSx - 2] with the
@@ -289,24 +289,32 @@ __device__ __forceinline__ float4 bp_entry_y(const nr_geom& g, const ViewSrc& vs
     return make_float4(__int_as_float(r * g.nbx), p0, p1, k * (ddy * ddy + ddz * ddz));
 }
 
-// One view's back-projection term of one voxel, added to capL (and, for the
-// OS-SART kinds, the sensitivity), from its table entries ex, ey and the taps
-// q of its pair (c, c + 1) x rows (r, r + 1); off-detector taps are weighted 0
-// and their loads kept in bounds by the tables.
-template <int KIND>
+// One view's back-projection term of one voxel, added to capL, from its table
+// entries ex, ey and the taps of its pair (c, c + 1) x rows (r, r + 1);
+// off-detector taps are weighted 0 and their loads kept in bounds by the
+// tables.
 __device__ __forceinline__ void bp_view(const float* __restrict__ p, const float4 ex,
-                                        const float4 ey, const nr_geom& g, float& capL,
-                                        float& sens) {
+                                        const float4 ey, const nr_geom& g, float& capL) {
     const float* q0 = p + (__float_as_int(ey.x) + __float_as_int(ex.x));
     const float* q1 = q0 + g.nbx;
     const float dw = rcp_approx(ex.w + ey.w);
     const float d1 = __fmaf_rn(ex.z, __ldg(q0 + 1), __fmul_rn(ex.y, __ldg(q0)));
     const float d2 = __fmaf_rn(ex.z, __ldg(q1 + 1), __fmul_rn(ex.y, __ldg(q1)));
     capL = __fmaf_rn(__fmaf_rn(ey.z, d2, __fmul_rn(ey.y, d1)), dw, capL);
-    if (KIND != UPD_OSTR) {  // sensitivity: the same weights on ones
-        const float s1 = ex.y + ex.z;
-        sens = __fmaf_rn(__fmaf_rn(ey.z, s1, __fmul_rn(ey.y, s1)), dw, sens);
-    }
+}
+
+// The OS-SART kinds' term and its sensitivity (the same weights on ones), from
+// tables with k = 1; s2 = |source|^2.
+__device__ __forceinline__ void bp_sart(const float4& ex, const float4& ey, const float (&q)[4],
+                                        float s2, const nr_geom& g, float& capL, float& sens) {
+    const float dw = __fdividef(s2, ex.w + ey.w);
+    float d1 = ex.y * q[0];
+    d1 = d1 + ex.z * q[1];
+    float d2 = ex.y * q[2];
+    d2 = d2 + ex.z * q[3];
+    capL = capL + (ey.y * d1 + ey.z * d2) * g.vz * dw;
+    const float s1 = ex.y + ex.z;
+    sens = sens + (ey.y * s1 + ey.z * s1) * g.vz * dw;
 }
 
 // The value of the OSTR step, xc - (M capL + beta rd) / (dv + 2 beta rdd).
@@ -334,14 +342,12 @@ __device__ __forceinline__ bool not_finite(float v) {
     return !(fabsf(v) < __int_as_float(0x7f800000));
 }
 
-// The update of one voxel from its sums, stored at out (non-finite values
+// The OSTR update of one voxel from its sums, stored at out (non-finite values
 // flagged in status).
-template <int KIND>
-__device__ __forceinline__ void upd_store(float xc, float capL, float sens, float rd, float rdd,
-                                          float dv, float M, float beta, float* __restrict__ out,
+__device__ __forceinline__ void upd_store(float xc, float capL, float rd, float rdd, float dv,
+                                          float M, float beta, float* __restrict__ out,
                                           int* __restrict__ status) {
-    const float xn = KIND == UPD_OSTR ? ostr_step(xc, capL, rd, rdd, dv, M, beta)
-                                      : sart_step<KIND>(xc, capL, sens, rd, M, beta);
+    const float xn = ostr_step(xc, capL, rd, rdd, dv, M, beta);
     if (not_finite(xn)) atomicOr(status, NR_FLAG_NONFINITE);
     *out = xn < 0.f ? 0.f : xn;
 }
@@ -372,19 +378,13 @@ struct UpdView {
         qb[2] = __ldg(b);
         qb[3] = __ldg(b + 1);
     }
-    template <int KIND>
-    __device__ __forceinline__ void add(f32x2& cap, f32x2& sens) const {
+    __device__ __forceinline__ void add(f32x2& cap) const {
         const f32x2 dw = pk2(rcp_approx(ex.w + ea.w), rcp_approx(ex.w + eb.w));
         const f32x2 w0 = pk2(ex.y, ex.y), w1 = pk2(ex.z, ex.z);
         const f32x2 v0 = pk2(ea.y, eb.y), v1 = pk2(ea.z, eb.z);
         const f32x2 d1 = fma2(w1, pk2(qa[1], qb[1]), mul2(w0, pk2(qa[0], qb[0])));
         const f32x2 d2 = fma2(w1, pk2(qa[3], qb[3]), mul2(w0, pk2(qa[2], qb[2])));
         cap = fma2(fma2(v1, d2, mul2(v0, d1)), dw, cap);
-        if (KIND != UPD_OSTR) {
-            const float s = ex.y + ex.z;
-            const f32x2 s2 = pk2(s, s);
-            sens = fma2(fma2(v1, s2, mul2(v0, s2)), dw, sens);
-        }
     }
 };
 
@@ -461,6 +461,47 @@ __device__ __forceinline__ void upd_own_plane(const UpdRows& R, const PriorW5& W
     nb_class2<POT, EDGE, W_DIAG>(b2, R.lr(1), R.lr(3), W, delta, inv_delta, S.sddb, S.sdb);
 }
 
+// The OS-SART prior's gradient of voxels A and B, pair by pair as the sums of
+// update_tile's first form were: the rows' (x - 1, x + 1) pairs plane by plane,
+// then the centre cells' pairs, each term weighted by itself.  The order is
+// kept because this step can amplify a last bit -- lambda beta RD / sens where
+// few rays see a voxel -- until runs that round differently part ways.
+template <bool EDGE, int CLS>
+__device__ __forceinline__ void sart_pair(f32x2 c2, f32x2 n2, const PriorW5& W, f32x2& sd) {
+    f32x2 t2 = sub2(c2, n2);
+    const f32x2 o2 = omega2<NR_POT_HYPERBOLA, EDGE>(t2, W, 0.f, 0.f);
+    sd = fma2(mul2(ld2(W.w[CLS]), o2), t2, sd);
+}
+// The three row pairs of a plane: classes SIDE, MID, SIDE.
+template <bool EDGE, int SIDE, int MID>
+__device__ __forceinline__ void sart_rows(const UpdRows& R, float ca, float cb, const PriorW5& W,
+                                          UpdSums& S) {
+    const f32x2 a2 = pk2(ca, ca), b2 = pk2(cb, cb);
+    sart_pair<EDGE, SIDE>(a2, R.lr(0), W, S.sda);
+    sart_pair<EDGE, SIDE>(b2, R.lr(1), W, S.sdb);
+    sart_pair<EDGE, MID>(a2, R.lr(1), W, S.sda);
+    sart_pair<EDGE, MID>(b2, R.lr(2), W, S.sdb);
+    sart_pair<EDGE, SIDE>(a2, R.lr(2), W, S.sda);
+    sart_pair<EDGE, SIDE>(b2, R.lr(3), W, S.sdb);
+}
+// The centre cells' pairs: cp the plane below, N the voxels' own, F the plane
+// above; lo / hi: the planes are in the volume.
+template <bool EDGE>
+__device__ __forceinline__ void sart_centres(const float (&cp)[4], const UpdRows& N,
+                                             const UpdRows& F, bool lo, bool hi, const PriorW5& W,
+                                             UpdSums& S) {
+    const float ca = N.c[1], cb = N.c[2];
+    const float la = lo ? ca : 0.f, lb = lo ? cb : 0.f, ha = hi ? ca : 0.f, hb = hi ? cb : 0.f;
+    sart_pair<EDGE, W_ZEDGE>(pk2(la, la), pk2(cp[0], cp[2]), W, S.sda);
+    sart_pair<EDGE, W_ZEDGE>(pk2(lb, lb), pk2(cp[1], cp[3]), W, S.sdb);
+    sart_pair<EDGE, W_ZEDGE>(pk2(ha, ha), pk2(F.c[0], F.c[2]), W, S.sda);
+    sart_pair<EDGE, W_ZEDGE>(pk2(hb, hb), pk2(F.c[1], F.c[3]), W, S.sdb);
+    sart_pair<EDGE, W_ZFACE>(pk2(la, ha), pk2(cp[1], F.c[1]), W, S.sda);
+    sart_pair<EDGE, W_ZFACE>(pk2(lb, hb), pk2(cp[2], F.c[2]), W, S.sdb);
+    sart_pair<EDGE, W_FACE>(pk2(ca, ca), pk2(N.c[0], N.c[2]), W, S.sda);
+    sart_pair<EDGE, W_FACE>(pk2(cb, cb), pk2(N.c[1], N.c[3]), W, S.sdb);
+}
+
 // One sub-iteration's update, fused: SBP of h (subset views, [view][j][i]),
 // the penalty, and the update_est step.  Each block owns a 32 x 8 tile of
 // (x, y) columns and walks ZC planes in z; a thread owns two voxels of each
@@ -498,7 +539,8 @@ template <int POT, int ZC = UZC, int KIND = UPD_OSTR, int NV = 0>
 __device__ __forceinline__ void update_tile(
     const Geo& G, const PriorW5& W, const float* __restrict__ x, float* __restrict__ x_out,
     const float* __restrict__ d, const float* __restrict__ h, const BpTab& T, int a0, int nv,
-    float M, float beta, float delta, int* __restrict__ status, int bx, int by, int bz) {
+    float M, float beta, float delta, int* __restrict__ status, int bx, int by, int bz,
+    const ProjView* __restrict__ views = nullptr) {
     const nr_geom& g = G.g;
     const int x0t = bx * UTX, y0t = by * UTY;
     const int ix = x0t + threadIdx.x, iy = y0t + 2 * threadIdx.y;
@@ -528,8 +570,18 @@ __device__ __forceinline__ void update_tile(
     // view's taps are loaded): upd_store's steps, packed for the OSTR kind.
     auto finish = [&](int z, float ca, float cb) {
         const int v = z * plane + at;
-        f32x2 cap = pk2(0.f, 0.f), sens = cap;
-        V.add<KIND>(cap, sens);
+        f32x2 cap = pk2(0.f, 0.f);
+        float capa = 0.f, capb = 0.f, sa = 0.f, sb = 0.f;
+        auto add = [&](int t) {
+            if (KIND == UPD_OSTR) {
+                V.add(cap);
+            } else {
+                const float s2 = __ldg(&views[a0 + t].src.s2);
+                bp_sart(V.ex, V.ea, V.qa, s2, g, capa, sa);
+                bp_sart(V.ex, V.eb, V.qb, s2, g, capb, sb);
+            }
+        };
+        add(0);
         if (NV != 1) {
             const float* p = h;
             int tix = (a0 * g.nz + z) * g.nx + ix;
@@ -541,30 +593,28 @@ __device__ __forceinline__ void update_tile(
                 tiy += sy;
                 V.entries(T, tix, tiy, jb);
                 V.taps(p, g.nbx);
-                V.add<KIND>(cap, sens);
+                add(t);
             }
         }
-        float u, w, rdda, rda, rddb, rdb, xa, xb;
-        upk2(S.sdda, u, w);
-        rdda = u + w;
+        float u, w, rda, rdb, xa, xb;
         upk2(S.sda, u, w);
         rda = u + w;
-        upk2(S.sddb, u, w);
-        rddb = u + w;
         upk2(S.sdb, u, w);
         rdb = u + w;
         if (KIND == UPD_OSTR) {
+            float rdda, rddb;
+            upk2(S.sdda, u, w);
+            rdda = u + w;
+            upk2(S.sddb, u, w);
+            rddb = u + w;
             const f32x2 num = fma2(pk2(-M, -M), cap, mul2(pk2(-beta, -beta), pk2(rda, rdb)));
             const f32x2 den =
                 fma2(pk2(2.f * beta, 2.f * beta), pk2(rdda, rddb), pk2(dva, dvb));
             upk2(den, u, w);
             upk2(fma2(num, pk2(rcp_approx(u), rcp_approx(w)), pk2(ca, cb)), xa, xb);
         } else {
-            float sa, sb;
-            upk2(cap, u, w);
-            upk2(sens, sa, sb);
-            xa = sart_step<KIND>(ca, u, sa, rda, M, beta);
-            xb = sart_step<KIND>(cb, w, sb, rdb, M, beta);
+            xa = sart_step<KIND>(ca, capa, sa, rda, M, beta);
+            xb = sart_step<KIND>(cb, capb, sb, rdb, M, beta);
         }
         if (not_finite(xa) || (has_b && not_finite(xb))) atomicOr(status, NR_FLAG_NONFINITE);
         x_out[v] = xa < 0.f ? 0.f : xa;
@@ -599,22 +649,38 @@ __device__ __forceinline__ void update_tile(
         constexpr bool EDGE = decltype(edge_c)::value;
         // Starts plane z's voxels (rows N; P holds plane z - 1), then loads plane
         // z + 1 into P.
+        float cp[4];   // OS-SART: the centre cells of the plane below
         auto start = [&](UpdRows& P, const UpdRows& N, int z) {
             fetch(z);
             S.sdda = S.sda = S.sddb = S.sdb = pk2(0.f, 0.f);
             // a plane outside the volume (zeros) against zeros: t = 0
-            upd_far_plane<POT, EDGE, 0>(P, z > 0 ? N.c[1] : 0.f, z > 0 ? N.c[2] : 0.f, W, delta,
-                                        inv_delta, S);
+            const float ca = z > 0 ? N.c[1] : 0.f, cb = z > 0 ? N.c[2] : 0.f;
+            if (KIND == UPD_SART_R) {
+                sart_rows<EDGE, W_ZCORNER, W_ZEDGE>(P, ca, cb, W, S);
+#pragma unroll
+                for (int r = 0; r < 4; r++) cp[r] = P.c[r];
+            } else {
+                upd_far_plane<POT, EDGE, 0>(P, ca, cb, W, delta, inv_delta, S);
+            }
             upd_rows<EDGE>(g, x, z + 1, at, ix, iy, P);
             V.taps(h, g.nbx);
             prefetch(z + 3);
-            upd_own_plane<POT, EDGE>(N, W, delta, inv_delta, S);
+            if (KIND == UPD_SART_R)
+                sart_rows<EDGE, W_DIAG, W_FACE>(N, N.c[1], N.c[2], W, S);
+            else
+                upd_own_plane<POT, EDGE>(N, W, delta, inv_delta, S);
         };
-        // Plane z + 1 is in F: finishes plane z's voxels ca, cb.
-        auto end = [&](const UpdRows& F, float ca, float cb, int z) {
+        // Plane z + 1 is in F: finishes plane z's voxels (rows N).
+        auto end = [&](const UpdRows& F, const UpdRows& N, int z) {
             const bool in = z + 1 < g.nz;
-            upd_far_plane<POT, EDGE, 1>(F, in ? ca : 0.f, in ? cb : 0.f, W, delta, inv_delta, S);
-            finish(z, ca, cb);
+            const float ca = in ? N.c[1] : 0.f, cb = in ? N.c[2] : 0.f;
+            if (KIND == UPD_SART_R) {
+                sart_rows<EDGE, W_ZCORNER, W_ZEDGE>(F, ca, cb, W, S);
+                sart_centres<EDGE>(cp, N, F, z > 0, in, W, S);
+            } else {
+                upd_far_plane<POT, EDGE, 1>(F, ca, cb, W, delta, inv_delta, S);
+            }
+            finish(z, N.c[1], N.c[2]);
         };
         UpdRows A, C;
         prefetch(zb + 1);
@@ -623,10 +689,10 @@ __device__ __forceinline__ void update_tile(
         upd_rows<EDGE>(g, x, zb, at, ix, iy, C);
         for (int z = zb;; z += 2) {
             start(A, C, z);
-            end(A, C.c[1], C.c[2], z);
+            end(A, C, z);
             if (z + 1 == ze) break;
             start(C, A, z + 1);
-            end(C, A.c[1], A.c[2], z + 1);
+            end(C, A, z + 1);
             if (z + 2 == ze) break;
         }
     };
@@ -721,7 +787,7 @@ __device__ __forceinline__ void prior_ring(const float* __restrict__ pb,
     *rd = u + w;
 }
 
-template <int POT, int ZC = UZC, int KIND = UPD_OSTR, int NV = 0>
+template <int POT, int ZC = UZC, int NV = 0>
 __device__ __forceinline__ void update_tile_tma(
     const Geo& G, const PriorW5& W, const CUtensorMap* map, float* __restrict__ x_out,
     const float* __restrict__ d, const float* __restrict__ h, const BpTab& T, int a0, int nv,
@@ -782,23 +848,21 @@ __device__ __forceinline__ void update_tile_tma(
         const float* pa = sm.ring[sa];
         if (active) {
             const int v = z * plane + iy * g.nx + ix;
-            const float dv = KIND == UPD_OSTR ? __ldg(d + v) : 0.f;
+            const float dv = __ldg(d + v);
             const float xc = pc[base];
-            float capL = 0.f, sens = 0.f;
+            float capL = 0.f;
             const float* p = h;
             int tix = (a0 * g.nz + z) * g.nx + ix;
             int tiy = (a0 * g.nz + z) * g.ny + iy;
             const int sx = g.nz * g.nx, sy = g.nz * g.ny;
             for (int t = 0; t < (NV ? NV : nv); t++, p += B, tix += sx, tiy += sy)
-                bp_view<KIND>(p, __ldg(T.x + tix), __ldg(T.y + tiy), g, capL, sens);
+                bp_view(p, __ldg(T.x + tix), __ldg(T.y + tiy), g, capL);
             float rdd = 0.f, rd = 0.f;
-            if (KIND != UPD_SART) {
-                if (edge_xy || z == 0 || z == g.nz - 1)
-                    prior_ring<POT, true>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
-                else
-                    prior_ring<POT, false>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
-            }
-            upd_store<KIND>(xc, capL, sens, rd, rdd, dv, M, beta, x_out + v, status);
+            if (edge_xy || z == 0 || z == g.nz - 1)
+                prior_ring<POT, true>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
+            else
+                prior_ring<POT, false>(pb, pc, pa, base, xc, W, delta, inv_delta, &rdd, &rd);
+            upd_store(xc, capL, rd, rdd, dv, M, beta, x_out + v, status);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.empty[sb]);
@@ -842,7 +906,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 6 : 0) update_tma_kernel(
     const float* __restrict__ d, const float* __restrict__ h, const __grid_constant__ BpTab T,
     int a0, int nv, float M, float beta, float delta, int* __restrict__ status) {
     __shared__ UpdSmemT sm;
-    update_tile_tma<POT, ZC, UPD_OSTR, NV>(G, W, &map, x_out, d, h, T, a0, nv, M, beta, delta,
+    update_tile_tma<POT, ZC, NV>(G, W, &map, x_out, d, h, T, a0, nv, M, beta, delta,
                                            status, blockIdx.x, blockIdx.y, blockIdx.z, sm);
 }
 
