@@ -83,7 +83,6 @@ __device__ __forceinline__ float sbp_term(const nr_geom& g, const ViewSrc& v, fl
 
 // vol[v] += sum_{views} SBP term.  prj planes are consecutive per view
 // (view a-a0 at prj + (a-a0)*B).  index == nullptr means identity order.
-template <bool JI>
 __global__ void __launch_bounds__(128) bp_kernel(const __grid_constant__ Geo G,
                                                  float* __restrict__ vol,
                                                  const float* __restrict__ prj,
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(128) bp_kernel(const __grid_constant__ Geo G,
         __syncthreads();
         if (ix < g.nx)
             for (int t = 0; t < cn; t++)
-                total = total + sbp_term<JI>(g, sv[t], x1, y1, z1, prj + (int64_t)(c0 + t) * B);
+                total = total + sbp_term<false>(g, sv[t], x1, y1, z1, prj + (int64_t)(c0 + t) * B);
     }
     if (ix < g.nx) {
         const int64_t v = ((int64_t)iz * g.ny + iy) * g.nx + ix;
@@ -157,16 +156,6 @@ __global__ void __launch_bounds__(128) bp_ossart_kernel(const __grid_constant__ 
     }
 }
 
-nr_status launch_bp(const nr_geom& g, bool ji, float* vol, const float* prj, const float* angles,
-                    const int32_t* index, int a0, int nv, cudaStream_t st) {
-    dim3 blk(128), grd(cdiv(g.nx, 128), g.ny, g.nz);
-    if (ji)
-        bp_kernel<true><<<grd, blk, 0, st>>>(make_geo(g), vol, prj, angles, index, a0, nv);
-    else
-        bp_kernel<false><<<grd, blk, 0, st>>>(make_geo(g), vol, prj, angles, index, a0, nv);
-    return launch_status();
-}
-
 }  // namespace nr
 
 using namespace nr;
@@ -177,7 +166,9 @@ NR_API nr_status nr_bp_sbp(const nr_geom* g, float* vol, const float* prj, const
     if (!vol || !prj || !index || !angles || a0 < 0 || a1 < a0) return NR_ERR_BAD_ARGUMENT;
     if (g->ny > 65535 || g->nz > 65535) return NR_ERR_BAD_GEOMETRY;
     if (a1 == a0) return NR_OK;
-    return launch_bp(*g, false, vol, prj, angles, index, a0, a1 - a0, as_stream(stream));
+    dim3 blk(128), grd(cdiv(g->nx, 128), g->ny, g->nz);
+    bp_kernel<<<grd, blk, 0, as_stream(stream)>>>(make_geo(*g), vol, prj, angles, index, a0, a1 - a0);
+    return launch_status();
 }
 
 NR_API nr_status nr_bp_ossart(const nr_geom* g, float* x, const float* diff, const float* prior,

@@ -172,35 +172,86 @@ __global__ void __launch_bounds__(128, (SZ >= 4 ? 6 : 10)) fp_h_slab_kernel(
 }
 
 // gamma * yry for every view in one pass (the d precompute's detector term,
-// Tomo_OSTR_gold.cpp:183-218), [view][j][i], original view order, identity
-// index.  yry = (y-r)^2/y with the reference's guards.
-template <int MODE>
-__global__ void __launch_bounds__(128) gamma_yry_kernel(const __grid_constant__ Geo G,
+// Tomo_OSTR_gold.cpp:183-218): y (and r) by subset position, out by original
+// view, [view][j][i].  yry = (y-r)^2/y with the reference's guards.
+__device__ __forceinline__ float yry_of(float y, float r) {
+    if (y == 0.f) return 0.f;
+    float dif = y - r;
+    if (dif <= 0.f) dif = y;
+    return __fdiv_rn(dif * dif, y);
+}
+
+__global__ void __launch_bounds__(128) gamma_chord_kernel(const __grid_constant__ Geo G,
                                                         float* __restrict__ out,
-                                                        const float* __restrict__ angles,
+                                                        const ProjView* __restrict__ views,
+                                                        const int32_t* __restrict__ index,
                                                         const float* __restrict__ y,
                                                         const float* __restrict__ r) {
-    __shared__ ViewSrc src;
     const nr_geom& g = G.g;
     const int a = blockIdx.z;
-    if (threadIdx.x == 0 && threadIdx.y == 0) src = view_source(g, angles[a]);
-    __syncthreads();
+    const ViewSrc& src = views[a].src;
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.nbx || j >= g.nby) return;
     float gam = 0.f;  // gamma buffer is zeroed before the projection (Tomo_OSTR_gold.cpp:441)
     float v;
-    if (trace<MODE>(G, nullptr, src.x0, src.y0, src.z0, bin_x(g, i), bin_y(g, j), -g.detectorR, &v))
+    if (trace<1>(G, nullptr, src.x0, src.y0, src.z0, bin_x(g, i), bin_y(g, j), -g.detectorR, &v))
         gam = v;
-    const int64_t o = (int64_t)a * g.nbx * g.nby + bin_off<true>(g, i, j);
-    const float yy = y[o];
-    float c = 0.f;
-    if (yy != 0.f) {
-        float dif = yy - (r ? r[o] : 0.f);
-        if (dif <= 0.f) dif = yy;
-        c = __fdiv_rn(dif * dif, yy);
+    const int64_t B = (int64_t)g.nbx * g.nby, o = bin_off<true>(g, i, j);
+    const int64_t q = (int64_t)a * B + o;
+    out[(int64_t)index[a] * B + o] = yry_of(y[q], r ? r[q] : 0.f) * gam;
+}
+
+// The same for the "length" gamma, whose slab test splits by axis: the x part
+// of ray_axes's interval belongs to the column, the z part to the view and the
+// y part to the row, so a thread that walks GL_ROWS rows of its column has one
+// quotient pair per bin to form instead of three.  The interval's ends are the
+// same minima and maxima, the ray meets the volume or not as there.  125 M
+// bins with scatter: 0.56 ms against 1.78 ms with a block's view computed by
+// one of its threads and three pairs per bin.
+constexpr int GL_ROWS = 8;
+__global__ void __launch_bounds__(128) gamma_length_kernel(const __grid_constant__ Geo G,
+                                                           float* __restrict__ out,
+                                                           const ProjView* __restrict__ views,
+                                                           const int32_t* __restrict__ index,
+                                                           const float* __restrict__ y,
+                                                           const float* __restrict__ r) {
+    const nr_geom& g = G.g;
+    const int a = blockIdx.z;
+    const ViewSrc S = views[a].src;
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    if (i >= g.nbx) return;
+    float lo = -NR_FINF, hi = NR_FINF;
+    auto clip = [](float o, float d, float p0, float p1, float& lo, float& hi) {
+        if (d != 0.f) {
+            const float a0 = __fdiv_rn(p0 - o, d), a1 = __fdiv_rn(p1 - o, d);
+            lo = fmaxf(lo, fminf(a0, a1));
+            hi = fminf(hi, fmaxf(a0, a1));
+        } else if (o >= p1 || o <= p0) {
+            hi = -NR_FINF;
+        }
+    };
+    const float dx = bin_x(g, i) - S.x0, dz = -g.detectorR - S.z0;
+    clip(S.x0, dx, g.x_p0, G.xmax, lo, hi);
+    clip(S.z0, dz, g.z_p0, G.zmax, lo, hi);
+    const int64_t B = (int64_t)g.nbx * g.nby;
+    const float* ya = y + (int64_t)a * B;
+    const float* ra = r ? r + (int64_t)a * B : nullptr;
+    float* oa = out + (int64_t)index[a] * B;
+#pragma unroll 2
+    for (int k = 0; k < GL_ROWS; k++) {
+        const int j = (blockIdx.y * GL_ROWS + k) * 4 + threadIdx.y;
+        if (j >= g.nby) break;
+        const float dy = bin_y(g, j) - S.y0;
+        // the roundings of ray_axes: dx^2, + dy^2, + dz^2 fused
+        const float L =
+            sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
+        float l = lo, h = hi;
+        clip(S.y0, dy, g.y_p0, G.ymax, l, h);
+        const float gam = (L > 0.f && L < NR_FINF && l < h) ? L : 0.f;
+        const int64_t o = bin_off<true>(g, i, j);
+        oa[o] = yry_of(ya[o], ra ? ra[o] : 0.f) * gam;
     }
-    out[o] = c * gam;
 }
 
 }  // namespace nr
@@ -416,20 +467,18 @@ nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* ind
     return launch_status();
 }
 
-nr_status launch_fp_ji(const nr_geom& g, const float* x, float* line, const float* angles,
-                       const int32_t* index, int a0, int nviews, cudaStream_t st) {
-    dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), nviews);
-    fp_kernel<0, true><<<grd, blk, 0, st>>>(make_geo(g), x, line, angles, index, a0);
-    return launch_status();
-}
-
-nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const float* angles,
-                           const float* y, const float* r, cudaStream_t st) {
-    dim3 blk(32, 4), grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), g.n_angles);
-    if (gamma_mode == NR_GAMMA_CHORD)
-        gamma_yry_kernel<1><<<grd, blk, 0, st>>>(make_geo(g), out, angles, y, r);
-    else
-        gamma_yry_kernel<2><<<grd, blk, 0, st>>>(make_geo(g), out, angles, y, r);
+// y, r: by subset position; out: by original view.
+nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const ProjView* views,
+                           const int32_t* index, const float* y, const float* r,
+                           cudaStream_t st) {
+    dim3 blk(32, 4);
+    if (gamma_mode == NR_GAMMA_CHORD) {
+        dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), g.n_angles);
+        gamma_chord_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r);
+    } else {
+        dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4 * GL_ROWS), g.n_angles);
+        gamma_length_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r);
+    }
     return launch_status();
 }
 

@@ -14,7 +14,6 @@
 //   h        float[Vs][BINSy][BINSx]    subset gradient in the detector domain
 //   bpx, bpy float4[A][nz][nx], [A][nz][ny]  back-projection tables (update.cuh)
 //   gc       float[A][BINSy][BINSx]     gamma*yry (setup only)
-//   gr       float[A][BINSy][BINSx]     scatter in original order (setup only; with scatter)
 #include <cuda.h>
 
 #include "update.cuh"
@@ -27,10 +26,10 @@ nr_status launch_fp_h(const nr_geom& g, int k, int stage, const float* x, float*
                       const float* r, int* status,
                       const CUtensorMap* premap, cudaStream_t st);
 bool slab_map(const nr_geom& g, const float* x, CUtensorMap* map);
-nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const float* angles,
-                           const float* y, const float* r, cudaStream_t st);
-nr_status launch_bp(const nr_geom& g, bool ji, float* vol, const float* prj, const float* angles,
-                    const int32_t* index, int a0, int nv, cudaStream_t st);
+nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const ProjView* views,
+                           const int32_t* index, const float* y, const float* r, cudaStream_t st);
+nr_status launch_curvature(const nr_geom& g, float* d, const float* prj, const int32_t* index,
+                           const BpTab& T, cudaStream_t st);
 nr_status launch_update(const nr_geom& g, int pot, int zc, int tile, const float* x, float* x_out,
                         const float* d, const float* h, const BpTab& T, int a0, int nv, float M, float beta, float delta,
                         int* status, const CUtensorMap* map, cudaStream_t st);
@@ -44,8 +43,8 @@ static bool update_map(const nr_geom& g, const nr_ostr_params& p, const float* x
                        CUtensorMap* map) {
     return p.upd_tile == NR_TILE_TMA && volume_map_nan(g, x, UTW, USH, 1, map);
 }
-nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t* index,
-                           float4* tx, float4* ty, bool scaled, cudaStream_t st);
+nr_status launch_bp_tables(const nr_geom& g, const ProjView* views, float4* tx, float4* ty,
+                           bool exact, cudaStream_t st);
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,
                            int Vs, cudaStream_t st);
 nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
@@ -63,7 +62,7 @@ nr_status launch_penalty(const nr_geom& g, int pot, float delta, const float* x,
                          int64_t red_n, double* out, cudaStream_t st);
 
 struct Layout {
-    size_t status, red, index, angles, views, y, b, r, d, xtmp, h, bpx, bpy, gc, gr, total;
+    size_t status, red, index, angles, views, y, b, r, d, xtmp, h, bpx, bpy, gc, total;
     int64_t red_n;
 };
 
@@ -94,8 +93,7 @@ static Layout layout(const nr_geom& g, const nr_ostr_params& p) {
     L.h = take((Vs * B + bp_pad(g)) * sizeof(float));  // + zeros the tap pairs may reach
     L.bpx = take((size_t)A * g.nz * g.nx * sizeof(float4));
     L.bpy = take((size_t)A * g.nz * g.ny * sizeof(float4));
-    L.gc = take(A * B * sizeof(float));
-    L.gr = p.has_scatter ? take(A * B * sizeof(float)) : (size_t)-1;
+    L.gc = take((A * B + bp_pad(g)) * sizeof(float));  // + zeros, as h
     L.total = o;
     return L;
 }
@@ -105,7 +103,7 @@ struct WS {
     double* red;
     int32_t* index;
     ProjView* views;
-    float *angles, *y, *b, *r, *d, *xtmp, *h, *gc, *gr;
+    float *angles, *y, *b, *r, *d, *xtmp, *h, *gc;
     float4 *bpx, *bpy;
     int64_t red_n;
     BpTab tab() const { return BpTab{bpx, bpy}; }
@@ -128,7 +126,6 @@ static WS carve(void* base, const Layout& L) {
     w.bpx = (float4*)(c + L.bpx);
     w.bpy = (float4*)(c + L.bpy);
     w.gc = (float*)(c + L.gc);
-    w.gr = L.gr == (size_t)-1 ? nullptr : (float*)(c + L.gr);
     w.red_n = L.red_n;
     return w;
 }
@@ -245,29 +242,26 @@ NR_API nr_status nr_ostr_setup(const nr_geom* g, const nr_ostr_params* p, const 
     cudaStream_t s = as_stream(stream);
     WS w = carve(workspace, L);
     const int A = g->n_angles, M = p->subset_num, Vs = A / M;
-    const int64_t N = (int64_t)g->nx * g->ny * g->nz;
     clear_status_kernel<<<1, 64, 0, s>>>(w.status);
     index_kernel<<<1, 256, 0, s>>>(w.index, angles, w.angles, A, M);
     if ((st = launch_status()) != NR_OK) return st;
     if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
-    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, true, s)) != NR_OK) return st;
+    if ((st = launch_bp_tables(*g, w.views, w.bpx, w.bpy, true, s)) != NR_OK) return st;
     // [view][i][j] original order -> [view][j][i] subset order.
     if ((st = launch_transpose(w.y, prj, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
     if ((st = launch_transpose(w.b, blank, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
     if (w.r && (st = launch_transpose(w.r, scat, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;
-    // gamma*yry is formed in original view order (identity index, as the
-    // reference does before it regroups): stage y (and r) there.
-    if ((st = launch_transpose(w.gc, prj, g->nbx, g->nby, A, 0, 1, s)) != NR_OK) return st;
-    if (w.r && (st = launch_transpose(w.gr, scat, g->nbx, g->nby, A, 0, 1, s)) != NR_OK) return st;
-    // gc <- yry(gc, r) * gamma, original order, identity index.
-    if ((st = launch_gamma_yry(*g, p->gamma_mode, w.gc, angles, w.gc, w.gr, s)) != NR_OK)
+    // gc <- yry(y, r) * gamma, back in original view order
+    if ((st = launch_gamma_yry(*g, p->gamma_mode, w.gc, w.views, w.index, w.y, w.r, s)) != NR_OK)
         return st;
+    if (cudaMemsetAsync(w.gc + (int64_t)A * g->nbx * g->nby, 0, bp_pad(*g) * sizeof(float), s) !=
+        cudaSuccess)
+        return NR_ERR_CUDA;
     if (cudaMemsetAsync(w.h + (int64_t)Vs * g->nbx * g->nby, 0, bp_pad(*g) * sizeof(float), s) !=
         cudaSuccess)
         return NR_ERR_CUDA;
-    if (cudaMemsetAsync(w.d, 0, N * sizeof(float), s) != cudaSuccess) return NR_ERR_CUDA;
-    // d = SBP(gamma*yry) over all views, original order (Tomo_OSTR_gold.cpp:528-565).
-    if ((st = launch_bp(*g, true, w.d, w.gc, angles, nullptr, 0, A, s)) != NR_OK) return st;
+    // d = SBP(gamma*yry) over all views (Tomo_OSTR_gold.cpp:528-565)
+    if ((st = launch_curvature(*g, w.d, w.gc, w.index, w.tab(), s)) != NR_OK) return st;
     return NR_OK;
 }
 

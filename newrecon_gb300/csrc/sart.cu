@@ -45,8 +45,8 @@ nr_status launch_transpose(float* out, const float* in, int rows, int cols, int 
                            int Vs, cudaStream_t st);
 nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
                        ProjView* views, cudaStream_t st);
-nr_status launch_bp_tables(const nr_geom& g, const float* angles, const int32_t* index,
-                           float4* tx, float4* ty, bool scaled, cudaStream_t st);
+nr_status launch_bp_tables(const nr_geom& g, const ProjView* views, float4* tx, float4* ty,
+                           bool exact, cudaStream_t st);
 
 namespace {
 
@@ -373,7 +373,7 @@ NR_API nr_status nr_sart_setup(const nr_geom* g, const nr_sart_params* p, const 
     if ((st = launch_clear_status(w.status, s)) != NR_OK) return st;
     if ((st = launch_subset_index(w.index, angles, w.angles, A, M, s)) != NR_OK) return st;
     if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
-    if ((st = launch_bp_tables(*g, w.angles, w.index, w.bpx, w.bpy, false, s)) != NR_OK) return st;
+    if ((st = launch_bp_tables(*g, w.views, w.bpx, w.bpy, false, s)) != NR_OK) return st;
     if (cudaMemsetAsync(w.diff + (int64_t)Vs * g->nbx * g->nby, 0, bp_pad(*g) * sizeof(float),
                         s) != cudaSuccess)
         return NR_ERR_CUDA;

@@ -196,8 +196,7 @@ constexpr int UPD_SART_R = 2;   // OS-SART with the hyperbola prior, backprj_OSS
 // and the row (jlb, fracJ) only on its y (the ray from the source through
 // the voxel centre meets the detector plane at x0 + (x1 - x0) t(z), y0 +
 // (y1 - y0) t(z)).  Neither depends on the volume, so they are tabulated once
-// per reconstruction, per view (subset order), plane and column / row, with
-// the arithmetic of bp.cu's sbp_term in reciprocal-multiply form, as a tap
+// per reconstruction, per view (subset order), plane and column / row, as a tap
 // pair and its weights:
 //   x[(a nz + z) nx + i] = {c, w0, w1, k (x0 - x1)^2}
 //   y[(a nz + z) ny + j] = {r * BINSx, v0, v1, k ((y0 - y1)^2 + (z0 - z1)^2)}
@@ -254,39 +253,31 @@ __device__ __forceinline__ void bp_pair(int lb, float w0, float w1, int n, int& 
     }
 }
 
-__device__ __forceinline__ float4 bp_entry_x(const nr_geom& g, const ViewSrc& vs, float tt,
-                                             int i, float inv_bx, float k) {
-    const float x1 = vox_x(g, i);
-    const float ddx = vs.x0 - x1;
-    const float x2 = vs.x0 + (x1 - vs.x0) * tt;
-    const float imb = (x2 - g.x_d0) * inv_bx;
-    int ilb = (int)floorf(imb);
-    if (imb < (float)ilb + 0.5f) ilb -= 1;
-    const float fracI = imb - ((float)ilb + 0.5f);
-    const bool i0 = (ilb < g.nbx) && (ilb >= 0);
-    const bool i1 = (ilb < g.nbx - 1) && (ilb >= -1);
+// Taps (lb, lb + 1) on a line of n bins from lb and the fraction f, 0 <= f <= 1,
+// past bin lb's centre: the pair and its weights.
+__device__ __forceinline__ float4 bp_taps(int lb, float f, int n, bool valid) {
+    const bool t0 = valid && (lb < n) && (lb >= 0);
+    const bool t1 = valid && (lb < n - 1) && (lb >= -1);
     int c;
     float p0, p1;
-    bp_pair(ilb, i0 ? 1.f - fracI : 0.f, i1 ? fracI : 0.f, g.nbx, c, p0, p1);
-    return make_float4(__int_as_float(c), p0, p1, k * (ddx * ddx));
+    bp_pair(lb, t0 ? 1.f - f : 0.f, t1 ? f : 0.f, n, c, p0, p1);
+    return make_float4(__int_as_float(c), p0, p1, 0.f);
 }
 
-__device__ __forceinline__ float4 bp_entry_y(const nr_geom& g, const ViewSrc& vs, float z1,
-                                             float tt, int j, float inv_by, float k) {
-    const bool valid = z1 != vs.z0;
-    const float y1 = vox_y(g, j);
-    const float ddy = vs.y0 - y1, ddz = vs.z0 - z1;
-    const float y2 = vs.y0 + (y1 - vs.y0) * tt;
-    const float jmb = (y2 - g.y_d0) * inv_by;
-    int jlb = (int)floorf(jmb);
-    if (jmb < (float)jlb + 0.5f) jlb -= 1;
-    const float fracJ = jmb - ((float)jlb + 0.5f);
-    const bool j0 = valid && (jlb < g.nby) && (jlb >= 0);
-    const bool j1 = valid && (jlb < g.nby - 1) && (jlb >= -1);
-    int r;
-    float p0, p1;
-    bp_pair(jlb, j0 ? 1.f - fracJ : 0.f, j1 ? fracJ : 0.f, g.nby, r, p0, p1);
-    return make_float4(__int_as_float(r * g.nbx), p0, p1, k * (ddy * ddy + ddz * ddz));
+// The same from a detector position in bins.
+__device__ __forceinline__ float4 bp_taps_at(float mb, int n, bool valid) {
+    int lb = (int)floorf(mb);
+    if (mb < (float)lb + 0.5f) lb -= 1;
+    return bp_taps(lb, mb - ((float)lb + 0.5f), n, valid);
+}
+
+// EXACT: positions in double, the fraction rounded once (a float position of
+// some thousand bins is 1e-4 bin off); otherwise the float arithmetic that the
+// OS-SART update keeps.
+__device__ __forceinline__ float4 bp_taps_at(double mb, int n, bool valid) {
+    const double f = floor(mb - 0.5);
+    const int lb = (int)f;
+    return bp_taps(lb, (float)(mb - 0.5 - f), n, valid);
 }
 
 // One view's back-projection term of one voxel, added to capL, from its table
@@ -554,7 +545,7 @@ __device__ __forceinline__ void update_tile(
     const int jb = has_b ? 1 : 0;       // B's offsets, kept in bounds
     const float inv_delta = 1.f / delta;
     const int64_t B = (int64_t)g.nbx * g.nby;
-    UpdSums S;
+    UpdSums S = {0, 0, 0, 0};
     UpdView V;
     float dva = 0.f, dvb = 0.f;
     // d and the first view's table entries of plane z's voxels
@@ -620,7 +611,6 @@ __device__ __forceinline__ void update_tile(
         x_out[v] = xa < 0.f ? 0.f : xa;
         if (has_b) x_out[v + g.nx] = xb < 0.f ? 0.f : xb;
     };
-    S.sdda = S.sda = S.sddb = S.sdb = pk2(0.f, 0.f);
     if (KIND == UPD_SART) {
         fetch(zb);
         for (int z = zb; z < ze; z++) {

@@ -60,11 +60,16 @@ struct WalkView {
 struct ProjView {
     ViewSrc src;
     WalkView w;
+    double x0, z0;   // the source, not rounded (the back-projection tables)
 };
 
 __device__ __forceinline__ void proj_view(const Geo& G, float theta, ProjView& V) {
     const nr_geom& g = G.g;
     V.src = view_source(g, theta);
+    double sn, cs;
+    sincos((double)theta, &sn, &cs);
+    V.x0 = (double)g.sourceR * sn;
+    V.z0 = (double)g.sourceR * cs;
     const double x0 = V.src.x0, y0 = V.src.y0, z0 = V.src.z0;
     const double dz = -(double)g.detectorR - z0, rz = 1.0 / dz;
     const double at = ((double)G.zmax - z0) * rz;   // of the way at the top plane
