@@ -194,13 +194,16 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 
 // K chunk kc of the strip of row `row` (-1: zeros) from x0 - 1, 130 rows of 16
 // bytes: the part inside [0, nx) from the activations, the rest zeros.
+// inner: only the rows inside [0, nx) (the others hold zeros already).
 __device__ __forceinline__ void load_chunk(uint8_t* dst, const __nv_bfloat16* in, int nx, int x0,
-                                           int64_t row, int kc, uint64_t* bar) {
-    if (row < 0) {
-        bulk_load(dst, g_zero_rows, SROWS * 16, bar);
+                                           int64_t row, int kc, bool inner, uint64_t* bar) {
+    const int lo = x0 == 0 ? 1 : 0, hi = min(x0 + SROWS - 1, nx) - x0 + 1;  // strip rows [lo, hi)
+    if (row < 0 || inner) {
+        const void* src = row < 0 ? (const void*)g_zero_rows
+                                  : in + ((row * KCH + kc) * nx + x0 - 1 + lo) * 8;
+        bulk_load(dst + (inner ? lo * 16 : 0), src, (uint32_t)(inner ? hi - lo : SROWS) * 16, bar);
         return;
     }
-    const int lo = x0 == 0 ? 1 : 0, hi = min(x0 + SROWS - 1, nx) - x0 + 1;  // strip rows [lo, hi)
     if (lo) bulk_load(dst, g_zero_rows, 16, bar);
     bulk_load(dst + lo * 16, in + ((row * KCH + kc) * nx + x0 - 1 + lo) * 8, (uint32_t)(hi - lo) * 16,
               bar);
@@ -275,6 +278,13 @@ __global__ void __launch_bounds__(Y_THREADS, 1) conv32_ys_kernel(
     for (int k = tid; k < Y_WBYTES / 16; k += Y_THREADS)
         ((uint4*)sW)[k] = __ldg((const uint4*)wpk + k);
     if (EPI == EPI_RELU && tid < C) K->bias[tid] = bias[tid];
+    // a row of one tile: the strips' rows outside it are zeros once and for all,
+    // one copy per chunk instead of three (bulk copies of 16 bytes cost as much
+    // as a row's): 34 us per launch instead of 40 at 126 x 32 x 16 x 8
+    const bool one = d.nx <= TM;
+    if (one)
+        for (int k = tid; k < Y_R * Y_SET / 16; k += Y_THREADS)
+            ((uint4*)ring)[k] = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
         for (int s = 0; s < Y_R; s++) {
             tc::mbar_init(&K->full[s], 1);
@@ -318,13 +328,14 @@ __global__ void __launch_bounds__(Y_THREADS, 1) conv32_ys_kernel(
                     stop = true;
                     break;
                 }
-                if (lane == 0) mbar_arrive_tx(&K->full[s], 4 * KCH * SROWS * 16);
+                if (lane == 0)
+                    mbar_arrive_tx(&K->full[s], 4 * KCH * 16 * (uint32_t)(one ? d.nx : SROWS));
                 __syncwarp();
                 const int Y = y0 - 1 + j;
                 const bool ok = zz >= 0 && zz < d.nz && Y >= 0 && Y < d.ny;
                 if (lane < 4 * KCH)
                     load_chunk(ring + s * Y_SET + sp * TSTRIP + kc * PLANE, in, d.nx, x0,
-                               ok ? ((int64_t)b * d.nz + zz) * d.ny + Y : -1, kc, &K->full[s]);
+                               ok ? ((int64_t)b * d.nz + zz) * d.ny + Y : -1, kc, one, &K->full[s]);
             }
         }
         // no copy may be in flight when the block exits (T row-sets were issued)
@@ -568,36 +579,37 @@ __global__ void __launch_bounds__(LR_THREADS) last_rows_kernel(
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {
-            // MMA issuer: per dx, the strip at offset dx rows against its 16 x 32 block
-            constexpr uint32_t idesc = tc::idesc_bf16(TM, 16);
-            const uint64_t ad0 = tc::sdesc(tc::smem_u32(ring), PLANE, 128);
-            const uint64_t bd0 = tc::sdesc(tc::smem_u32(sW), 128, 512);
-            int64_t lt = 0;
-            for (int64_t t = blockIdx.x; t < nt && !*abort; t += gridDim.x, lt++) {
-                const int a = (int)(lt & 1), s = (int)(lt % LR_STAGE);
-                if (lt >= 2 && !wait_live(&K->acce[a], (uint32_t)(((lt >> 1) - 1) & 1), abort)) {
-                    fail();
-                    break;
-                }
-                if (!wait_live(&K->full[s], (uint32_t)((lt / LR_STAGE) & 1), abort)) {
-                    fail();
-                    break;
-                }
-                tc::fence_after();
-                const uint64_t adr = ad0 + (uint64_t)((s * TSTRIP) >> 4);
-#pragma unroll
-                for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                    for (int j = 0; j < 2; j++)
-                        tc::mma_bf16(tmem + (uint32_t)(a * 32),
-                                     adr + (uint64_t)((dx * 16 + j * 2 * PLANE) >> 4),
-                                     bd0 + (uint64_t)((dx * 16 * C * 2 + j * 256) >> 4), idesc,
-                                     (dx | j) ? 1u : 0u);
-                tc::commit(&K->empty[s]);
-                tc::commit(&K->accf[a]);
+        // MMA issuer (the warp, one elected lane: issued by one lane of a diverged
+        // warp an MMA takes 96 to 140 clocks): per dx, the strip at offset dx
+        // rows against its 16 x 32 block
+        constexpr uint32_t idesc = tc::idesc_bf16(TM, 16);
+        const uint64_t ad0 = tc::sdesc(tc::smem_u32(ring), PLANE, 128);
+        const uint64_t bd0 = tc::sdesc(tc::smem_u32(sW), 128, 512);
+        int64_t lt = 0;
+        for (int64_t t = blockIdx.x; t < nt; t += gridDim.x, lt++) {
+            const int a = (int)(lt & 1), s = (int)(lt % LR_STAGE);
+            const bool go =
+                (lt < 2 || wait_live(&K->acce[a], (uint32_t)(((lt >> 1) - 1) & 1), abort)) &&
+                wait_live(&K->full[s], (uint32_t)((lt / LR_STAGE) & 1), abort);
+            if (!__all_sync(0xffffffffu, go)) {
+                if (lane == 0) fail();
+                break;
             }
+            tc::fence_after();
+            const uint32_t alo = (uint32_t)ad0 + (uint32_t)((s * TSTRIP) >> 4);
+#pragma unroll
+            for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    tc::mma_bf16_warp(tmem + (uint32_t)(a * 32),
+                                      alo + (uint32_t)((dx * 16 + j * 2 * PLANE) >> 4),
+                                      (uint32_t)(ad0 >> 32),
+                                      (uint32_t)bd0 + (uint32_t)((dx * 16 * C * 2 + j * 256) >> 4),
+                                      (uint32_t)(bd0 >> 32), idesc, (dx | j) ? 1u : 0u);
+            tc::commit_warp(&K->empty[s]);
+            tc::commit_warp(&K->accf[a]);
         }
+        __syncwarp();
     } else {
         // epilogue warps 0-3: row 32 warp + lane of each tile.  Test hook: the
         // workspace's second status word k + 1 > 0 makes the wait for this
@@ -629,7 +641,7 @@ __global__ void __launch_bounds__(LR_THREADS) last_rows_kernel(
         }
     }
     __syncthreads();
-    if (warp == 5 && lane == 0) tc::commit(&K->drain);
+    if (warp == 5) tc::commit_warp(&K->drain);
     if (!tc::mbar_wait(&K->drain, 0, WAIT_LIMIT)) tc::mbar_wait(&K->drain, 0, WAIT_LIMIT);
     tc::fence_before();
     __syncthreads();
@@ -638,10 +650,15 @@ __global__ void __launch_bounds__(LR_THREADS) last_rows_kernel(
 
 // Pass 2: grid (row of the stacked volume, block of 256 x VEC); VEC = 4 when
 // rows are 16-byte aligned (nx % 4 == 0): four x per thread in float4 loads.
-template <int VEC>
+// RESID: the network's output max(0, x_in + f / s) instead of f.  Bound by DRAM
+// (36 bytes of q, 8 of x and the output per voxel): 213 us at 1024 x 512 x 60,
+// where the sum alone took 195 us and a residual pass over f another 55 us.
+template <int VEC, bool RESID>
 __global__ void __launch_bounds__(256) last_sum_kernel(Dims d, const float* __restrict__ q,
                                                        const float* __restrict__ bias,
-                                                       float* __restrict__ f) {
+                                                       const float* __restrict__ x_in,
+                                                       float inv_s, float* __restrict__ f) {
+    auto out = [&](float v, float xi) { return RESID ? fmaxf(xi + v * inv_s, 0.f) : v; };
     const int64_t row = blockIdx.x;
     const int x = (blockIdx.y * 256 + threadIdx.x) * VEC;
     if (x >= d.nx) return;
@@ -663,8 +680,11 @@ __global__ void __launch_bounds__(256) last_sum_kernel(Dims d, const float* __re
             }
         }
         const float b0 = bias[0];
+        const float4 xi = RESID ? __ldg((const float4*)(x_in + row * d.nx + x))
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
         *(float4*)(f + row * d.nx + x) =
-            make_float4(sum.x + b0, sum.y + b0, sum.z + b0, sum.w + b0);
+            make_float4(out(sum.x + b0, xi.x), out(sum.y + b0, xi.y), out(sum.z + b0, xi.z),
+                        out(sum.w + b0, xi.w));
     } else {
         float sum = 0.f;
 #pragma unroll
@@ -673,7 +693,7 @@ __global__ void __launch_bounds__(256) last_sum_kernel(Dims d, const float* __re
             if (zz >= 0 && zz < d.nz && yy >= 0 && yy < d.ny)
                 sum += __ldg(q + n * V + ((b * d.nz + zz) * d.ny + yy) * d.nx + x);
         }
-        f[row * d.nx + x] = sum + bias[0];
+        f[row * d.nx + x] = out(sum + bias[0], RESID ? __ldg(x_in + row * d.nx + x) : 0.f);
     }
 }
 
@@ -986,49 +1006,50 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgrad_tc_kernel(
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer.  Test hook: the workspace's second status word k + 1
-            // > 0 makes the wait for this CTA's K block k report giving up
-            // once it has in fact succeeded.
-            const int force_at = status[1] - 1;
-            int64_t kb = 0;
-            for (int64_t t = blockIdx.x; t < nt && !*abort; t += gridDim.x, kb++) {
-                const int sg = (int)(kb & 1);
-                const uint32_t par = (uint32_t)((kb >> 1) & 1);
-                bool got = wait_live(&K->tfull[sg], par, abort);
-                if (got) got = wait_live(&K->bfull[sg], par, abort);
-                if (kb == force_at) got = false;
-                if (!got) {
-                    fail();
-                    break;
-                }
-                tc::fence_after();
-                const uint32_t sb = tc::smem_u32(smem + sg * Cfg::STAGE);
-                if (MODE == WG_FIRST) {
+        // MMA issuer (the warp, one elected lane).  Test hook: the workspace's
+        // second status word k + 1 > 0 makes the wait for this CTA's K block k
+        // report giving up once it has in fact succeeded.
+        const int force_at = status[1] - 1;
+        auto mma = [&](uint32_t dacc, uint64_t ad, uint64_t bd, uint32_t acc) {
+            tc::mma_bf16_warp(dacc, (uint32_t)ad, (uint32_t)(ad >> 32), (uint32_t)bd,
+                              (uint32_t)(bd >> 32), Cfg::IDESC, acc);
+        };
+        int64_t kb = 0;
+        for (int64_t t = blockIdx.x; t < nt; t += gridDim.x, kb++) {
+            const int sg = (int)(kb & 1);
+            const uint32_t par = (uint32_t)((kb >> 1) & 1);
+            bool got = !*abort && wait_live(&K->tfull[sg], par, abort);
+            if (got) got = wait_live(&K->bfull[sg], par, abort);
+            if (kb == force_at) got = false;
+            if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) fail();
+                break;
+            }
+            tc::fence_after();
+            const uint32_t sb = tc::smem_u32(smem + sg * Cfg::STAGE);
+            if (MODE == WG_FIRST) {
+#pragma unroll
+                for (int k = 0; k < TM / 16; k++)
+                    mma(tmem, tc::sdesc(sb + Cfg::OFF_X + k * 256, 128, WG_GROUP),
+                        tc::sdesc(sb + Cfg::OFF_G + 16 + k * 256, 128, WG_PLANE),
+                        (kb > 0 || k > 0) ? 1u : 0u);
+            } else {
+                for (int gi = 0; gi < 3; gi++) {
+                    const int g0 = gi == 0 ? 0 : (gi == 1 ? 4 : 5);
+                    // the three dx accumulators in turn
 #pragma unroll
                     for (int k = 0; k < TM / 16; k++)
-                        tc::mma_bf16(tmem, tc::sdesc(sb + Cfg::OFF_X + k * 256, 128, WG_GROUP),
-                                     tc::sdesc(sb + Cfg::OFF_G + 16 + k * 256, 128, WG_PLANE),
-                                     Cfg::IDESC, (kb > 0 || k > 0) ? 1u : 0u);
-                } else {
-                    for (int gi = 0; gi < 3; gi++) {
-                        const int g0 = gi == 0 ? 0 : (gi == 1 ? 4 : 5);
 #pragma unroll
-                        for (int dx = 0; dx < 3; dx++) {
-                            const uint32_t dacc = tmem + (uint32_t)((gi * 3 + dx) * 32);
-#pragma unroll
-                            for (int k = 0; k < TM / 16; k++)
-                                tc::mma_bf16(
-                                    dacc,
-                                    tc::sdesc(sb + g0 * WG_STRIP + dx * 16 + k * 256, 128, WG_PLANE),
-                                    tc::sdesc(sb + Cfg::OFF_X + k * 256, 128, WG_GROUP),
-                                    Cfg::IDESC, (kb > 0 || k > 0) ? 1u : 0u);
-                        }
-                    }
+                        for (int dx = 0; dx < 3; dx++)
+                            mma(tmem + (uint32_t)((gi * 3 + dx) * 32),
+                                tc::sdesc(sb + g0 * WG_STRIP + dx * 16 + k * 256, 128, WG_PLANE),
+                                tc::sdesc(sb + Cfg::OFF_X + k * 256, 128, WG_GROUP),
+                                (kb > 0 || k > 0) ? 1u : 0u);
                 }
-                tc::commit(&K->empty[sg]);
             }
+            tc::commit_warp(&K->empty[sg]);
         }
+        __syncwarp();
     } else {
         // warps 2-5: the built operand and the bias sum
         const int h = warp - 2;
@@ -1094,7 +1115,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgrad_tc_kernel(
     }
     // drain: every MMA issued has completed before TMEM is read or released
     __syncthreads();
-    if (warp == 1 && lane == 0) tc::commit(&K->drain);
+    if (warp == 1) tc::commit_warp(&K->drain);
     if (!tc::mbar_wait(&K->drain, 0, WAIT_LIMIT)) tc::mbar_wait(&K->drain, 0, WAIT_LIMIT);
     tc::fence_after();
     const bool ok = *abort == 0;
@@ -1264,57 +1285,58 @@ __global__ void __launch_bounds__(GW_THREADS, 1) wgrad_walk_kernel(
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer.  Test hook: the workspace's second status word k + 1
-            // > 0 makes the wait for this CTA's K block k report giving up
-            // once it has in fact succeeded.
-            const int force_at = status[1] - 1;
-            constexpr uint32_t idesc = tc::idesc_bf16(TM, 96) | (1u << 15) | (1u << 16);
-            const uint64_t ad0 = tc::sdesc(tc::smem_u32(gst), 128, WG_PLANE);
-            const uint64_t bd0 = tc::sdesc(tc::smem_u32(ring), 128, WG_PLANE);
-            int64_t G = 0, kb = 0;
-            bool stop = false;
-            for (int64_t it = blockIdx.x; it < wp.nitems && !stop && !*abort; it += gridDim.x) {
-                int b, z, x0, y0, ly;
-                item_pos(d, wp, it, b, z, x0, y0, ly);
-                for (int i = 0; i < ly; i++, kb++) {
-                    const int gs = (int)(kb & 1);
-                    bool got = wait_live(&K->gbuilt[gs], (uint32_t)((kb >> 1) & 1), abort);
-                    int slot[3];
-                    for (int dy = 0; dy < 3 && got; dy++) {
-                        const int64_t g2 = G + i + dy;
-                        slot[dy] = (int)(g2 % GW_R);
-                        if (i == 0 || dy == 2)
-                            got = wait_live(&K->rfull[slot[dy]], (uint32_t)((g2 / GW_R) & 1), abort);
-                    }
-                    if (kb == force_at) got = false;
-                    if (!got) {
-                        fail();
-                        stop = true;
-                        break;
-                    }
-                    tc::fence_after();
-                    const uint64_t adg = ad0 + (uint64_t)((gs * GW_G) >> 4);
+        // MMA issuer (the warp, one elected lane).  Test hook: the workspace's
+        // second status word k + 1 > 0 makes the wait for this CTA's K block k
+        // report giving up once it has in fact succeeded.
+        const int force_at = status[1] - 1;
+        constexpr uint32_t idesc = tc::idesc_bf16(TM, 96) | (1u << 15) | (1u << 16);
+        const uint64_t ad0 = tc::sdesc(tc::smem_u32(gst), 128, WG_PLANE);
+        const uint64_t bd0 = tc::sdesc(tc::smem_u32(ring), 128, WG_PLANE);
+        int64_t G = 0, kb = 0;
+        bool stop = false;
+        for (int64_t it = blockIdx.x; it < wp.nitems && !stop; it += gridDim.x) {
+            int b, z, x0, y0, ly;
+            item_pos(d, wp, it, b, z, x0, y0, ly);
+            for (int i = 0; i < ly; i++, kb++) {
+                const int gs = (int)(kb & 1);
+                bool got = !*abort && wait_live(&K->gbuilt[gs], (uint32_t)((kb >> 1) & 1), abort);
+                int slot[3];
 #pragma unroll
-                    for (int ks = 0; ks < TM / 16; ks++)
-#pragma unroll
-                        for (int dy = 0; dy < 3; dy++)
-                            tc::mma_bf16(tmem + (uint32_t)(dy * 96),
-                                         adg + (uint64_t)((ks * 256) >> 4),
-                                         bd0 + (uint64_t)((slot[dy] * W_SET + 16 + ks * 256) >> 4),
-                                         idesc, (kb > 0 || ks > 0) ? 1u : 0u);
-                    tc::commit(&K->gempty[gs]);
-                    // row-set i is not read after this K block; the last one of
-                    // the item also frees row-sets ly and ly + 1
-                    tc::commit(&K->rempty[slot[0]]);
-                    if (i == ly - 1) {
-                        tc::commit(&K->rempty[slot[1]]);
-                        tc::commit(&K->rempty[slot[2]]);
-                    }
+                for (int dy = 0; dy < 3; dy++) {
+                    const int64_t g2 = G + i + dy;
+                    slot[dy] = (int)(g2 % GW_R);
+                    if (got && (i == 0 || dy == 2))
+                        got = wait_live(&K->rfull[slot[dy]], (uint32_t)((g2 / GW_R) & 1), abort);
                 }
-                G += ly + 2;
+                if (kb == force_at) got = false;
+                if (!__all_sync(0xffffffffu, got)) {
+                    if (lane == 0) fail();
+                    stop = true;
+                    break;
+                }
+                tc::fence_after();
+                const uint32_t alo = (uint32_t)ad0 + (uint32_t)((gs * GW_G) >> 4);
+#pragma unroll
+                for (int ks = 0; ks < TM / 16; ks++)
+#pragma unroll
+                    for (int dy = 0; dy < 3; dy++)
+                        tc::mma_bf16_warp(
+                            tmem + (uint32_t)(dy * 96), alo + (uint32_t)((ks * 256) >> 4),
+                            (uint32_t)(ad0 >> 32),
+                            (uint32_t)bd0 + (uint32_t)((slot[dy] * W_SET + 16 + ks * 256) >> 4),
+                            (uint32_t)(bd0 >> 32), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+                tc::commit_warp(&K->gempty[gs]);
+                // row-set i is not read after this K block; the last one of
+                // the item also frees row-sets ly and ly + 1
+                tc::commit_warp(&K->rempty[slot[0]]);
+                if (i == ly - 1) {
+                    tc::commit_warp(&K->rempty[slot[1]]);
+                    tc::commit_warp(&K->rempty[slot[2]]);
+                }
             }
+            G += ly + 2;
         }
+        __syncwarp();
     } else {
         // warps 2-5: the shifted gradient copies and the bias sum
         const int h = warp - 2;
@@ -1357,7 +1379,7 @@ __global__ void __launch_bounds__(GW_THREADS, 1) wgrad_walk_kernel(
     }
     // drain: every MMA issued has completed before TMEM is read or released
     __syncthreads();
-    if (warp == 1 && lane == 0) tc::commit(&K->drain);
+    if (warp == 1) tc::commit_warp(&K->drain);
     if (!tc::mbar_wait(&K->drain, 0, WAIT_LIMIT)) tc::mbar_wait(&K->drain, 0, WAIT_LIMIT);
     tc::fence_after();
     const bool ok = *abort == 0;
@@ -1516,14 +1538,6 @@ __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float*
         v[k] = vk;
         p[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
     }
-}
-
-// x_warm = x + f / s (and a non-negativity clamp, the OSTR constraint).
-__global__ void residual_out_kernel(const float* __restrict__ x, const float* __restrict__ f,
-                                    float inv_s, int64_t V, float* __restrict__ out) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
-         v += (int64_t)gridDim.x * blockDim.x)
-        out[v] = fmaxf(x[v] + f[v] * inv_s, 0.f);
 }
 
 }  // namespace cnn
@@ -1685,9 +1699,11 @@ static nr_status launch_conv1(const Dims& d, const float* in, float scale,
     return launch_status();
 }
 
-// The 32 -> 1 layer (two passes); q: 9 V floats of scratch.
+// The 32 -> 1 layer (two passes); q: 9 V floats of scratch.  f: the layer's
+// output, or with x_in the network's, max(0, x_in + inv_s f).
 static nr_status launch_last(const Dims& d, const __nv_bfloat16* in, const __nv_bfloat16* wpk,
-                             const float* bias, float* q, float* f, int* status, cudaStream_t s) {
+                             const float* bias, float* q, const float* x_in, float inv_s, float* f,
+                             int* status, cudaStream_t s) {
     ActMaps map;
     if (!act_maps(d, in, &map)) return NR_ERR_CUDA;
     const size_t smem = (size_t)LR_STAGE * TSTRIP + 3 * 16 * C * 2 + sizeof(LastCtl);
@@ -1698,14 +1714,18 @@ static nr_status launch_last(const Dims& d, const __nv_bfloat16* in, const __nv_
     const int grid = (int)(nt < (int64_t)sm_count() * 4 ? nt : (int64_t)sm_count() * 4);
     last_rows_kernel<<<grid, LR_THREADS, smem, s>>>(d, map.lo, map.hi, wpk, q, status);
     // q planes start at multiples of V floats: with nx % 4 == 0 every row is 16-byte
-    // aligned (the workspace is 256-byte aligned)
-    if (d.nx % 4 == 0) {
-        const dim3 g2((unsigned)((int64_t)d.nb * d.nz * d.ny), (unsigned)((d.nx / 4 + 255) / 256));
-        last_sum_kernel<4><<<g2, 256, 0, s>>>(d, q, bias, f);
-    } else {
-        const dim3 g2((unsigned)((int64_t)d.nb * d.nz * d.ny), (unsigned)((d.nx + 255) / 256));
-        last_sum_kernel<1><<<g2, 256, 0, s>>>(d, q, bias, f);
-    }
+    // aligned (the workspace is 256-byte aligned; x_in and f are the caller's)
+    const bool vec = d.nx % 4 == 0 && (((uintptr_t)x_in | (uintptr_t)f) & 15) == 0;
+    const dim3 g2((unsigned)((int64_t)d.nb * d.nz * d.ny),
+                  (unsigned)(((vec ? d.nx / 4 : d.nx) + 255) / 256));
+    if (vec && x_in)
+        last_sum_kernel<4, true><<<g2, 256, 0, s>>>(d, q, bias, x_in, inv_s, f);
+    else if (vec)
+        last_sum_kernel<4, false><<<g2, 256, 0, s>>>(d, q, bias, nullptr, 0.f, f);
+    else if (x_in)
+        last_sum_kernel<1, true><<<g2, 256, 0, s>>>(d, q, bias, x_in, inv_s, f);
+    else
+        last_sum_kernel<1, false><<<g2, 256, 0, s>>>(d, q, bias, nullptr, 0.f, f);
     return launch_status();
 }
 
@@ -1714,9 +1734,10 @@ static void pack(const float* w, int mode, int ni, int no, int nout, __nv_bfloat
     pack_kernel<<<64, 256, 0, s>>>(w, mode, ni, no, nout, out);
 }
 
-// Forward through layer 6: f = conv6(a5) in `f`; activations in `acts`
-// (5 buffers when `keep`, else 2 ping-pong buffers).
-static nr_status forward(const Dims& d, const float* params, const float* x, float s,
+// Forward through layer 6: f = conv6(a5) in the workspace's `f`, or with out
+// given the network's output there; activations in `acts` (5 buffers when
+// `keep`, else 2 ping-pong buffers).
+static nr_status forward(const Dims& d, const float* params, const float* x, float s, float* out,
                          char* ws, const WSL& L, bool keep, cudaStream_t st) {
     int64_t wo[6], bo[6], P;
     param_offsets(wo, bo, &P);
@@ -1738,7 +1759,8 @@ static nr_status forward(const Dims& d, const float* params, const float* x, flo
     // q of the last layer: a buffer idle by now (the gradient buffer when the
     // activations are kept for training, else layer 4's ping-pong buffer)
     float* q = (float*)(ws + (keep ? L.dpre[0] : L.act[1]));
-    return launch_last(d, act(4), pkf(5), params + bo[5], q, (float*)(ws + L.f), status, st);
+    return launch_last(d, act(4), pkf(5), params + bo[5], q, out ? x : nullptr, 1.f / s,
+                       out ? out : (float*)(ws + L.f), status, st);
 }
 
 __global__ void target_kernel(const float* __restrict__ x, const float* __restrict__ t, float s,
@@ -1814,7 +1836,7 @@ static nr_status loss_grad(const Dims& d, const float* params, const float* x, c
     param_offsets(wo, bo, &P);
     int* status = (int*)(ws + L.status);
     nr_status e;
-    if ((e = forward(d, params, x, s, ws, L, true, st)) != NR_OK) return e;
+    if ((e = forward(d, params, x, s, nullptr, ws, L, true, st)) != NR_OK) return e;
     float* r = (float*)(ws + L.r);
     float* g6 = (float*)(ws + L.g6);
     target_kernel<<<1024, 256, 0, st>>>(x, target, s, V, r);
@@ -1876,11 +1898,7 @@ NR_API nr_status nr_cnn_forward(const nr_cnn_dims* d, const float* params, const
     const WSL L = layout(D, false);
     if (!ws || ws_bytes < L.total || ((uintptr_t)ws & 255)) return NR_ERR_WORKSPACE;
     cudaStream_t st = as_stream(stream);
-    nr_status e = forward(D, params, x, in_scale, (char*)ws, L, false, st);
-    if (e != NR_OK) return e;
-    residual_out_kernel<<<1024, 256, 0, st>>>(x, (const float*)((char*)ws + L.f), 1.f / in_scale,
-                                              nvox(D), x_out);
-    return launch_status();
+    return forward(D, params, x, in_scale, x_out, (char*)ws, L, false, st);
 }
 
 NR_API nr_status nr_cnn_loss_grad(const nr_cnn_dims* d, const float* params, const float* x,
