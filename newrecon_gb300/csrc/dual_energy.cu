@@ -7,7 +7,7 @@
 // lines.  MATLAB reads the float32 files as double, so d is
 //     float(double(he) - double(le) * w)        (two roundings in double)
 // which the kernel reproduces bit for bit: in FP32 by error-free transforms
-// where a bound on what they drop decides the rounding (de_fast), and with
+// where a bound on what they drop decides the rounding (de_fast2), and with
 // separate double multiply and subtract (no contraction to an FMA) where it
 // cannot -- GB300's FP64 pipe runs at about 1/64 of the FP32 rate.  The K
 // outputs of one voxel are written from one read of he and le.
@@ -22,11 +22,12 @@
 namespace nr {
 
 constexpr int DE_MAX_WEIGHTS = 16;
+constexpr int DE_BLOCKS = 4;  // per SM, all resident
 
 struct DeWeights {
     double w[DE_MAX_WEIGHTS];
     float w1[DE_MAX_WEIGHTS], w2[DE_MAX_WEIGHTS];  // w = w1 + w2 + (|.| <= 2^-47 |w|)
-    unsigned fast;     // bit k: weight k takes the FP32 path (de_fast)
+    unsigned fast;     // bit k: weight k takes the FP32 path (de_fast2)
     unsigned pow2;     // bit k: weight k is a power of two (a w exact in float)
     int k;
     int masked;        // 1: he and le multiplied by (he > level) first
@@ -44,8 +45,7 @@ __device__ __forceinline__ double de_value(double h, double l, double w) {
     return __dadd_rn(h, -__dmul_rn(l, w));
 }
 
-// float(double(b) - double(a) * w) without the FP64 pipe, or NaN when the
-// FP32 evaluation cannot decide it (the caller then takes the FP64 path).
+// The FP32 evaluation of double(b) - double(a) * w, without the FP64 pipe.
 //
 // a w1 = p1 + e1 exactly (FMA), a w2 rounds once; two error-free sums give
 // b - a w ~ hi + lo with hi = RN(hi + lo).  The terms dropped on the way (a
@@ -53,11 +53,7 @@ __device__ __forceinline__ double de_value(double h, double l, double w) {
 // small terms, under 2^-48 (2 |s| + 3 |p1|), s = RN(b - p1)) and both
 // roundings of the double evaluation (under 2^-53 (|b| + 2 |p1|)) add up to
 // less than 2^-45.2 |p1| + 2^-46.9 |b|; B = 2^-44 |p1| + 2^-46 |b| bounds
-// them with a factor of 1.8 to spare.  If hi + m and hi - m, m = |lo| + B,
-// both round back to hi, the double evaluation lies strictly inside hi's
-// rounding interval and rounds to hi too.  Otherwise -- about 2^-20 |p1| /
-// |hi| of the outputs (cancellation), and tiny, huge or non-finite products
-// -- the answer is left to FP64.
+// them with a factor of 1.8 to spare.
 // b - a w ~ hi + lo as above, with B bounding |the double value - (hi + lo)|;
 // false for tiny, huge or non-finite products.
 __device__ __forceinline__ bool de_sum(float b, float a, float w1, float w2, float& hi, float& lo,
@@ -80,13 +76,38 @@ __device__ __forceinline__ bool de_sum(float b, float a, float w1, float w2, flo
     return true;
 }
 
-__device__ __forceinline__ float de_fast(float b, float a, float w1, float w2) {
-    float hi, lo, B;
-    if (de_sum(b, a, w1, w2, hi, lo, B)) {
-        const float m = __fadd_rn(fabsf(lo), B);
-        if (__fadd_rn(hi, m) == hi && __fsub_rn(hi, m) == hi) return hi;
-    }
-    return __int_as_float(0x7fc00000);
+// float(double(b) - double(a) * w) for a weight of the fast class, and a bit
+// for each of the two the FP32 evaluation did not decide.  As de_sum with a w2 + e1 in one FMA:
+// b - a w = s + t + (dropped terms), and the double evaluation lies within B of
+// s + t, B = 2^-43 |p1| + 2^-45 |b|.  The dropped terms and the double's own
+// roundings are below 2^-45.2 |p1| + 2^-46.9 |b| as above (one rounding less),
+// and rounding t + B and t - B, |t| <= 2^-24 (|b| + 3 |p1|), adds at most
+// 2^-46.3 |p1| + 2^-47.9 |b|: a factor of 2 to spare.  Rounding is monotone: where
+// s + (t + B) and s + (t - B) round to one float, so does the double value.
+// Overflow gives an infinity less an infinity on the way, a NaN, which decides
+// nothing.  |p1| >= min_p: 2^-100, where every error term is a normal number or
+// exact; 0 for a voxel with a = 0 and b not -0, whose terms are all exact and
+// whose zeros come out positive as in double.
+//
+// Two voxels at a time in packed pairs and without a branch: 16 instructions per
+// output of 22 in scalar form (the kernel is bound by instruction issue).
+__device__ __forceinline__ uint32_t de_fast2(f32x2 b, float bb0, float bb1, float a0, float a1,
+                                             float min0, float min1, float w1, float w2, float& r0,
+                                             float& r1) {
+    const f32x2 neg = pk2(-1.f, -1.f), a = pk2(a0, a1);
+    const float p0 = __fmul_rn(a0, -w1), p1 = __fmul_rn(a1, -w1);  // -p1 of each
+    const f32x2 np = pk2(p0, p1);
+    const f32x2 t1 = fma2(a, pk2(w2, w2), fma2(a, pk2(w1, w1), np));
+    const f32x2 s = add2(b, np);  // TwoSum(b, -p1)
+    const f32x2 bp = fma2(b, neg, s);
+    const f32x2 ap = fma2(bp, neg, s);
+    const f32x2 serr = add2(fma2(ap, neg, b), fma2(bp, neg, np));
+    const f32x2 t = fma2(t1, neg, serr);
+    const f32x2 B = pk2(__fmaf_rn(fabsf(p0), 0x1p-43f, bb0), __fmaf_rn(fabsf(p1), 0x1p-43f, bb1));
+    float d0, d1;
+    upk2(add2(s, add2(t, B)), r0, r1);
+    upk2(add2(s, fma2(B, neg, t)), d0, d1);
+    return (r0 == d0 && fabsf(p0) >= min0 ? 0u : 1u) | (r1 == d1 && fabsf(p1) >= min1 ? 0u : 2u);
 }
 
 // im8_bin of a double value v known as |v - (hi + lo)| <= B: round(255 v)
@@ -109,78 +130,129 @@ __device__ __noinline__ float de_slow(float b, float a, double w) {
     return __double2float_rn(de_value(b, a, w));
 }
 
-template <int K>
-__device__ __forceinline__ float de_out(float b, float a, const DeWeights& W) {
-    if ((W.pow2 >> K) & 1u) {
-        // a w exact: double(b) - a w needs more than 53 bits only when one
-        // operand is below 2^-29 of the other, and then both roundings land
-        // on the float of b - a w (the nearest float midpoint is 2^-25 away)
-        const float p = __fmul_rn(a, W.w1[K]);
-        const float ap = fabsf(p);
-        if (a == 0.f || (ap >= 0x1p-100f && ap <= 0x1p100f)) return __fsub_rn(b, p);
-    } else if ((W.fast >> K) & 1u) {
-        const float r = de_fast(b, a, W.w1[K], W.w2[K]);
-        if (r == r) return r;
-        // a = 0 is exact in float: b - 0 w1, with IEEE's signed zeros as in double
-        if (a == 0.f) return __fsub_rn(b, __fmul_rn(a, W.w1[K]));
-    }
-    return de_slow(b, a, W.w[K]);
+// A weight that is a power of two: a w is exact, and double(b) - a w needs more
+// than 53 bits only when one operand is below 2^-29 of the other, where both
+// roundings land on the float of b - a w (the nearest float midpoint is 2^-25
+// away).
+__device__ __forceinline__ bool de_pow2(float b, float a, float w1, float& r) {
+    const float p = __fmul_rn(a, w1);
+    r = __fsub_rn(b, p);
+    return a == 0.f || (fabsf(p) >= 0x1p-100f && fabsf(p) <= 0x1p100f);
 }
 
-// Weights K, K + 1, ... of four voxels (16-byte store per weight) or of one.
-template <int K>
-__device__ __forceinline__ void de_row(const float (&h)[4], const float (&l)[4],
-                                       const DeWeights& W, float* __restrict__ d, int64_t n,
-                                       int64_t q) {
-    if constexpr (K < DE_MAX_WEIGHTS) {
-        if (K >= W.k) return;
-        float4 o;
-        o.x = de_out<K>(h[0], l[0], W);
-        o.y = de_out<K>(h[1], l[1], W);
-        o.z = de_out<K>(h[2], l[2], W);
-        o.w = de_out<K>(h[3], l[3], W);
-        __stcs(reinterpret_cast<float4*>(d + (int64_t)K * n) + q, o);
-        de_row<K + 1>(h, l, W, d, n, q);
-    }
-}
+// d[k][i] = float(he[i] - le[i] * w_k), 128 voxels per warp and step.  VEC (n a
+// multiple of 4, so that every output row d + k n stays 16-byte aligned): a
+// lane's voxels are adjacent, with 16-byte loads and stores; otherwise they lie
+// 32 apart.
+//
+// What FP32 leaves open is not rare where the weights are tenths: for one a in
+// ten the exact product lies within 2^-53 of a float, and 2 to 3 % of the
+// outputs are ties that the double product's own rounding decides.  One such
+// lane holds its warp for the FP64 instructions' full time (evaluated in place,
+// the FP64 pipe was 66 % busy and bound the kernel), so a warp writes its open
+// outputs' numbers to a list and evaluates the list with all lanes.
+//
+// Bound by instruction issue (231 M warp instructions, 66 % issue): 295 us for
+// nine weights of 1024 x 512 x 60 (its 1.38 GB take 204 us), from 790 us with
+// FP64 in place; 350 us with scalar FP32.
+constexpr int DE_TILE = 128;
 
-template <int K>
-__device__ __forceinline__ void de_one(float h, float l, const DeWeights& W,
-                                       float* __restrict__ d, int64_t n, int64_t i) {
-    if constexpr (K < DE_MAX_WEIGHTS) {
-        if (K >= W.k) return;
-        d[(int64_t)K * n + i] = de_out<K>(h, l, W);
-        de_one<K + 1>(h, l, W, d, n, i);
-    }
-}
-
-// d[k][i] = float(he[i] - le[i] * w_k).  VEC (n a multiple of 4, so that every
-// output row d + k n stays 16-byte aligned): four voxels per thread per step
-// with 16-byte loads and stores; otherwise one voxel per step.
 template <bool VEC>
-__global__ void __launch_bounds__(256) de_subtract_kernel(const float* __restrict__ he,
-                                                          const float* __restrict__ le,
-                                                          float* __restrict__ d, int64_t n,
-                                                          const __grid_constant__ DeWeights W) {
-    const int64_t n4 = VEC ? n / 4 : 0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n4; q += stride) {
-        const float4 h4 = __ldg(reinterpret_cast<const float4*>(he) + q);
-        const float4 l4 = __ldg(reinterpret_cast<const float4*>(le) + q);
-        float h[4] = {h4.x, h4.y, h4.z, h4.w};
-        float l[4] = {l4.x, l4.y, l4.z, l4.w};
-        if (W.masked)
+__global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
+    const float* he, const float* le, float* d, int64_t n,
+    const __grid_constant__ DeWeights W) {
+    __shared__ uint16_t list[8][DE_TILE * DE_MAX_WEIGHTS];
+    __shared__ double sw[DE_MAX_WEIGHTS];
+    if (threadIdx.x < DE_MAX_WEIGHTS) sw[threadIdx.x] = W.w[threadIdx.x];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint16_t* open = list[warp];
+    const int64_t step = (int64_t)gridDim.x * 8 * DE_TILE;
+    for (int64_t i0 = (blockIdx.x * 8 + warp) * (int64_t)DE_TILE; i0 < n; i0 += step) {
+        const int64_t i = i0 + (VEC ? 4 * lane : lane);
+        float h[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f}, hb[4], lm[4];
+        if (VEC) {
+            if (i < n) {
+                const float4 h4 = __ldg(reinterpret_cast<const float4*>(he + i));
+                const float4 l4 = __ldg(reinterpret_cast<const float4*>(le + i));
+                h[0] = h4.x; h[1] = h4.y; h[2] = h4.z; h[3] = h4.w;
+                l[0] = l4.x; l[1] = l4.y; l[2] = l4.z; l[3] = l4.w;
+            }
+        } else {
+#pragma unroll
             for (int t = 0; t < 4; t++)
-                if (!(h[t] > W.level_f)) h[t] = l[t] = 0.f;
-        // unrolled over the weights: each weight's constants are fixed
-        // constant-bank operands
-        de_row<0>(h, l, W, d, n, q);
-    }
-    // everything when !VEC
-    for (int64_t i = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-        float h = he[i], l = le[i];
-        if (W.masked && !(h > W.level_f)) h = l = 0.f;
-        de_one<0>(h, l, W, d, n, i);
+                if (i + 32 * t < n) {
+                    h[t] = __ldg(he + i + 32 * t);
+                    l[t] = __ldg(le + i + 32 * t);
+                }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            if (W.masked && !(h[t] > W.level_f)) h[t] = l[t] = 0.f;
+            hb[t] = __fmul_rn(fabsf(h[t]), 0x1p-45f);
+            lm[t] = l[t] == 0.f && __float_as_uint(h[t]) != 0x80000000u ? 0.f : 0x1p-100f;
+        }
+        uint64_t bad = 0;  // bit 4 k + t: weight k of voxel t is left to FP64
+        float* row = d + i;
+#pragma unroll 1
+        for (int k = 0; k < W.k; k++, row += n) {
+            float o[4];
+            uint32_t m = 0;
+            if ((W.pow2 >> k) & 1u) {
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    m |= de_pow2(h[t], l[t], W.w1[k], o[t]) ? 0u : 1u << t;
+            } else if ((W.fast >> k) & 1u) {
+                const float w1 = W.w1[k], w2 = W.w2[k];
+#pragma unroll
+                for (int t = 0; t < 4; t += 2)
+                    m |= de_fast2(pk2(h[t], h[t + 1]), hb[t], hb[t + 1], l[t], l[t + 1], lm[t],
+                                  lm[t + 1], w1, w2, o[t], o[t + 1]) << t;
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; t++) o[t] = de_slow(h[t], l[t], W.w[k]);
+            }
+            bad |= (uint64_t)m << (4 * k);
+            if (VEC) {
+                if (i < n)
+                    __stcs(reinterpret_cast<float4*>(row), make_float4(o[0], o[1], o[2], o[3]));
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    if (i + 32 * t < n) __stcs(row + 32 * t, o[t]);
+            }
+        }
+        if (!__any_sync(0xffffffffu, bad != 0)) continue;
+        const int cnt = __popcll(bad);
+        int end = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += up;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        int pos = end - cnt;
+        for (; bad; bad &= bad - 1) open[pos++] = (uint16_t)(((__ffsll(bad) - 1) << 5) | lane);
+        __syncwarp();  // the list, and the stores above before those below
+        // he and le from their lanes' registers: d may lie over them
+        for (int j0 = 0; j0 < total; j0 += 32) {
+            const bool on = j0 + lane < total;
+            const int e = on ? open[j0 + lane] : 0, t = (e >> 5) & 3, k = e >> 7, from = e & 31;
+            float b = 0.f, a = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float bu = __shfl_sync(0xffffffffu, h[u], from);
+                const float au = __shfl_sync(0xffffffffu, l[u], from);
+                if (t == u) {
+                    b = bu;
+                    a = au;
+                }
+            }
+            if (on)
+                d[(int64_t)k * n + i0 + (VEC ? 4 * from + t : from + 32 * t)] =
+                    __double2float_rn(de_value(b, a, sw[k]));
+        }
+        __syncwarp();
     }
 }
 
@@ -274,10 +346,12 @@ NR_API nr_status nr_de_subtract(const float* he, const float* le, const double* 
     if ((double)lf > mask_level) lf = std::nextafterf(lf, -INFINITY);
     W.level_f = lf;
     cudaStream_t s = as_stream(stream);
+    const int64_t steps = (n + 8 * DE_TILE - 1) / (8 * DE_TILE);
+    const unsigned blocks = (unsigned)(steps > 152 * DE_BLOCKS ? 152 * DE_BLOCKS : steps);
     if (n > 0 && n % 4 == 0)
-        de_subtract_kernel<true><<<de_blocks(n / 4), 256, 0, s>>>(he, le, d, n, W);
+        de_subtract_kernel<true><<<blocks, 256, 0, s>>>(he, le, d, n, W);
     else if (n > 0)
-        de_subtract_kernel<false><<<de_blocks(n), 256, 0, s>>>(he, le, d, n, W);
+        de_subtract_kernel<false><<<blocks, 256, 0, s>>>(he, le, d, n, W);
     if (hist) {
         if (cudaMemsetAsync(hist, 0, (size_t)n_weights * 256 * sizeof(int32_t), s) != cudaSuccess)
             return NR_ERR_CUDA;

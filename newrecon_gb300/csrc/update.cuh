@@ -78,42 +78,6 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
     return r;
 }
 
-// Packed FP32 pairs (add / sub / mul / fma on .f32x2): two neighbour terms per
-// instruction, each lane rounded as the scalar operation would be.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk2(f32x2 r, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
-}
-// A duplicated pair stored as float2, read as one 64-bit value.
-__device__ __forceinline__ f32x2 ld2(const float2& v) {
-    return *reinterpret_cast<const f32x2*>(&v);
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // omega(t) of two differences of one potential, divided by delta for Huber
 // (min(1, delta/|t|) = delta / max(|t|, delta): the class factor carries the
 // delta).  EDGE: a difference with an out-of-volume cell (NaN) counts as t = 0.
