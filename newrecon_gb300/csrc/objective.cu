@@ -47,24 +47,29 @@ __global__ void __launch_bounds__(128) data_term_kernel(
     block_partial(term, red, blk);
 }
 
-// psi(t) in double (Lange, hyperbola): t is the exact difference of two
-// floats (a double holds it), and the weights are the double values
-// 1/sqrt(...), so the only roundings left are the double operations' own.
-template <int POT>
-__device__ __forceinline__ double psi(double t, double delta) {
-    if (POT == NR_POT_Q2) return 0.5 * t * t;
-    if (POT == NR_POT_LANGE) {
-        const double a = fabs(t) / delta;
-        return delta * delta * (a - log1p(a));
-    }
-    if (POT == NR_POT_HYPERBOLA) {
-        // d^2 (sqrt(1+u^2) - 1) = d^2 u^2 / (sqrt(1+u^2) + 1): no cancellation
-        const double u = t / delta;
-        const double u2 = u * u;
-        return delta * delta * (u2 / (sqrt(1.0 + u2) + 1.0));
-    }
-    const double a = fabs(t);
-    return a <= delta ? 0.5 * t * t : delta * a - 0.5 * delta * delta;
+// Lange's psi(t) in double: t is the exact difference of two floats (a double
+// holds it), and the weights are the double values 1/sqrt(...), so the only
+// roundings left are the double operations' own (inv = 1 / delta).
+__device__ __forceinline__ double psi_lange(double t, double delta, double inv) {
+    const double a = fabs(t) * inv;
+    return delta * delta * (a - log1p(a));
+}
+
+// The hyperbola's psi(t) = d^2 (sqrt(1 + u^2) - 1), u = t / d, as the fraction
+// t^2 / (sqrt(1 + u^2) + 1): no cancellation.
+struct Frac {
+    double n, d;
+};
+__device__ __forceinline__ Frac psi_hyperbola(double t, double inv) {
+    const double u = t * inv;
+    return {t * t, sqrt(fma(u, u, 1.0)) + 1.0};
+}
+// w1 a + w2 b with one division: the kernel is bound by the FP64 pipe and a
+// division is a dozen of its instructions (512 x 256 x 60: 5.75 ms with two
+// divisions per pair of neighbours and one by delta, 4.27 with these; Lange without
+// the division by delta 6.75 -> 5.42).  The denominators are at least 2.
+__device__ __forceinline__ double add_fracs(double w1, Frac a, double w2, Frac b) {
+    return fma(w1 * a.n, b.d, w2 * b.n * a.d) / (a.d * b.d);
 }
 
 struct PairW {
@@ -144,6 +149,9 @@ __global__ void __launch_bounds__(128) penalty_kernel(const __grid_constant__ Ge
         const float xc = x[v];
         int k = 0;
         FF sum = {0.f, 0.f};  // Q2 / Huber: float-float sum of the voxel's terms
+        const double inv = 1.0 / (double)delta;
+        Frac held = {0.0, 1.0};  // hyperbola: the term that waits for its partner
+        double held_w = 0.0;
         auto pair = [&](int dx, int dy, int dz) {
             const int kx = ix + dx, ky = iy + dy, kz = iz + dz;
             if ((unsigned)kx < (unsigned)g.nx && (unsigned)ky < (unsigned)g.ny &&
@@ -160,8 +168,21 @@ __global__ void __launch_bounds__(128) penalty_kernel(const __grid_constant__ Ge
                     sum = {s2.hi, __fadd_rn(sum.lo, __fadd_rn(s2.lo, lo))};
                 } else {
                     const double t = (double)xc - (double)xn;
-                    acc += W.w[k] * psi<POT>(t, (double)delta);
+                    if (POT == NR_POT_LANGE) {
+                        acc += W.w[k] * psi_lange(t, (double)delta, inv);
+                    } else if (k % 2 == 0) {
+                        held = psi_hyperbola(t, inv);
+                        held_w = W.w[k];
+                    } else {
+                        acc += add_fracs(held_w, held, W.w[k], psi_hyperbola(t, inv));
+                        held_w = 0.0;
+                    }
                 }
+            }
+            if (POT == NR_POT_HYPERBOLA && (k % 2 == 1 || k == 12)) {
+                // the partner lies outside the volume, or there is none
+                if (held_w != 0.0) acc += held_w * held.n / held.d;
+                held_w = 0.0;
             }
             k++;
         };
