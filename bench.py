@@ -300,12 +300,10 @@ def run_ours(args):
     ach = kern[dom]["gbs"]
     traffic = None
     prof_traffic = os.path.join(HERE, "profiles", "dram_traffic.txt")
-    # the ncu figure of the variant that ran (the two-voxel update tile has its own)
-    tkey = dom + ("_x2" if dom == "ostr_update" and plan.params.upd_tile == 1 and Vs == 1 else "")
     if os.path.isfile(prof_traffic) and args.config == "clinical":
         for ln in open(prof_traffic):
             parts = ln.split()
-            if len(parts) >= 2 and not ln.startswith("#") and parts[0] == tkey:
+            if len(parts) >= 2 and not ln.startswith("#") and parts[0] == dom:
                 traffic = float(parts[1])
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
