@@ -546,7 +546,8 @@ nr_status nr_sart_workspace_section(const nr_geom* g, const nr_sart_params* p,
  * NULL it gets hist[k][b] = the number of i in [hist_begin, hist_begin +
  * hist_len) whose double d_k falls in 8-bit bin b = round(255 d) saturated to
  * [0, 255] (the histogram MATLAB's entropy(d(:,:,slice)) counts, :34).
- * he, le and d 16-byte aligned; d holds n_weights * n floats. */
+ * he, le and d 16-byte aligned; d holds n_weights * n floats, and a row of d
+ * may be he or le itself (the histogram is of the values they had). */
 nr_status nr_de_subtract(const float* he, const float* le, const double* weights,
                          int32_t n_weights, int64_t n, double mask_level, float* d,
                          int64_t hist_begin, int64_t hist_len, int32_t* hist, void* stream);

@@ -346,12 +346,7 @@ NR_API nr_status nr_de_subtract(const float* he, const float* le, const double* 
     if ((double)lf > mask_level) lf = std::nextafterf(lf, -INFINITY);
     W.level_f = lf;
     cudaStream_t s = as_stream(stream);
-    const int64_t steps = (n + 8 * DE_TILE - 1) / (8 * DE_TILE);
-    const unsigned blocks = (unsigned)(steps > 152 * DE_BLOCKS ? 152 * DE_BLOCKS : steps);
-    if (n > 0 && n % 4 == 0)
-        de_subtract_kernel<true><<<blocks, 256, 0, s>>>(he, le, d, n, W);
-    else if (n > 0)
-        de_subtract_kernel<false><<<blocks, 256, 0, s>>>(he, le, d, n, W);
+    // first, while he and le are as given: d may lie over them
     if (hist) {
         if (cudaMemsetAsync(hist, 0, (size_t)n_weights * 256 * sizeof(int32_t), s) != cudaSuccess)
             return NR_ERR_CUDA;
@@ -359,6 +354,12 @@ NR_API nr_status nr_de_subtract(const float* he, const float* le, const double* 
             de_hist_kernel<<<de_blocks(hist_len), 256, 0, s>>>(he, le, hist_begin, hist_len,
                                                                hist, W);
     }
+    const int64_t steps = (n + 8 * DE_TILE - 1) / (8 * DE_TILE);
+    const unsigned blocks = (unsigned)(steps > 152 * DE_BLOCKS ? 152 * DE_BLOCKS : steps);
+    if (n > 0 && n % 4 == 0)
+        de_subtract_kernel<true><<<blocks, 256, 0, s>>>(he, le, d, n, W);
+    else if (n > 0)
+        de_subtract_kernel<false><<<blocks, 256, 0, s>>>(he, le, d, n, W);
     return launch_status();
 }
 
