@@ -173,8 +173,10 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
         float h[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f}, hb[4], lm[4];
         if (VEC) {
             if (i < n) {
-                const float4 h4 = __ldg(reinterpret_cast<const float4*>(he + i));
-                const float4 l4 = __ldg(reinterpret_cast<const float4*>(le + i));
+                // plain loads: d may lie over he or le, which rules out the
+                // read-only path
+                const float4 h4 = *reinterpret_cast<const float4*>(he + i);
+                const float4 l4 = *reinterpret_cast<const float4*>(le + i);
                 h[0] = h4.x; h[1] = h4.y; h[2] = h4.z; h[3] = h4.w;
                 l[0] = l4.x; l[1] = l4.y; l[2] = l4.z; l[3] = l4.w;
             }
@@ -182,8 +184,8 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
 #pragma unroll
             for (int t = 0; t < 4; t++)
                 if (i + 32 * t < n) {
-                    h[t] = __ldg(he + i + 32 * t);
-                    l[t] = __ldg(le + i + 32 * t);
+                    h[t] = he[i + 32 * t];
+                    l[t] = le[i + 32 * t];
                 }
         }
 #pragma unroll
