@@ -81,26 +81,29 @@ __device__ __forceinline__ int find_case(const int* off, int n, int it) {
     return c;
 }
 
-// Projection items [0, hi) of step `step` (hi: the active prefix).  12 resident
-// blocks per SM: at fp_h_kernel's 16 the runtime case index spills (four mixed
-// cases: 6.86 against 6.47 ms).
-__global__ void __launch_bounds__(128, 12) fp_batch_kernel(const __grid_constant__ BatchTable P,
-                                                           int step, int hi) {
+// Projection items of step `step`, a block each (the grid is the active prefix).
+// 12 resident blocks per SM: at fp_h_kernel's 16 the runtime case index spills
+// (four mixed cases: 6.86 against 6.47 ms).  LONG as fp_h_kernel's, when an active
+// case's rows take several lists (one iteration of 256 x 128 x 300 and 128 x 64 x
+// 400, nine views each: 1.59 ms at 8 blocks, 1.79 at 10, 2.25 with the lists past
+// the first out of line; 1.65 with the walk of siddon.cuh for such rows).
+template <bool LONG>
+__global__ void __launch_bounds__(128, LONG ? 8 : 12) fp_batch_kernel(
+    const __grid_constant__ BatchTable P, int step) {
     __shared__ float2 rows[4][WALK_ROWS];
-    for (int it = blockIdx.x; it < hi; it += gridDim.x) {
-        const int p = find_case(P.fp_off, P.n, it);
-        const CaseDev& cd = P.c[P.fp_case[p]];
-        __syncthreads();  // previous item's readers of src are done
-        if (step >= cd.total_sub) continue;
-        const int local = it - P.fp_off[p];
-        const int bx = local % cd.fp_tx;
-        const int by = (local / cd.fp_tx) % cd.fp_ty;
-        const int bz = local / (cd.fp_tx * cd.fp_ty);
-        const int a0 = (step % (int)cd.M) * cd.Vs;
-        const float* cur = (step & 1) ? cd.xtmp : cd.x;
-        const Geo G = cd.G;  // copied once per item, as in update_batch_kernel
-        fp_h_tile(G, cur, cd.h, cd.views, a0, cd.y, cd.b, cd.r, bx, by, bz, rows);
-    }
+    const int it = blockIdx.x;
+    const int p = find_case(P.fp_off, P.n, it);
+    const CaseDev& cd = P.c[P.fp_case[p]];
+    if (step >= cd.total_sub) return;
+    const int local = it - P.fp_off[p];
+    const int bx = local % cd.fp_tx;
+    const int by = (local / cd.fp_tx) % cd.fp_ty;
+    const int bz = local / (cd.fp_tx * cd.fp_ty);
+    const int a0 = (step % (int)cd.M) * cd.Vs;
+    const float* cur = (step & 1) ? cd.xtmp : cd.x;
+    const Geo G = cd.G;  // copied once per item, as in update_batch_kernel
+    fp_h_tile<4, false, LONG>(G, cur, cd.h, cd.views, a0, cd.y, cd.b, cd.r, bx, by, bz, rows,
+                              cd.G);
 }
 
 // Update items [lo, hi) of one (potential, NV, ZC) class.  NV = 1 serves the
@@ -325,7 +328,12 @@ nr_status enqueue_steps(const BatchTable& P, int32_t first, int32_t count, cudaS
         int np = 0;
         while (np < P.n && P.c[P.fp_case[np]].total_sub > k) np++;
         if (np == 0) continue;  // every case is done
-        fp_batch_kernel<<<P.fp_off[np], dim3(32, 4), 0, s>>>(P, k, P.fp_off[np]);
+        bool far = false;
+        for (int c = 0; c < np; c++) far = far || walk_long(P.c[P.fp_case[c]].G.g);
+        if (far)
+            fp_batch_kernel<true><<<P.fp_off[np], dim3(32, 4), 0, s>>>(P, k);
+        else
+            fp_batch_kernel<false><<<P.fp_off[np], dim3(32, 4), 0, s>>>(P, k);
         for (int cls = 0; cls < N_CLASSES; cls++) {
             int e = P.cls_first[cls];
             while (e < P.cls_end[cls] && P.c[e].total_sub > k) e++;

@@ -119,8 +119,17 @@ __global__ void __launch_bounds__(256) fp_4r_kernel(const __grid_constant__ Geo 
 // view computed by one of its threads (107 M, 59 %: a fifth of the warps' time
 // at that barrier), 0.122 with the views from the workspace (100 M, 69 %) and
 // 0.117 at FP_BLOCKS = 16.
-template <int K>
-__global__ void __launch_bounds__(128, (K >= 8 ? 8 : FP_BLOCKS)) fp_h_kernel(const __grid_constant__ Geo G,
+//
+// LONG (rows of more cells than a list): the walk over several lists takes more
+// registers than 16 blocks leave.  256 x 128 x 300, three views, K = 4: 55 us
+// at 10 blocks, 77 with the lists past the first out of line in the
+// 16-block form, 73 with the walk of siddon.cuh at 12 blocks (100 at 16);
+// 512 x 256 x 400: 239, 376, 270.  At 10 blocks rows of one list take the same time on these
+// volumes and 4 % more on the clinical workload, so the form goes by the rows.
+constexpr int long_blocks(int k) { return k >= 8 ? 8 : (k >= 4 ? 10 : 12); }
+
+template <int K, bool LONG>
+__global__ void __launch_bounds__(128, LONG || K >= 8 ? long_blocks(K) : FP_BLOCKS) fp_h_kernel(const __grid_constant__ Geo G,
                                                    const float* __restrict__ vol,
                                                    float* __restrict__ h,
                                                    const ProjView* __restrict__ views, int a0,
@@ -128,7 +137,18 @@ __global__ void __launch_bounds__(128, (K >= 8 ? 8 : FP_BLOCKS)) fp_h_kernel(con
                                                    const float* __restrict__ b,
                                                    const float* __restrict__ r) {
     __shared__ float2 rows[4][WALK_ROWS];
-    fp_h_tile<K>(G, vol, h, views, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z, rows);
+    fp_h_tile<K, false, LONG>(G, vol, h, views, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z,
+                              rows, G);
+}
+
+template <int K>
+static void launch_fp_h_k(const Geo& G, dim3 grd, dim3 blk, const float* x, float* h,
+                          const ProjView* views, int a0, const float* y, const float* b,
+                          const float* r, cudaStream_t st) {
+    if (walk_long(G.g))
+        fp_h_kernel<K, true><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
+    else
+        fp_h_kernel<K, false><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
 }
 
 // fp_h_kernel with the subset's FP64 data term: one partial per block in red
@@ -144,7 +164,7 @@ __global__ void __launch_bounds__(128) fp_h_data_kernel(const __grid_constant__ 
                                                         double* __restrict__ red) {
     __shared__ float2 rows[4][WALK_ROWS];
     fp_h_tile<K, true>(G, vol, h, views, a0, y, b, r, blockIdx.x, blockIdx.y, blockIdx.z, rows,
-                       red);
+                       G, red);
 }
 
 __global__ void __launch_bounds__(1024) partials_sum_kernel(const double* __restrict__ red,
@@ -427,11 +447,11 @@ nr_status launch_fp_h(const nr_geom& g, int k, int stage, const float* x, float*
         return launch_status();
     }
     if (k == 2)
-        fp_h_kernel<2><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
+        launch_fp_h_k<2>(G, grd, blk, x, h, views, a0, y, b, r, st);
     else if (k == 8)
-        fp_h_kernel<8><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
+        launch_fp_h_k<8>(G, grd, blk, x, h, views, a0, y, b, r, st);
     else
-        fp_h_kernel<4><<<grd, blk, 0, st>>>(G, x, h, views, a0, y, b, r);
+        launch_fp_h_k<4>(G, grd, blk, x, h, views, a0, y, b, r, st);
     return launch_status();
 }
 

@@ -21,7 +21,7 @@
 
 namespace nr {
 
-__global__ void __launch_bounds__(128) data_term_kernel(
+__global__ void __launch_bounds__(128, 10) data_term_kernel(
     const __grid_constant__ Geo G, const float* __restrict__ x,
     const ProjView* __restrict__ views, const float* __restrict__ y, const float* __restrict__ b,
     const float* __restrict__ r, double* __restrict__ red) {
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(128) data_term_kernel(
     double term = 0.0;
     float v, l = 0.f;
     const bool on = i < g.nbx && j < g.nby;
-    if (line_integral<4>(G, x, view, bin_x(g, i), bin_y(g, j), on, rows[threadIdx.y], &v))
+    if (line_integral<4>(G, G, x, view, bin_x(g, i), bin_y(g, j), on, rows[threadIdx.y], &v))
         l = v * view.src.ct;
     if (on) {
         const int64_t o = (int64_t)a * g.nbx * g.nby + (int64_t)j * g.nbx + i;

@@ -29,20 +29,21 @@ __device__ __forceinline__ int64_t bin_off(const nr_geom& g, int i, int j) {
 // Tomo_OSTR_gold.cpp:245-260.
 // One block of 32 x 4 bins (bx, by) of subset view bz, a warp per detector row.
 // Every thread of the block must call it (with DATA it synchronises the block).
-// views: the plan's views in subset order; rows: the warps' lists (walk.cuh).
+// views: the plan's views in subset order; rows: the warps' lists, LONG and Gmem
+// as in line_integral (walk.cuh).
 //
 // DATA: also the subset's FP64 data term, sum over its bins of
 // ybar + r - y log(ybar + r) with ybar = b exp(-l) -- the data term of the
 // objective (objective.cu) restricted to these views, each bin's term formed
 // exactly as there -- as this block's partial in red[block] (warp shuffles,
 // then a fixed-order block sum).
-template <int K = 4, bool DATA = false>
+template <int K = 4, bool DATA = false, bool LONG = false>
 __device__ __forceinline__ void fp_h_tile(const Geo& G, const float* __restrict__ vol,
                                           float* __restrict__ h,
                                           const ProjView* __restrict__ views, int a0,
                                           const float* __restrict__ y, const float* __restrict__ b,
                                           const float* __restrict__ r, int bx, int by, int bz,
-                                          float2 (*rows)[WALK_ROWS],
+                                          float2 (*rows)[WALK_ROWS], const Geo& Gmem,
                                           double* __restrict__ red = nullptr) {
     const nr_geom& g = G.g;
     const int a = a0 + bz;
@@ -53,7 +54,8 @@ __device__ __forceinline__ void fp_h_tile(const Geo& G, const float* __restrict_
     if (!DATA && j >= g.nby) return;
     double term = 0.0;
     float v, l = 0.f;
-    if (line_integral<K>(G, vol, view, bin_x(g, i), bin_y(g, j), on, rows[threadIdx.y], &v))
+    if (line_integral<K, LONG>(G, Gmem, vol, view, bin_x(g, i), bin_y(g, j), on,
+                               rows[threadIdx.y], &v))
         l = v * view.src.ct;
     if (on) {
         const int64_t B = (int64_t)g.nbx * g.nby;

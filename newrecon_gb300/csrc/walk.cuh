@@ -28,13 +28,15 @@
 namespace nr {
 
 constexpr int WALK_ROWS = 256;   // list entries of a warp (2 KB)
+constexpr int WALK_PAD = 8;      // entries past the last that a round of gathers may step over
 constexpr float WALK_CROSSINGS = 1e6f;   // crossings of an axis: exact in FP32
+constexpr float WALK_RATE = 200.f;       // y crossings per plane: a plane's fit one list
 
 // A view's rays as functions of the bin's position, in voxels and per plane of
 // depth, one line for x and one for y.  down: every ray of the view
-// travels down, at most 2 mm sideways per mm (steeper views, where w resolves
-// positions less well than the path length does, and rays that travel up
-// take the walk of siddon.cuh).
+// travels down, at most 2 mm sideways per mm and WALK_RATE rows per plane
+// (steeper views, where w resolves positions less well than the path length
+// does, and rays that travel up take the walk of siddon.cuh).
 struct WalkLine {
     float c0, c1, s0, s1;   // position c0 + c1 bin, slope s0 + s1 bin: rounded
     float c0l, c1l;         // what c0 and c1 leave out
@@ -52,6 +54,20 @@ struct WalkView {
     WalkLine x, y;
     int down;
 };
+
+// Whether rows of a view take more than one list: the planes and the y
+// crossings of the outermost row that meets the volume, seen from the source
+// straight above (an estimate: either form of the walk takes any row).
+__host__ inline bool walk_long(const nr_geom& g) {
+    auto reach = [&](float a, float len) {
+        return fmaxf(fabsf(a - g.sourceY), fabsf(a + len - g.sourceY));
+    };
+    const float top = g.sourceR - (g.z_p0 + (float)g.nz * g.vz);
+    float slope = reach(g.y_d0, (float)g.nby * g.by) / (g.sourceR + g.detectorR);
+    if (top > 0.f) slope = fminf(slope, reach(g.y_p0, (float)g.ny * g.vy) / top);
+    const float cross = fminf((float)g.ny, slope * g.vz / g.vy * (float)g.nz);
+    return (float)g.nz + cross > (float)(WALK_ROWS - WALK_PAD);
+}
 
 // What the projection of a view starts from.  The device-resident paths keep
 // one per view in their workspace: computed by a thread of each block (sincos
@@ -94,7 +110,8 @@ __device__ __forceinline__ void proj_view(const Geo& G, float theta, ProjView& V
         down = down && fabsf(x - V.src.x0) <= -2.f * fz && fabsf(y - V.src.y0) <= -2.f * fz;
         const float ex = fabsf(V.w.x.at(x)) + (float)g.nz * fabsf(V.w.x.slope(x));
         const float ey = fabsf(V.w.y.at(y)) + (float)g.nz * fabsf(V.w.y.slope(y));
-        down = down && ex < WALK_CROSSINGS && ey < WALK_CROSSINGS;
+        down = down && ex < WALK_CROSSINGS && ey < WALK_CROSSINGS &&
+               fabsf(V.w.y.slope(y)) <= WALK_RATE;
     }
     V.w.down = down;
 }
@@ -157,35 +174,48 @@ __device__ __forceinline__ void depth_range(const DepthAxis& a, float e, int n, 
     }
 }
 
-// The list of a detector row: entries (end depth, offset of the volume row
-// as int bits), n of them, from depth w0 to w1.
+// The list of a stretch of a detector row: entries (end depth, offset of the
+// volume row as int bits), n of them, from depth w0 to w1.  more: the row goes
+// on below w1.
 struct RowList {
     int n;
     float w0, w1;
+    bool more;
 };
 
-// Built by a whole warp; y1: the row's bin centre.  n = 0 when the row misses
-// the volume in y, -1 when the list does not fit.
-template <int PAD>
+// Built by a whole warp; y1: the row's bin centre, from: the end of the stretch
+// before (0: none).  n = 0 when the row misses the volume in y.  WHOLE: only
+// a row that one list holds (n = -1: more).
+template <bool WHOLE>
 __device__ __forceinline__ RowList row_list(const nr_geom& g, const WalkView& V, float y1,
-                                            float2* __restrict__ L) {
+                                            float from, float2* __restrict__ L) {
     RowList R;
     const float e = V.y.at(y1);
     const DepthAxis Y = depth_axis(e, V.y.slope(y1));
     depth_range(Y, e, g.ny, R.w0, R.w1);
-    R.w0 = fmaxf(R.w0, 0.f);
+    R.w0 = fmaxf(R.w0, from);
     R.w1 = fminf(R.w1, (float)g.nz);
     R.n = 0;
+    R.more = false;
     if (!(R.w0 < R.w1)) return R;
     const int ca = depth_first<false>(Y, R.w0);   // y crossings inside: ca, ca + 1, ...
-    const int ny = max(0, depth_first<true>(Y, R.w1) - ca);
     const int ka = (int)R.w0 + 1;                 // z planes inside: ka, ka + 1, ...
-    const int nz = max(0, (int)ceilf(R.w1) - ka);
-    R.n = ny + nz + 1;
-    if (R.n + PAD > WALK_ROWS) {
-        R.n = -1;
-        return R;
+    int ny = max(0, depth_first<true>(Y, R.w1) - ca);
+    int nz = max(0, (int)ceilf(R.w1) - ka);
+    if (ny + nz + 1 + WALK_PAD > WALK_ROWS) {
+        if (WHOLE) {
+            R.n = -1;
+            return R;
+        }
+        // p planes hold at most p rate + 2 crossings and p - 1 planes inside
+        const int p = max(1, (int)__fdividef((float)(WALK_ROWS - WALK_PAD - 4), 1.f + Y.rate));
+        R.more = (float)(ka - 1 + p) < R.w1;
+        R.w1 = fminf(R.w1, (float)(ka - 1 + p));
+        ny = max(0, depth_first<true>(Y, R.w1) - ca);
+        nz = max(0, (int)ceilf(R.w1) - ka);
+        ny = min(ny, WALK_ROWS - WALK_PAD - 1 - nz);
     }
+    R.n = ny + nz + 1;
     const int lane = threadIdx.x;
     auto put = [&](int at, float w, int planes, int rows) {
         const int z = g.nz - ka - planes;
@@ -203,18 +233,20 @@ __device__ __forceinline__ RowList row_list(const nr_geom& g, const WalkView& V,
         const int p = min(nz, max(0, (int)w - ka + 1));
         put(t + p, w, p, t);
     }
-    for (int t = lane; t <= PAD; t += 32) put(ny + nz + t, t == 0 ? R.w1 : NR_FINF, nz, ny);
+    for (int t = lane; t <= WALK_PAD; t += 32)
+        put(ny + nz + t, t == 0 ? R.w1 : NR_FINF, nz, ny);
     __syncwarp();
     return R;
 }
 
-// sum over the segments of one ray of its length in depth times the voxel it
-// lies in: the ray of column x1 through the row list R, L.  K steps per round
-// of reads, as in siddon.cuh.  False (nothing in out) when the ray misses.
+// Adds to *out the segments of one ray, its length in depth times the voxel it
+// lies in each: the ray of column x1 through the row list R, L.  K steps per
+// round of reads (K <= WALK_PAD), as in siddon.cuh.  False when the ray misses.
 template <int K>
 __device__ __forceinline__ bool depth_walk(const nr_geom& g, const WalkView& V, const RowList& R,
                                            const float2* __restrict__ L,
                                            const float* __restrict__ vol, float x1, float* out) {
+    static_assert(K <= WALK_PAD, "list padding");
     const float e = V.x.at(x1);
     const DepthAxis X = depth_axis(e, V.x.slope(x1));
     float s, end;
@@ -235,7 +267,7 @@ __device__ __forceinline__ bool depth_walk(const nr_geom& g, const WalkView& V, 
         L += lo;
     }
     float2 ent = *L;
-    float sum = 0.f;
+    float sum = *out;
     while (s < end) {
         float seg[K];
         int id[K];
@@ -273,26 +305,62 @@ __device__ __forceinline__ float depth_mm(const nr_geom& g, const ViewSrc& S, fl
     return __fdiv_rn(g.vz * sqrtf(dx * dx + dy * dy + dz * dz), fabsf(dz));
 }
 
+// line_integral for the rows that take several lists and for the views of the
+// general walk: {value, 1 where the ray meets the volume}.
+template <int K>
+__device__ __forceinline__ float2 line_far(const Geo& G, const float* __restrict__ vol,
+                                           const ProjView& V, float x1, float y1, bool on,
+                                           float2* __restrict__ L) {
+    const nr_geom& g = G.g;
+    float sum = 0.f;
+    bool hit = false;
+    if (V.w.down) {
+        RowList R;
+        R.w1 = 0.f;
+        do {
+            R = row_list<false>(g, V.w, y1, R.w1, L);
+            if (R.n > 0 && on) hit |= depth_walk<K>(g, V.w, R, L, vol, x1, &sum);
+        } while (R.more);
+        sum *= depth_mm(g, V.src, x1, y1);
+    } else if (on) {
+        hit = trace<0, K>(G, vol, V.src.x0, V.src.y0, V.src.z0, x1, y1, -g.detectorR, &sum);
+    }
+    return make_float2(sum, hit ? 1.f : 0.f);
+}
+template <int K>
+__device__ __noinline__ float2 line_far_call(const Geo& G, const float* __restrict__ vol,
+                                             const ProjView& V, float x1, float y1, bool on,
+                                             float2* __restrict__ L) {
+    return line_far<K>(G, vol, V, x1, y1, on, L);
+}
+
 // The line integral of the ray to (x1, y1), called by a whole warp with one y1
 // (on: the lane has a ray).  False (out untouched) where the ray misses the
-// volume.  L: the warp's list, WALK_ROWS entries of shared memory.
-template <int K>
-__device__ __forceinline__ bool line_integral(const Geo& G, const float* __restrict__ vol,
-                                              const ProjView& V, float x1, float y1, bool on,
+// volume.  L: the warp's list, WALK_ROWS entries of shared memory.  LONG: for
+// volumes whose rows take several lists (walk_long); otherwise those are walked
+// out of line, so that the common walk keeps its registers (FP_BLOCKS).  Gmem:
+// G where it lies in memory, for that call (the address of a copy in registers
+// would put the copy on the stack).
+template <int K, bool LONG = false>
+__device__ __forceinline__ bool line_integral(const Geo& G, const Geo& Gmem,
+                                              const float* __restrict__ vol, const ProjView& V,
+                                              float x1, float y1, bool on,
                                               float2* __restrict__ L, float* out) {
     const nr_geom& g = G.g;
-    if (V.w.down) {
-        const RowList R = row_list<K>(g, V.w, y1, L);
-        if (R.n == 0 || !on) return false;
+    if (!LONG && V.w.down) {
+        const RowList R = row_list<true>(g, V.w, y1, 0.f, L);
+        if (R.n == 0) return false;
         if (R.n > 0) {
-            float sum;
-            if (!depth_walk<K>(g, V.w, R, L, vol, x1, &sum)) return false;
+            float sum = 0.f;
+            if (!on || !depth_walk<K>(g, V.w, R, L, vol, x1, &sum)) return false;
             *out = sum * depth_mm(g, V.src, x1, y1);
             return true;
         }
     }
-    if (!on) return false;
-    return trace<0, K>(G, vol, V.src.x0, V.src.y0, V.src.z0, x1, y1, -g.detectorR, out);
+    const float2 r = LONG ? line_far<K>(G, vol, V, x1, y1, on, L)
+                          : line_far_call<K>(Gmem, vol, V, x1, y1, on, L);
+    if (r.y != 0.f) *out = r.x;
+    return r.y != 0.f;
 }
 
 }  // namespace nr
