@@ -86,6 +86,36 @@ __device__ __forceinline__ float bp_edge(const nr_geom& g, const BpTap& ti, cons
     return bp_rows(d1, d2, tj.frac);
 }
 
+// Adds a view's samples u and (SENS) sn at a distance (ddx, ddy, ddz) from its
+// source to the voxel's sums.
+template <bool SENS>
+__device__ __forceinline__ void bp_add(const nr_geom& g, float s2, float ddx, float ddy, float ddz,
+                                       float u, float sn, float& total, float& total_sens) {
+    const float depth_weight = __fdiv_rn(
+        s2, __fmaf_rn(ddz, ddz, __fmaf_rn(ddx, ddx, __fmul_rn(ddy, ddy))));  // Tomo_OSTR.cu:1634
+    total = __fadd_rn(total, __fmul_rn(__fmul_rn(u, g.vz), depth_weight));
+    if (SENS)
+        total_sens = __fadd_rn(total_sens, __fmul_rn(__fmul_rn(sn, g.vz), depth_weight));
+}
+
+// Writes voxel v from its sums (OSSART: see bp_kernel).
+template <bool OSSART>
+__device__ __forceinline__ void bp_store(float* __restrict__ vol, const float* __restrict__ prior,
+                                         int64_t v, float total, float total_sens, float lambda,
+                                         float beta) {
+    if (!OSSART) {
+        vol[v] = vol[v] + total;
+        return;
+    }
+    float u = 0.f, bt = 0.f;
+    if (total_sens != 0.f) {
+        u = __fdiv_rn(total, total_sens);
+        if (prior) bt = __fdiv_rn(beta * prior[v], total_sens);
+    }
+    const float xn = vol[v] + lambda * (u + bt);
+    vol[v] = xn < 0.f ? 0.f : xn;
+}
+
 // vol[v] += sum_{views} SBP term.  prj planes are consecutive per view
 // (view a-a0 at prj + (a-a0)*B).  index == nullptr means identity order.
 // Block: tile blockIdx.x of the plane, planes [zc blockIdx.y, + zc).
@@ -157,14 +187,7 @@ __global__ void __launch_bounds__(THREADS) bp_kernel(
                     in = in && (unsigned)ti[c].lb < (unsigned)(g.nbx - 1);
                 }
                 auto add = [&](int c, float u, float sn) {
-                    const float ddx = v.x0 - x1[c];
-                    const float depth_weight = __fdiv_rn(
-                        v.s2,
-                        __fmaf_rn(ddz, ddz, __fmaf_rn(ddx, ddx, __fmul_rn(ddy, ddy))));  // :1634
-                    total[c] = __fadd_rn(total[c], __fmul_rn(__fmul_rn(u, g.vz), depth_weight));
-                    if (OSSART)
-                        total_sens[c] =
-                            __fadd_rn(total_sens[c], __fmul_rn(__fmul_rn(sn, g.vz), depth_weight));
+                    bp_add<OSSART>(g, v.s2, v.x0 - x1[c], ddy, ddz, u, sn, total[c], total_sens[c]);
                 };
                 if (__all_sync(0xffffffffu, in)) {
                     float val[NC][4];
@@ -206,27 +229,60 @@ __global__ void __launch_bounds__(THREADS) bp_kernel(
         for (int r = warp; r < BP_T && y0 + r < g.ny; r += THREADS / 32) {
             if (ix >= g.nx) break;
             const int64_t v = ((int64_t)iz * g.ny + y0 + r) * g.nx + ix;
-            if (!OSSART) {
-                vol[v] = vol[v] + sums[0][r][lane];
-                continue;
-            }
-            const float sens = sums[OSSART ? 1 : 0][r][lane];
-            float u = 0.f, bt = 0.f;
-            if (sens != 0.f) {
-                u = __fdiv_rn(sums[0][r][lane], sens);
-                if (prior) bt = __fdiv_rn(beta * prior[v], sens);
-            }
-            const float xn = vol[v] + lambda * (u + bt);
-            vol[v] = xn < 0.f ? 0.f : xn;
+            bp_store<OSSART>(vol, prior, v, sums[0][r][lane], sums[OSSART ? 1 : 0][r][lane], lambda,
+                             beta);
         }
     }
 }
 
-// Planes per block: as many as leave two rounds of resident blocks, at most 8.
-// Four columns per thread (256 threads), so that the views' and rows' values are
-// read once for four voxels; one (1024 threads) while the tiles of all planes
-// leave SMs idle and the chain of one thread is what the call takes (64 x 64 x 20,
-// five views: 8.8 us against 10.6; 140 x 100 x 30: 19.1 against 14.7).
+// The same, a thread per voxel of the volume taken as one row: for volumes that
+// tiles would leave mostly idle (launch_sbp).  What these calls take is the chain
+// of one thread, and this one has neither the tables nor the turn.
+template <bool OSSART>
+__global__ void __launch_bounds__(128) bp_small_kernel(
+    const __grid_constant__ Geo G, float* __restrict__ vol, const float* __restrict__ prj,
+    const float* __restrict__ prior, const float* __restrict__ angles,
+    const int32_t* __restrict__ index, int a0, int nv, float lambda, float beta) {
+    __shared__ ViewSrc sv[2 * BP_VIEWS];
+    const nr_geom& g = G.g;
+    const unsigned n = (unsigned)g.nx * g.ny * g.nz;
+    const unsigned at = blockIdx.x * 128 + threadIdx.x, v = min(at, n - 1);
+    const unsigned row = v / (unsigned)g.nx, z = row / (unsigned)g.ny;
+    const float x1 = vox_x(g, v - row * g.nx), y1 = vox_y(g, row - z * g.ny), z1 = vox_z(g, z);
+    const int64_t B = (int64_t)g.nbx * g.nby;
+    float total = 0.f, total_sens = 0.f;
+    for (int c0 = 0; c0 < nv; c0 += 2 * BP_VIEWS) {
+        const int cn = min(2 * BP_VIEWS, nv - c0);
+        if (c0) __syncthreads();
+        load_views(g, sv, angles, index, a0 + c0, cn);
+        __syncthreads();
+#pragma unroll 4
+        for (int t = 0; t < cn; t++) {
+            const ViewSrc s = sv[t];
+            if (z1 == s.z0) continue;  // the term is 0
+            const float r = __fdiv_rn(-g.detectorR - s.z0, z1 - s.z0);
+            const BpTap ti = bp_tap(__fmaf_rn(x1 - s.x0, r, s.x0), g.x_d0, g.bx);
+            const BpTap tj = bp_tap(__fmaf_rn(y1 - s.y0, r, s.y0), g.y_d0, g.by);
+            float sn = 0.f;
+            const float u = bp_edge<OSSART>(g, ti, tj, prj + (int64_t)(c0 + t) * B, &sn);
+            bp_add<OSSART>(g, s.s2, s.x0 - x1, s.y0 - y1, s.z0 - z1, u, sn, total, total_sens);
+        }
+    }
+    if (at < n) bp_store<OSSART>(vol, prior, v, total, total_sens, lambda, beta);
+}
+
+// The form by size; all give the same bits.
+//  - A thread per voxel while that makes at most four blocks per SM, or where the
+//    tiles would be filled to less than two fifths.  40 x 24 x 8, five views:
+//    5.4 us against 6.5 by tiles; 1000 x 1 x 300: 14.9 against 98; 33 x 33 x 640 (a
+//    fill of 0.27): 26 against 46; but 1000 x 33 x 33 (0.5): 43 against 29, and
+//    96 x 96 x 32 (295 k voxels): 30 against 8.3.
+//  - Tiles of one column per thread (1024 threads) while all planes' tiles leave SMs
+//    idle: 64 x 64 x 38, five views: 6.8 us against 8.1; 140 x 100 x 30: 16.7
+//    against 10.9.
+//  - Tiles of four columns per thread, so that the views' and rows' values are read
+//    once for four voxels.  Planes per block: as many as leave two rounds of
+//    resident blocks, at most 8.
 template <bool OSSART>
 static nr_status launch_sbp(const nr_geom& g, float* vol, const float* prj, const float* prior,
                             const float* angles, const int32_t* index, int a0, int a1,
@@ -235,7 +291,11 @@ static nr_status launch_sbp(const nr_geom& g, float* vol, const float* prj, cons
     const int64_t full = tiles * g.nz / (152 * 16);
     const int zc = (int)(full < 1 ? 1 : (full > 8 ? 8 : full));
     const dim3 grd((unsigned)tiles, cdiv(g.nz, zc));
-    if (tiles * g.nz <= 152)
+    const int64_t voxels = (int64_t)g.nx * g.ny * g.nz;
+    if (voxels <= 152 * 4 * 128 || 5 * voxels < 2 * tiles * BP_T * BP_T * g.nz)
+        bp_small_kernel<OSSART><<<cdiv(voxels, 128), 128, 0, s>>>(
+            make_geo(g), vol, prj, prior, angles, index, a0, a1 - a0, lambda, beta);
+    else if (tiles * g.nz <= 152)
         bp_kernel<OSSART, 1024><<<grd, 1024, 0, s>>>(make_geo(g), vol, prj, prior, angles, index,
                                                      a0, a1 - a0, zc, lambda, beta);
     else
