@@ -263,9 +263,9 @@ __global__ void __launch_bounds__(128) gamma_length_kernel(const __grid_constant
         const int j = (blockIdx.y * GL_ROWS + k) * 4 + threadIdx.y;
         if (j >= g.nby) break;
         const float dy = bin_y(g, j) - S.y0;
-        // the roundings of ray_axes: dx^2, + dy^2, + dz^2 fused
+        // the roundings of ray_axes as compiled: dy^2, then dx^2 and dz^2 fused
         const float L =
-            sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))));
+            sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy))));
         float l = lo, h = hi;
         clip(S.y0, dy, g.y_p0, G.ymax, l, h);
         const float gam = (L > 0.f && L < NR_FINF && l < h) ? L : 0.f;
