@@ -40,9 +40,7 @@ struct ViewSrc {
     float x0, y0, z0, ct, s2;
 };
 
-__device__ __forceinline__ ViewSrc view_source(const nr_geom& g, float theta) {
-    double s, c;
-    sincos((double)theta, &s, &c);
+__device__ __forceinline__ ViewSrc view_source(const nr_geom& g, double s, double c) {
     ViewSrc v;
     v.x0 = (float)((double)g.sourceR * s);
     v.z0 = (float)((double)g.sourceR * c);
@@ -50,6 +48,11 @@ __device__ __forceinline__ ViewSrc view_source(const nr_geom& g, float theta) {
     v.ct = (float)c;
     v.s2 = v.x0 * v.x0 + v.y0 * v.y0 + v.z0 * v.z0;
     return v;
+}
+__device__ __forceinline__ ViewSrc view_source(const nr_geom& g, float theta) {
+    double s, c;
+    sincos((double)theta, &s, &c);
+    return view_source(g, s, c);
 }
 
 // Bin centre on the stationary detector, Tomo_OSTR.cu:1349-1356.  The

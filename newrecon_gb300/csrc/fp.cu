@@ -228,14 +228,15 @@ __global__ void __launch_bounds__(128) gamma_chord_kernel(const __grid_constant_
 // quotient pair per bin to form instead of three.  The interval's ends are the
 // same minima and maxima, the ray meets the volume or not as there.  125 M
 // bins with scatter: 0.56 ms against 1.78 ms with a block's view computed by
-// one of its threads and three pairs per bin.
+// one of its threads and three pairs per bin.  rows: GL_ROWS, or fewer while that
+// leaves SMs without eight blocks.
 constexpr int GL_ROWS = 8;
 __global__ void __launch_bounds__(128) gamma_length_kernel(const __grid_constant__ Geo G,
                                                            float* __restrict__ out,
                                                            const ProjView* __restrict__ views,
                                                            const int32_t* __restrict__ index,
                                                            const float* __restrict__ y,
-                                                           const float* __restrict__ r) {
+                                                           const float* __restrict__ r, int rows) {
     const nr_geom& g = G.g;
     const int a = blockIdx.z;
     const ViewSrc S = views[a].src;
@@ -259,8 +260,8 @@ __global__ void __launch_bounds__(128) gamma_length_kernel(const __grid_constant
     const float* ra = r ? r + (int64_t)a * B : nullptr;
     float* oa = out + (int64_t)index[a] * B;
 #pragma unroll 2
-    for (int k = 0; k < GL_ROWS; k++) {
-        const int j = (blockIdx.y * GL_ROWS + k) * 4 + threadIdx.y;
+    for (int k = 0; k < rows; k++) {
+        const int j = (blockIdx.y * rows + k) * 4 + threadIdx.y;
         if (j >= g.nby) break;
         const float dy = bin_y(g, j) - S.y0;
         // the roundings of ray_axes as compiled: dy^2, then dx^2 and dz^2 fused
@@ -474,16 +475,23 @@ nr_status launch_fp_h_data(const nr_geom& g, int k, const float* x, float* h,
     return launch_status();
 }
 
-// The views of a plan, subset order (angles[index[a]]).
-__global__ void views_kernel(const __grid_constant__ Geo G, const float* __restrict__ angles,
-                             const int32_t* __restrict__ index, ProjView* __restrict__ views) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < G.g.n_angles) proj_view(G, angles[index[a]], views[a]);
+// A plan's view order and views, its status words cleared.  Subset-major
+// order, Tomo_OSTR_gold.cpp:628-642: position i Vs + j holds original view j M + i.
+__global__ void plan_views_kernel(const __grid_constant__ Geo G, const float* __restrict__ angles,
+                                  int M, int32_t* __restrict__ index,
+                                  ProjView* __restrict__ views, int* __restrict__ status) {
+    const int a = blockIdx.x * 32 + threadIdx.x, A = G.g.n_angles, Vs = A / M;
+    if (blockIdx.x == 0) status[threadIdx.x] = status[threadIdx.x + 32] = 0;
+    if (a >= A) return;
+    const int from = (a % Vs) * M + a / Vs;
+    index[a] = from;
+    proj_view(G, angles[from], views[a]);
 }
 
-nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
-                       ProjView* views, cudaStream_t st) {
-    views_kernel<<<cdiv(g.n_angles, 32), 32, 0, st>>>(make_geo(g), angles, index, views);
+nr_status launch_plan_views(const nr_geom& g, const float* angles, int M, int32_t* index,
+                            ProjView* views, int* status, cudaStream_t st) {
+    plan_views_kernel<<<cdiv(g.n_angles, 32), 32, 0, st>>>(make_geo(g), angles, M, index, views,
+                                                           status);
     return launch_status();
 }
 
@@ -496,8 +504,11 @@ nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const P
         dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4), g.n_angles);
         gamma_chord_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r);
     } else {
-        dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4 * GL_ROWS), g.n_angles);
-        gamma_length_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r);
+        const int64_t single = (int64_t)cdiv(g.nbx, 32) * cdiv(g.nby, 4) * g.n_angles;
+        const int64_t n = single / (152 * 8);
+        const int rows = (int)(n < 1 ? 1 : (n > GL_ROWS ? GL_ROWS : n));
+        dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4 * rows), g.n_angles);
+        gamma_length_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r, rows);
     }
     return launch_status();
 }

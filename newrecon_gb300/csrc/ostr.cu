@@ -6,7 +6,6 @@
 //   status   int32[64]                  device status word (NR_FLAG_*)
 //   red      double[red_n]              per-block partial sums of the objective
 //   index    int32[A]                   view order (subset-major)
-//   angles   float[A]
 //   views    ProjView[A]                projection constants, subset order (walk.cuh)
 //   y, b, r  float[A][BINSy][BINSx]     scan in subset order, detector i fastest
 //   d        float[N]                   curvature denominators
@@ -47,8 +46,8 @@ nr_status launch_bp_tables(const nr_geom& g, const ProjView* views, float4* tx, 
                            bool exact, cudaStream_t st);
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,
                            int Vs, cudaStream_t st);
-nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
-                       ProjView* views, cudaStream_t st);
+nr_status launch_plan_views(const nr_geom& g, const float* angles, int M, int32_t* index,
+                            ProjView* views, int* status, cudaStream_t st);
 nr_status launch_objective(const nr_geom& g, int pot, float delta, const float* x,
                            const ProjView* views, const float* y,
                            const float* b, const float* r, double* red, int64_t red_n,
@@ -62,7 +61,7 @@ nr_status launch_penalty(const nr_geom& g, int pot, float delta, const float* x,
                          int64_t red_n, double* out, cudaStream_t st);
 
 struct Layout {
-    size_t status, red, index, angles, views, y, b, r, d, xtmp, h, bpx, bpy, gc, total;
+    size_t status, red, index, views, y, b, r, d, xtmp, h, bpx, bpy, gc, total;
     int64_t red_n;
 };
 
@@ -83,7 +82,6 @@ static Layout layout(const nr_geom& g, const nr_ostr_params& p) {
     L.status = take(64 * sizeof(int32_t));
     L.red = take((size_t)L.red_n * sizeof(double));
     L.index = take(A * sizeof(int32_t));
-    L.angles = take(A * sizeof(float));
     L.views = take(A * sizeof(ProjView));
     L.y = take(A * B * sizeof(float));
     L.b = take(A * B * sizeof(float));
@@ -103,7 +101,7 @@ struct WS {
     double* red;
     int32_t* index;
     ProjView* views;
-    float *angles, *y, *b, *r, *d, *xtmp, *h, *gc;
+    float *y, *b, *r, *d, *xtmp, *h, *gc;
     float4 *bpx, *bpy;
     int64_t red_n;
     BpTab tab() const { return BpTab{bpx, bpy}; }
@@ -115,7 +113,6 @@ static WS carve(void* base, const Layout& L) {
     w.status = (int*)(c + L.status);
     w.red = (double*)(c + L.red);
     w.index = (int32_t*)(c + L.index);
-    w.angles = (float*)(c + L.angles);
     w.views = (ProjView*)(c + L.views);
     w.y = (float*)(c + L.y);
     w.b = (float*)(c + L.b);
@@ -162,34 +159,11 @@ static nr_status check_ws(const nr_geom* g, const nr_ostr_params* p, void* ws, s
     return NR_OK;
 }
 
-// Subset-major view order, Tomo_OSTR_gold.cpp:628-642: position i*Vs + j
-// holds original view j*M + i.
-__global__ void index_kernel(int32_t* idx, const float* __restrict__ angles_in,
-                             float* __restrict__ angles_out, int A, int M) {
-    const int Vs = A / M;
-    for (int p = threadIdx.x; p < A; p += blockDim.x) {
-        idx[p] = (p % Vs) * M + p / Vs;
-        angles_out[p] = angles_in[p];
-    }
-}
-
 __global__ void clear_status_kernel(int* s) {
     if (threadIdx.x < 64) s[threadIdx.x] = 0;
 }
 
 __global__ void set_word_kernel(int* p, int v) { *p = v; }
-
-// The two set-up launches the OS-SART driver (sart.cu) shares.
-nr_status launch_subset_index(int32_t* idx, const float* angles_in, float* angles_out, int A,
-                              int M, cudaStream_t s) {
-    index_kernel<<<1, 256, 0, s>>>(idx, angles_in, angles_out, A, M);
-    return launch_status();
-}
-
-nr_status launch_clear_status(int* status, cudaStream_t s) {
-    clear_status_kernel<<<1, 64, 0, s>>>(status);
-    return launch_status();
-}
 
 // Section pointers of a set-up workspace, for the batched path (batch.cu).
 nr_status ostr_sections(const nr_geom* g, const nr_ostr_params* p, void* ws, size_t bytes,
@@ -242,10 +216,7 @@ NR_API nr_status nr_ostr_setup(const nr_geom* g, const nr_ostr_params* p, const 
     cudaStream_t s = as_stream(stream);
     WS w = carve(workspace, L);
     const int A = g->n_angles, M = p->subset_num, Vs = A / M;
-    clear_status_kernel<<<1, 64, 0, s>>>(w.status);
-    index_kernel<<<1, 256, 0, s>>>(w.index, angles, w.angles, A, M);
-    if ((st = launch_status()) != NR_OK) return st;
-    if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
+    if ((st = launch_plan_views(*g, angles, M, w.index, w.views, w.status, s)) != NR_OK) return st;
     if ((st = launch_bp_tables(*g, w.views, w.bpx, w.bpy, true, s)) != NR_OK) return st;
     // [view][i][j] original order -> [view][j][i] subset order.
     if ((st = launch_transpose(w.y, prj, g->nbx, g->nby, A, M, Vs, s)) != NR_OK) return st;

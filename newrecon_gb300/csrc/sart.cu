@@ -26,7 +26,6 @@
 // first, so nr_ostr_check reads it as for OSTR):
 //   status int32[64]
 //   index  int32[A]                   view order (subset-major)
-//   angles float[A]
 //   views  ProjView[A]                projection constants, subset order (walk.cuh)
 //   p      float[A][BINSy][BINSx]     line integrals, subset order, i fastest
 //   norm   float[A][BINSy][BINSx]     chord lengths, same layout
@@ -38,20 +37,17 @@
 
 namespace nr {
 
-nr_status launch_subset_index(int32_t* idx, const float* angles_in, float* angles_out, int A,
-                              int M, cudaStream_t s);
-nr_status launch_clear_status(int* status, cudaStream_t s);
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,
                            int Vs, cudaStream_t st);
-nr_status launch_views(const nr_geom& g, const float* angles, const int32_t* index,
-                       ProjView* views, cudaStream_t st);
+nr_status launch_plan_views(const nr_geom& g, const float* angles, int M, int32_t* index,
+                            ProjView* views, int* status, cudaStream_t st);
 nr_status launch_bp_tables(const nr_geom& g, const ProjView* views, float4* tx, float4* ty,
                            bool exact, cudaStream_t st);
 
 namespace {
 
 struct SartLayout {
-    size_t status, index, angles, views, p, norm, diff, xtmp, bpx, bpy, total;
+    size_t status, index, views, p, norm, diff, xtmp, bpx, bpy, total;
 };
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -69,7 +65,6 @@ SartLayout sart_layout(const nr_geom& g, const nr_sart_params& p) {
     };
     L.status = take(64 * sizeof(int32_t));
     L.index = take(A * sizeof(int32_t));
-    L.angles = take(A * sizeof(float));
     L.views = take(A * sizeof(ProjView));
     L.p = take(A * B * sizeof(float));
     L.norm = take(A * B * sizeof(float));
@@ -85,7 +80,7 @@ struct SartWS {
     int* status;
     int32_t* index;
     ProjView* views;
-    float *angles, *p, *norm, *diff, *xtmp;
+    float *p, *norm, *diff, *xtmp;
     float4 *bpx, *bpy;
 };
 
@@ -94,7 +89,6 @@ SartWS sart_carve(void* base, const SartLayout& L) {
     SartWS w;
     w.status = (int*)(c + L.status);
     w.index = (int32_t*)(c + L.index);
-    w.angles = (float*)(c + L.angles);
     w.views = (ProjView*)(c + L.views);
     w.p = (float*)(c + L.p);
     w.norm = (float*)(c + L.norm);
@@ -370,9 +364,7 @@ NR_API nr_status nr_sart_setup(const nr_geom* g, const nr_sart_params* p, const 
     cudaStream_t s = as_stream(stream);
     SartWS w = sart_carve(workspace, L);
     const int A = g->n_angles, M = p->subset_num, Vs = A / M;
-    if ((st = launch_clear_status(w.status, s)) != NR_OK) return st;
-    if ((st = launch_subset_index(w.index, angles, w.angles, A, M, s)) != NR_OK) return st;
-    if ((st = launch_views(*g, w.angles, w.index, w.views, s)) != NR_OK) return st;
+    if ((st = launch_plan_views(*g, angles, M, w.index, w.views, w.status, s)) != NR_OK) return st;
     if ((st = launch_bp_tables(*g, w.views, w.bpx, w.bpy, false, s)) != NR_OK) return st;
     if (cudaMemsetAsync(w.diff + (int64_t)Vs * g->nbx * g->nby, 0, bp_pad(*g) * sizeof(float),
                         s) != cudaSuccess)

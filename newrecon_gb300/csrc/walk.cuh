@@ -81,9 +81,9 @@ struct ProjView {
 
 __device__ __forceinline__ void proj_view(const Geo& G, float theta, ProjView& V) {
     const nr_geom& g = G.g;
-    V.src = view_source(g, theta);
     double sn, cs;
     sincos((double)theta, &sn, &cs);
+    V.src = view_source(g, sn, cs);
     V.x0 = (double)g.sourceR * sn;
     V.z0 = (double)g.sourceR * cs;
     const double x0 = V.src.x0, y0 = V.src.y0, z0 = V.src.z0;
