@@ -229,9 +229,9 @@ __global__ void __launch_bounds__(256) sart_fp_diff_4r_kernel(
     const int64_t B = (int64_t)g.nbx * g.nby;
     const int64_t off = bin_off<true>(g, i, j);
     const float nv = norm[(int64_t)a * B + off];
-    const float est = COS ? m * view.src.ct : m;
-    diff[(int64_t)blockIdx.z * B + off] = nv != 0.f ? __fdiv_rn(p[(int64_t)a * B + off] - est, nv)
-                                                    : 0.f;
+    const float line = p[(int64_t)a * B + off];
+    const float dif = COS ? __fmaf_rn(-m, view.src.ct, line) : line - m;  // one rounding
+    diff[(int64_t)blockIdx.z * B + off] = nv != 0.f ? __fdiv_rn(dif, nv) : 0.f;
 }
 
 template <int KIND, int ZC, int NV>
