@@ -149,7 +149,8 @@ typedef struct nr_ostr_params {
     float delta;               /* potential scale (1/mm), > 0 unless Q2          */
     int32_t fp_batch;          /* Siddon steps per gather round: 2, 4, 8 (0 = 4) */
     int32_t upd_planes;        /* z planes per update block: 8, 16, 32 (0: 16, or
-                                  fewer for a volume that would not fill the GPU) */
+                                  fewer for a volume -- in a batch, for cases --
+                                  that would not fill the GPU)                   */
     int32_t fp_stage;          /* NR_STAGE_OFF (default): the projection gathers
                                   the volume through L1/L2; NR_STAGE_TMA: it stages
                                   the volume slab by slab in shared memory by TMA

@@ -35,7 +35,7 @@
 namespace nr {
 
 constexpr int BATCH_MAX = 64;
-constexpr int N_ZC = 3;                      // update slab depths 8, 16, 32 planes
+constexpr int N_ZC = 4;                      // update slab depths 4, 8, 16, 32 planes
 constexpr int N_FORM = 2;                    // several views per subset; one view
 constexpr int N_CLASSES = 4 * N_FORM * N_ZC; // potential x form x slab depth
 
@@ -54,11 +54,13 @@ struct CaseDev {
     int fp_tx, fp_ty;      // detector tiles of 32 x 4 bins
     int up_tx, up_ty;      // volume tiles of 32 x 8 columns
     int form;              // update form (N_FORM)
-    int zc;                // z planes per update item (the plan's upd_planes)
+    int zc;                // z planes per update item (the plan's upd_planes, or by size)
     int64_t N;
 };
 
-__host__ __device__ constexpr int zc_index(int zc) { return zc == 8 ? 0 : (zc == 32 ? 2 : 1); }
+__host__ __device__ constexpr int zc_index(int zc) {
+    return zc == 4 ? 0 : (zc == 8 ? 1 : (zc == 16 ? 2 : 3));
+}
 __host__ __device__ constexpr int upd_class(int pot, int form, int zc) {
     return (N_FORM * pot + form) * N_ZC + zc_index(zc);
 }
@@ -201,11 +203,25 @@ NR_API nr_status nr_batch_prepare(const nr_batch_case* cases, int32_t n_cases, v
             return NR_ERR_BAD_ARGUMENT;
     }
     auto total_sub = [&](int c) { return cases[c].n_iters * cases[c].p.subset_num; };
-    auto zc_of = [&](int c) { return cases[c].p.upd_planes == 0 ? UZC : cases[c].p.upd_planes; };
-    auto cls_of = [&](int c) {
-        const nr_batch_case& k = cases[c];
-        return upd_class(k.p.potential, k.g.n_angles == k.p.subset_num ? 1 : 0, zc_of(c));
+    auto form_of = [&](int c) { return cases[c].g.n_angles == cases[c].p.subset_num ? 1 : 0; };
+    // the cases that leave the depth open share one per potential and form, and
+    // with it a launch; it goes by the blocks of them all
+    int open_zc[4][N_FORM];
+    for (int pot = 0; pot < 4; pot++)
+        for (int form = 0; form < N_FORM; form++)
+            open_zc[pot][form] = upd_planes_by([&](int zc) {
+                int64_t n = 0;
+                for (int c = 0; c < n_cases; c++)
+                    if (cases[c].p.upd_planes == 0 && cases[c].p.potential == pot &&
+                        form_of(c) == form && geom_ok(&cases[c].g))
+                        n += upd_blocks(cases[c].g, zc);
+                return n;
+            });
+    auto zc_of = [&](int c) {
+        const nr_ostr_params& p = cases[c].p;
+        return p.upd_planes == 0 ? open_zc[p.potential][form_of(c)] : p.upd_planes;
     };
+    auto cls_of = [&](int c) { return upd_class(cases[c].p.potential, form_of(c), zc_of(c)); };
     // case order: by class, then by sub-iteration count, longest first (stable)
     int order[BATCH_MAX];
     for (int c = 0; c < n_cases; c++) order[c] = c;
@@ -295,12 +311,14 @@ namespace {
 template <int POT, int NV>
 void launch_class_z(int zi, const BatchTable& P, int32_t k, int lo, int hi, cudaStream_t s) {
     const dim3 blk(UTX, UTY / 2);
-    if (zi == 0)
+    if (zi == zc_index(4))
+        update_batch_kernel<POT, NV, 4><<<hi - lo, blk, 0, s>>>(P, k, lo);
+    else if (zi == zc_index(8))
         update_batch_kernel<POT, NV, 8><<<hi - lo, blk, 0, s>>>(P, k, lo);
-    else if (zi == 2)
-        update_batch_kernel<POT, NV, 32><<<hi - lo, blk, 0, s>>>(P, k, lo);
-    else
+    else if (zi == zc_index(16))
         update_batch_kernel<POT, NV, 16><<<hi - lo, blk, 0, s>>>(P, k, lo);
+    else
+        update_batch_kernel<POT, NV, 32><<<hi - lo, blk, 0, s>>>(P, k, lo);
 }
 
 template <int POT>

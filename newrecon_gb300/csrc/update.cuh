@@ -26,12 +26,18 @@ constexpr int UPD_BLOCKS = 5;
 
 // Planes per block when the caller leaves the choice open: 16, or fewer when
 // that leaves SMs without their UPD_BLOCKS blocks (a 256 x 128 x 24 volume makes
-// 256 blocks of 16 planes, 768 of 4).
-__host__ inline int upd_planes_auto(const nr_geom& g) {
-    const int64_t tiles = (int64_t)((g.nx + UTX - 1) / UTX) * ((g.ny + UTY - 1) / UTY);
+// 256 blocks of 16 planes, 768 of 4).  blocks(zc): those of a launch.
+template <class F>
+__host__ inline int upd_planes_by(F blocks) {
     for (int zc = UZC; zc > 4; zc /= 2)
-        if (tiles * ((g.nz + zc - 1) / zc) >= 152 * UPD_BLOCKS) return zc;
+        if (blocks(zc) >= 152 * UPD_BLOCKS) return zc;
     return 4;
+}
+__host__ inline int64_t upd_blocks(const nr_geom& g, int zc) {
+    return (int64_t)cdiv(g.nx, UTX) * cdiv(g.ny, UTY) * cdiv(g.nz, zc);
+}
+__host__ inline int upd_planes_auto(const nr_geom& g) {
+    return upd_planes_by([&](int zc) { return upd_blocks(g, zc); });
 }
 
 // The five distinct neighbour weights 1/sqrt(dx^2+dy^2+(dz zr)^2) of the
