@@ -8,12 +8,13 @@ computes the same result, bit for bit):
   more registers (fewer resident warps); 2 and 4 are also tried with the
   volume staged slab by slab in shared memory by TMA (``fp_stage``), where
   the geometry allows it;
-* ``upd_planes`` -- z planes walked per block by the fused update (8, 16, 32):
-  deeper slabs amortise the planes beside the slab, shallower ones give more
-  blocks; tried with each update tile (``upd_tile``: two voxels per thread
-  walking the planes in registers; or one voxel per thread with the planes
-  streamed by TMA through a ring, where the volume's rows allow TMA); a tile
-  other than the default must win by ``TILE_MARGIN``.
+* ``upd_planes`` -- z planes walked per block by the fused update (8, 16, 32, or
+  0: the default, chosen by the volume's size): deeper slabs amortise the planes
+  beside the slab, shallower ones give more blocks; tried with each update tile
+  (``upd_tile``: two voxels per thread walking the planes in registers; or one
+  voxel per thread with the planes streamed by TMA through a ring, where the
+  volume's rows allow TMA); a tile other than the default must win by
+  ``TILE_MARGIN``.
 
 The tuner times each variant on the plan's own geometry (CUDA events on the
 launching stream, best of a few repetitions over all subsets) and keeps the
@@ -33,7 +34,7 @@ FP_BATCHES = (2, 4, 8)
 # (fp_batch, fp_stage) variants of the projection: direct gathers for every
 # batch, TMA-staged slabs for 2 and 4
 FP_VARIANTS = ((2, 0), (4, 0), (8, 0), (2, 1), (4, 1))
-UPD_PLANES = (8, 16, 32)
+UPD_PLANES = (8, 16, 32, 0)  # 0: by size (4 planes on small volumes)
 UPD_TILES = (0, 2)  # NR_TILE_1, NR_TILE_TMA (NR_TILE_2 runs NR_TILE_1's kernel)
 TILE_NAMES = {0: "", 2: "-tma"}
 # A tile other than the default is kept only when it beats the default's best
@@ -52,7 +53,7 @@ def signature(plan) -> str:
     p = plan.params
     dev = torch.cuda.get_device_name(plan.ws.device)
     return (f"{dev}|{g.nx}x{g.ny}x{g.nz}|{g.nbx}x{g.nby}|A{g.n_angles}|M{p.subset_num}"
-            f"|pot{p.potential}|scat{p.has_scatter}|v5")
+            f"|pot{p.potential}|scat{p.has_scatter}|v6")
 
 
 def _load() -> Dict[str, dict]:
@@ -153,7 +154,7 @@ def tune(plan, x: Optional[torch.Tensor] = None, reps: int = 3,
     plan.params.upd_tile = best_t
     rec = {"fp_batch": best_k, "fp_stage": best_st, "upd_planes": best_z, "upd_tile": best_t,
            "fp_ms": {f"{k}{'-tma' if st else ''}": v for (k, st), v in fp_ms.items()},
-           "update_ms": {f"{z}{TILE_NAMES[t]}": v for (t, z), v in up_ms.items()}}
+           "update_ms": {f"{z or 'auto'}{TILE_NAMES[t]}": v for (t, z), v in up_ms.items()}}
     if use_cache:
         _store(key, rec)
     return best_k, best_z, rec
