@@ -241,13 +241,32 @@ __device__ __forceinline__ float4 bp_taps_at(float mb, int n, bool valid) {
     return bp_taps(lb, mb - ((float)lb + 0.5f), n, valid);
 }
 
-// EXACT: positions in double, the fraction rounded once (a float position of
-// some thousand bins is 1e-4 bin off); otherwise the float arithmetic that the
-// OS-SART update keeps.
-__device__ __forceinline__ float4 bp_taps_at(double mb, int n, bool valid) {
-    const double f = floor(mb - 0.5);
-    const int lb = (int)f;
-    return bp_taps(lb, (float)(mb - 0.5 - f), n, valid);
+// Detector positions along a row of voxels, A + q B bins less a half, in two
+// floats each: the fraction is then rounded once (a float position of some
+// thousand bins is 1e-4 bin off) without FP64 per entry.
+struct BpLine {
+    float ah, al, bh, bl;
+};
+__device__ __forceinline__ BpLine bp_line(double a, double b) {
+    BpLine l;
+    l.ah = (float)a;
+    l.al = (float)(a - l.ah);
+    l.bh = (float)b;
+    l.bl = (float)(b - l.bh);
+    return l;
+}
+__device__ __forceinline__ float4 bp_taps_on(const BpLine& l, int q, int n, bool valid) {
+    const float x = (float)q;
+    const float p = __fmul_rn(x, l.bh), pe = __fmaf_rn(x, l.bh, -p);
+    const float s = __fadd_rn(l.ah, p), t = __fsub_rn(s, l.ah);
+    const float se = __fadd_rn(__fsub_rn(l.ah, __fsub_rn(s, t)), __fsub_rn(p, t));
+    const float lo = __fadd_rn(se, __fadd_rn(pe, __fmaf_rn(x, l.bl, l.al)));
+    float f = floorf(s), r = __fadd_rn(__fsub_rn(s, f), lo);
+    if (r >= 1.f || r < 0.f) {   // s and s + lo on two sides of an integer
+        f += r < 0.f ? -1.f : 1.f;
+        r = fmaxf(__fadd_rn(__fsub_rn(s, f), lo), 0.f);
+    }
+    return bp_taps((int)f, r, n, valid);
 }
 
 // One view's back-projection term of one voxel, added to capL, from its table
