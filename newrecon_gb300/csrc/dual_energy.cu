@@ -152,7 +152,7 @@ __device__ __forceinline__ bool de_pow2(float b, float a, float w1, float& r) {
 // the FP64 pipe was 66 % busy and bound the kernel), so a warp writes its open
 // outputs' numbers to a list and evaluates the list with all lanes.
 //
-// Bound by instruction issue (231 M warp instructions, 66 % issue): 295 us for
+// Bound by instruction issue (231 M warp instructions, 66 % issue): 280 us for
 // nine weights of 1024 x 512 x 60 (its 1.38 GB take 204 us), from 790 us with
 // FP64 in place; 350 us with scalar FP32.
 constexpr int DE_TILE = 128;
@@ -162,9 +162,6 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
     const float* he, const float* le, float* d, int64_t n,
     const __grid_constant__ DeWeights W) {
     __shared__ uint16_t list[8][DE_TILE * DE_MAX_WEIGHTS];
-    __shared__ double sw[DE_MAX_WEIGHTS];
-    if (threadIdx.x < DE_MAX_WEIGHTS) sw[threadIdx.x] = W.w[threadIdx.x];
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint16_t* open = list[warp];
     const int64_t step = (int64_t)gridDim.x * 8 * DE_TILE;
@@ -194,6 +191,10 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
             hb[t] = __fmul_rn(fabsf(h[t]), 0x1p-45f);
             lm[t] = l[t] == 0.f && __float_as_uint(h[t]) != 0x80000000u ? 0.f : 0x1p-100f;
         }
+        const int lim = (int)(n - i < DE_TILE ? n - i : DE_TILE);
+        // nothing to subtract in the warp's voxels (air, a masked background)
+        const bool air = __all_sync(0xffffffffu, lm[0] == 0.f && lm[1] == 0.f && lm[2] == 0.f &&
+                                                     lm[3] == 0.f);
         uint64_t bad = 0;  // bit 4 k + t: weight k of voxel t is left to FP64
         float* row = d + i;
 #pragma unroll 1
@@ -206,10 +207,15 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
                     m |= de_pow2(h[t], l[t], W.w1[k], o[t]) ? 0u : 1u << t;
             } else if ((W.fast >> k) & 1u) {
                 const float w1 = W.w1[k], w2 = W.w2[k];
+                if (air) {
 #pragma unroll
-                for (int t = 0; t < 4; t += 2)
-                    m |= de_fast2(pk2(h[t], h[t + 1]), hb[t], hb[t + 1], l[t], l[t + 1], lm[t],
-                                  lm[t + 1], w1, w2, o[t], o[t + 1]) << t;
+                    for (int t = 0; t < 4; t++) o[t] = __fsub_rn(h[t], __fmul_rn(l[t], w1));
+                } else {
+#pragma unroll
+                    for (int t = 0; t < 4; t += 2)
+                        m |= de_fast2(pk2(h[t], h[t + 1]), hb[t], hb[t + 1], l[t], l[t + 1], lm[t],
+                                      lm[t + 1], w1, w2, o[t], o[t + 1]) << t;
+                }
             } else {
 #pragma unroll
                 for (int t = 0; t < 4; t++) o[t] = de_slow(h[t], l[t], W.w[k]);
@@ -221,7 +227,7 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
             } else {
 #pragma unroll
                 for (int t = 0; t < 4; t++)
-                    if (i + 32 * t < n) __stcs(row + 32 * t, o[t]);
+                    if (32 * t < lim) __stcs(row + 32 * t, o[t]);
             }
         }
         if (!__any_sync(0xffffffffu, bad != 0)) continue;
@@ -252,7 +258,7 @@ __global__ void __launch_bounds__(256, DE_BLOCKS) de_subtract_kernel(
             }
             if (on)
                 d[(int64_t)k * n + i0 + (VEC ? 4 * from + t : from + 32 * t)] =
-                    __double2float_rn(de_value(b, a, sw[k]));
+                    __double2float_rn(de_value(b, a, W.w[k]));
         }
         __syncwarp();
     }
