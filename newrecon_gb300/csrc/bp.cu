@@ -288,14 +288,15 @@ static nr_status launch_sbp(const nr_geom& g, float* vol, const float* prj, cons
                             const float* angles, const int32_t* index, int a0, int a1,
                             float lambda, float beta, cudaStream_t s) {
     const int64_t tiles = (int64_t)cdiv(g.nx, BP_T) * cdiv(g.ny, BP_T);
-    const int64_t full = tiles * g.nz / (152 * 16);
+    const int sms = sm_count();
+    const int64_t full = tiles * g.nz / (sms * 16);
     const int zc = (int)(full < 1 ? 1 : (full > 8 ? 8 : full));
     const dim3 grd((unsigned)tiles, cdiv(g.nz, zc));
     const int64_t voxels = (int64_t)g.nx * g.ny * g.nz;
-    if (voxels <= 152 * 4 * 128 || 5 * voxels < 2 * tiles * BP_T * BP_T * g.nz)
+    if (voxels <= sms * 4 * 128 || 5 * voxels < 2 * tiles * BP_T * BP_T * g.nz)
         bp_small_kernel<OSSART><<<cdiv(voxels, 128), 128, 0, s>>>(
             make_geo(g), vol, prj, prior, angles, index, a0, a1 - a0, lambda, beta);
-    else if (tiles * g.nz <= 152)
+    else if (tiles * g.nz <= sms)
         bp_kernel<OSSART, 1024><<<grd, 1024, 0, s>>>(make_geo(g), vol, prj, prior, angles, index,
                                                      a0, a1 - a0, zc, lambda, beta);
     else

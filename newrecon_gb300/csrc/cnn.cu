@@ -1625,13 +1625,6 @@ static WSL layout(const Dims& d, bool training) {
     return L;
 }
 
-static int sm_count() {
-    int dev = 0, n = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-}
-
 }  // namespace cnn
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encode_fn();
 namespace cnn {

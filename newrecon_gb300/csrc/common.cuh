@@ -94,6 +94,15 @@ __host__ inline nr_status launch_status() {
     return e == cudaSuccess ? NR_OK : NR_ERR_LAUNCH;
 }
 
+// SMs of the current device (152 where there is none to ask: host-side set-up).
+__host__ inline int sm_count() {
+    int dev = 0, n = 152;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    return n;
+}
+
 __host__ inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
 // A captured launch sequence: the graph and its executable instance (the

@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(256) hist8_kernel(const float* __restrict__ x,
 }
 
 static unsigned de_blocks(int64_t work) {
-    int64_t b = (work + 255) / 256;
-    return (unsigned)(b > 152 * 16 ? 152 * 16 : (b < 1 ? 1 : b));
+    const int64_t b = (work + 255) / 256, most = 16 * sm_count();
+    return (unsigned)(b > most ? most : (b < 1 ? 1 : b));
 }
 
 }  // namespace nr
@@ -363,7 +363,8 @@ NR_API nr_status nr_de_subtract(const float* he, const float* le, const double* 
                                                                hist, W);
     }
     const int64_t steps = (n + 8 * DE_TILE - 1) / (8 * DE_TILE);
-    const unsigned blocks = (unsigned)(steps > 152 * DE_BLOCKS ? 152 * DE_BLOCKS : steps);
+    const int64_t most = DE_BLOCKS * sm_count();
+    const unsigned blocks = (unsigned)(steps > most ? most : steps);
     if (n > 0 && n % 4 == 0)
         de_subtract_kernel<true><<<blocks, 256, 0, s>>>(he, le, d, n, W);
     else if (n > 0)

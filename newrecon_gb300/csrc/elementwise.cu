@@ -116,8 +116,8 @@ __global__ void transpose_kernel(float* __restrict__ out, const float* __restric
 }
 
 static unsigned ew_blocks(int64_t n) {
-    int64_t b = (n + 255) / 256;
-    return (unsigned)(b > 152 * 64 ? 152 * 64 : (b < 1 ? 1 : b));
+    const int64_t b = (n + 255) / 256, most = 64 * sm_count();
+    return (unsigned)(b > most ? most : (b < 1 ? 1 : b));
 }
 
 nr_status launch_transpose(float* out, const float* in, int rows, int cols, int nviews, int M,

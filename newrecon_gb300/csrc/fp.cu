@@ -505,7 +505,7 @@ nr_status launch_gamma_yry(const nr_geom& g, int gamma_mode, float* out, const P
         gamma_chord_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r);
     } else {
         const int64_t single = (int64_t)cdiv(g.nbx, 32) * cdiv(g.nby, 4) * g.n_angles;
-        const int64_t n = single / (152 * 8);
+        const int64_t n = single / (8 * sm_count());
         const int rows = (int)(n < 1 ? 1 : (n > GL_ROWS ? GL_ROWS : n));
         dim3 grd(cdiv(g.nbx, 32), cdiv(g.nby, 4 * rows), g.n_angles);
         gamma_length_kernel<<<grd, blk, 0, st>>>(make_geo(g), out, views, index, y, r, rows);

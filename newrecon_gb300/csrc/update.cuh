@@ -29,8 +29,9 @@ constexpr int UPD_BLOCKS = 5;
 // 256 blocks of 16 planes, 768 of 4).  blocks(zc): those of a launch.
 template <class F>
 __host__ inline int upd_planes_by(F blocks) {
+    const int fill = sm_count() * UPD_BLOCKS;
     for (int zc = UZC; zc > 4; zc /= 2)
-        if (blocks(zc) >= 152 * UPD_BLOCKS) return zc;
+        if (blocks(zc) >= fill) return zc;
     return 4;
 }
 __host__ inline int64_t upd_blocks(const nr_geom& g, int zc) {
