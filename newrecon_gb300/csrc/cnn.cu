@@ -1606,12 +1606,12 @@ static WSL layout(const Dims& d, bool training) {
     L.pk_fwd[5] = take(PK_LAST);
     const int nact = training ? 5 : 2;
     for (int k = 0; k < nact; k++) L.act[k] = take((size_t)V * C * 2);
-    L.f = take((size_t)V * 4);
     L.nchunk = ntiles(d) < WG_MAXCTA ? ntiles(d) : WG_MAXCTA;  // CTAs of a weight gradient
     L.lblocks = 1024;
     if (training) {
         for (int l = 1; l < 5; l++) L.pk_bwd[l] = take(PK_HID);
         L.pk_bwd[5] = take(PK_ONE);
+        L.f = take((size_t)V * 4);
         L.r = take((size_t)V * 4);
         L.g6 = take((size_t)V * 4);
         L.dpre[0] = take((size_t)V * C * 2);
