@@ -157,7 +157,7 @@ typedef struct nr_ostr_params {
                                   where the volume allows it (IMGSIZx a multiple of
                                   4, x 16-byte aligned; fp_batch 2 or 4).  Same
                                   result either way; on the clinical workload the
-                                  staged form is slower (0.255 vs 0.162 ms).     */
+                                  staged form is slower (0.256 vs 0.114 ms).     */
     int32_t upd_tile;          /* NR_TILE_1 (default) and NR_TILE_2: each thread of
                                   the update owns two voxels, one above the other
                                   in y, of a 32 x 8-column tile.  NR_TILE_TMA: one
@@ -181,7 +181,7 @@ enum {
 /* fp_batch, fp_stage, upd_planes and upd_tile select kernel variants only
  * (every variant gives the same result); the autotuner
  * (newrecon_gb300/autotune.py) picks them per geometry.  The batched path
- * uses the defaults. */
+ * takes upd_planes and the default of the others. */
 
 /* Bytes of workspace the fused path needs for this geometry and parameters. */
 nr_status nr_ostr_workspace_size(const nr_geom* g, const nr_ostr_params* p,

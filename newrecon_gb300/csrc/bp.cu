@@ -16,7 +16,8 @@
 // instead of 1024, and keeps its views (a double sincos each) over several
 // planes.  One view of 1024 x 512 x 60: 189 us, from 505 us with a thread per
 // voxel along x; five views of 701 x 353 x 45: 143 us from 380.  Bound by the
-// instructions of the depth weight's division and the interpolation.
+// latency of the taps and of the barriers between a plane's phases: 94 M warp
+// instructions at 42 % issue-active, 31 warps per SM at 64 registers.
 #include "common.cuh"
 
 namespace nr {

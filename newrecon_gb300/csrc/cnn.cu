@@ -17,7 +17,7 @@
 // 16 B).  The strips arrive by TMA (activations are stored in 8-channel planes
 // so that a strip's K chunk is one contiguous block); a CTA walks along y and
 // adds each staged input row into the accumulators of the three output rows
-// that read it, and a producer warp, an MMA warp and groups of epilogue warps
+// that read it, and a producer warp, two MMA warps and groups of epilogue warps
 // overlap staging, MMAs and stores (conv32_ys_kernel).  Weights of all 27 taps
 // stay in shared memory.  1-channel inputs gather the 27 neighbours into one K = 32 row
 // instead.  Weight gradients are GEMMs over voxels on the tensor cores
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(Y_THREADS, 1) conv32_ys_kernel(
 //     f[v] = b + sum_{(dz, dy)} q[(dz, dy)][v + (0, dy - 1, dz - 1)]
 // (zero outside the patch), nine coalesced loads in a fixed order.  Pass 1:
 // a producer lane loads the strips into a ring of LR_STAGE stages, an issuer
-// lane runs the MMAs into one of two TMEM accumulators, four epilogue warps
+// warp runs the MMAs into one of two TMEM accumulators, four epilogue warps
 // store the nine planes of q; waits bounded as in conv32_ys_kernel.
 constexpr int LR_STAGE = 6;
 constexpr int LR_THREADS = 192;
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(128) conv1_kernel(Dims d, WalkPlan wp, const f
 //
 // Roles (6 warps): warp 0 lane 0 loads each K block's strips by TMA into one
 // of two stages (a strip outside the patch in z or y is loaded from row -1,
-// i.e. zero-filled); warp 1 lane 0 issues the MMAs and frees the stage by
+// i.e. zero-filled); warp 1 (one elected lane) issues the MMAs and frees the stage by
 // tcgen05.commit; warps 2-5 (x - x0 in 32 h .. 32 h + 31 for warp 2 + h) build
 // the split operand from global data fetched one block ahead and sum the
 // bias.  Every wait is bounded and gives up once another role has aborted; a

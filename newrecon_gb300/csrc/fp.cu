@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(256) fp_4r_kernel(const __grid_constant__ Geo 
 // the three-axis walk of siddon.cuh at 12 blocks per SM (145 M warp
 // instructions, 74 % issue-active), 0.151 with the row lists but each block's
 // view computed by one of its threads (107 M, 59 %: a fifth of the warps' time
-// at that barrier), 0.122 with the views from the workspace (100 M, 69 %) and
-// 0.117 at FP_BLOCKS = 16.
+// at that barrier), 0.122 with the views from the workspace (100 M, 69 %),
+// 0.117 at FP_BLOCKS = 16 and 0.114 with the rows of several lists out of line.
 //
 // LONG (rows of more cells than a list): the walk over several lists takes more
 // registers than 16 blocks leave.  256 x 128 x 300, three views, K = 4: 55 us
@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(1024) partials_sum_kernel(const double* __rest
 
 // The same with the volume staged slab by slab through shared memory by TMA
 // (slab.cuh); bit-identical to fp_h_kernel.  Measured on the clinical
-// workload it is slower than the direct gathers (0.255 ms with 4-plane slabs,
-// 0.346 ms with 2-plane slabs, against 0.162 ms): the walk's gathers already
+// workload it is slower than the direct gathers (0.256 ms with 4-plane slabs
+// against 0.114; with 2-plane slabs 0.346 before the row lists): the walk's gathers already
 // hit L1 three times in four and the walk is instruction bound, so the
 // per-slab synchronisation and bookkeeping cost more than the latency they
 // hide.  It is kept as an option (NR_STAGE_TMA).
