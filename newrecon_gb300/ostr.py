@@ -631,7 +631,8 @@ class Batch:
 
     tune=True runs the autotuner on each case's plan first (cached per
     geometry): the batched update then walks each case with its tuned slab
-    depth and tile.  The batched projection always uses 4-step gathers.
+    depth; cases that leave it open share one, by the size of them all.  The
+    batched projection always uses 4-step gathers.
 
     mode: "shared" advances all cases by the shared launches; "sequential"
     runs the cases one after another through their own iteration loops (a
